@@ -5,8 +5,9 @@
 // cannot carry at millions of bodies; this form keeps every pair term in FP32 and every
 // sum exact enough that the energy drift of a run can be read to a few 1e-9:
 //   - the potential is E_pot = -G sum_{i<j} m_i m_j / sqrt(|d_ij|^2 + eps2), over the
-//     upper triangle of 1024-body blocks: one CTA per block row I sums blocks J >= I, the
-//     diagonal block at half weight (it holds every pair of the block twice);
+//     upper triangle of 1024-body blocks: a CTA sums one chunk of 256-body tiles of a block
+//     row I (blocks J >= I), the diagonal block at half weight (it holds every pair of the
+//     block twice);
 //   - per target, packed FP32 pair terms m_j / r_ij (rsqrt on the SFU) are summed in FP32
 //     per 256-source tile and the tile sums folded into an (S, C) pair by an error-free
 //     TwoSum, as the direct sum folds its accelerations; m_i (S + C) is added in FP64;
@@ -15,6 +16,7 @@
 //   - E_kin = 1/2 sum_i m_i |v_i|^2 and P = sum_i m_i v_i in FP64;
 //   - every total is summed per block in a fixed tree order and the block partials in
 //     order on the host, so the result is deterministic.
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -27,15 +29,29 @@ namespace nbg
         constexpr int kEBlock = 256;            // threads per CTA; also sources per tile
         constexpr int kET = 4;                  // targets per thread (two packed pairs)
         constexpr int kRedBlock = 256;
+        constexpr size_t kEnergyChunks = 8192;  // CTAs the triangle is cut into, about
     }
 
-    // Row I of the block triangle: part[I] = sum over blocks J >= I of
-    // sum_{i in I, j in J} m_i m_j / r_ij, the diagonal block at half weight (unscaled by
-    // G). src is pos_mass (stride 1) or the Body array as float4 (stride 3: mass in the
-    // second record's w). The longest rows (small I) are the first CTAs, so the short ones
-    // fill in at the end.
+    // Tiles per CTA: a row has up to n / 256 tiles, and the rows' lengths fall linearly, so one
+    // CTA a row leaves the last rows' SMs idle (n = 200,003: 196 CTAs for 456 slots, as long as
+    // the longest: 10.2 ms; in chunks 5.1 ms, 3.9e12 pairs/s). About 8192 CTAs (18 waves of
+    // three per SM) balance to a few percent; 4096 took 1 % more there and 2 % at n = 2^19,
+    // 16384 the same to 1 %. Rows are whole chunks once there are 16384 of them (n = 2^24). A
+    // function of n only, so the total's bits are too.
+    int chunk_tiles(const size_t n)
+    {
+        const size_t rows = (n + kEBlock * kET - 1) / (kEBlock * kET), tiles = (n + kEBlock - 1) / kEBlock;
+        return static_cast<int>(std::max<size_t>(1, (rows + 1) * tiles / 2 / kEnergyChunks));
+    }
+
+    // CTA I * chunks + c sums chunk c of row I of the block triangle: part[I * chunks + c] = sum
+    // over i in I and the chunk's bodies j of m_i m_j / r_ij, those of the diagonal block at
+    // half weight (unscaled by G); 0 for a chunk past the row's end. src is pos_mass
+    // (stride 1) or the Body array as float4 (stride 3: mass in the second record's w).
+    // Bound by the SFU: one rsqrt a pair, 16 per clock and SM.
     __global__ void __launch_bounds__(kEBlock, 3) potential_rows_kernel(const float4* __restrict__ src, const int stride,
-                                                                        const int n, const float eps2,
+                                                                        const int n, const int tiles,
+                                                                        const unsigned chunks, const float eps2,
                                                                         double* __restrict__ part)
     {
         constexpr int P = kET / 2;
@@ -43,8 +59,17 @@ namespace nbg
         __shared__ float4 tile[kEBlock];
         __shared__ double red[kEBlock];
         const int tid = threadIdx.x;
-        const int row = blockIdx.x;
-        const int base = row * kRows;
+        const int base = static_cast<int>(blockIdx.x / chunks) * kRows;
+        double* out = part + blockIdx.x;
+        // the chunk's sources [first, last); 64-bit: a chunk past the end may start beyond 2^31
+        const long long first = static_cast<long long>(base) + static_cast<long long>(blockIdx.x % chunks) * tiles * kEBlock;
+        if (first >= n)
+        {
+            if (tid == 0)
+                *out = 0.0;
+            return;
+        }
+        const int last = static_cast<int>(min(static_cast<long long>(n), first + static_cast<long long>(tiles) * kEBlock));
         float2 nx[P], ny[P], nz[P], mt[P], acc[P], S[P], C[P];
 #pragma unroll
         for (int p = 0; p < P; ++p)
@@ -80,7 +105,7 @@ namespace nbg
                 S[p] = C[p] = make_float2(0.f, 0.f);
             }
         };
-        for (int j0 = base; j0 < n; j0 += kEBlock)
+        for (int j0 = static_cast<int>(first); j0 < last; j0 += kEBlock)
         {
             const int j = j0 + tid;
             float4 s = make_float4(0.f, 0.f, 0.f, 0.f);     // padding: massless, adds 0
@@ -119,11 +144,11 @@ namespace nbg
                 C[p] = add2(C[p], err);
                 acc[p] = make_float2(0.f, 0.f);
             }
-            // the diagonal block is complete after its last tile (a short one in the last row)
-            if (j0 < base + kRows && j0 + kEBlock >= min(n, base + kRows))
+            // the chunk's part of the diagonal block ends here, or with the chunk
+            if (j0 + kEBlock == base + kRows)
                 settle(diag);
         }
-        settle(off);
+        settle(last > base + kRows ? off : diag);
         red[tid] = 0.5 * diag + off;
         __syncthreads();
         for (int k = kEBlock / 2; k > 0; k >>= 1)
@@ -133,7 +158,7 @@ namespace nbg
             __syncthreads();
         }
         if (tid == 0)
-            part[row] = red[0];
+            *out = red[0];
     }
 
     // Per block: {sum m |v|^2, sum m v} in FP64, by a fixed-order tree.
@@ -196,13 +221,17 @@ namespace nbg
         const float eps2 = p->law == NBODY_LAW_SOFTENED ? p->eps2 : 0.f;
         const unsigned rows = ceil_div(n, kEBlock * kET);
         const unsigned red_blocks = ceil_div(n, kRedBlock);
-        const size_t words = static_cast<size_t>(rows) + 4 * static_cast<size_t>(red_blocks);
+        const int tiles = chunk_tiles(n);
+        const unsigned chunks = ceil_div(n, static_cast<size_t>(tiles) * kEBlock);
+        const size_t sums = static_cast<size_t>(rows) * chunks;
+        const size_t words = sums + 4 * static_cast<size_t>(red_blocks);
         if (const int st = ensure_scratch(ctx, words * sizeof(double)))
             return st;
         ctx->pending_partials = 0;      // the scratch is reused here
         double* rowsum = static_cast<double*>(ctx->scratch);
-        double* kin = rowsum + rows;
-        potential_rows_kernel<<<rows, kEBlock, 0, ctx->stream>>>(src, stride, ni, eps2, rowsum);
+        double* kin = rowsum + sums;
+        potential_rows_kernel<<<static_cast<unsigned>(sums), kEBlock, 0, ctx->stream>>>(src, stride, ni, tiles, chunks,
+                                                                                             eps2, rowsum);
         kinetic_kernel<<<red_blocks, kRedBlock, 0, ctx->stream>>>(src, aos ? nullptr : ctx->vr, stride, ni, kin);
         ctx->launches += 2;
         cudaError_t e = cudaGetLastError();
@@ -214,11 +243,11 @@ namespace nbg
         if (e != cudaSuccess)
             return ctx_cuda_fail(ctx, e, "energy diagnostics");
         double pot = 0.0, sum[4] = { 0.0, 0.0, 0.0, 0.0 };
-        for (unsigned r = 0; r < rows; ++r)
+        for (size_t r = 0; r < sums; ++r)
             pot += h[r];
         for (unsigned b = 0; b < red_blocks; ++b)
             for (int c = 0; c < 4; ++c)
-                sum[c] += h[rows + static_cast<size_t>(b) * 4 + c];
+                sum[c] += h[sums + static_cast<size_t>(b) * 4 + c];
         out[0] = 0.5 * sum[0];
         out[1] = -static_cast<double>(p->G) * pot;
         out[2] = sum[1];

@@ -78,3 +78,19 @@ def test_energy_empty_and_rejects(gpu):
         assert e["kinetic"] == 0 and e["potential"] == 0
         with pytest.raises(gpu.NbodyError):
             ctx.energy(gpu.params(law=gpu.LAW_SOFTENED, eps2=0.0))
+
+
+@pytest.mark.parametrize("n", [1024, 1025, 96001, 113501, 150001])
+def test_energy_chunked_rows(gpu, n):
+    """Rows cut into chunks that end inside the diagonal block (2 and 3 tiles a chunk), beyond
+    it (5) and on its edge, against the FP64 diagnostics: the file's bar, 1e-7."""
+    from nbody_gb300 import scenes
+    b = scenes.uniform_cube(n, seed=11)
+    p = gpu.params(law=gpu.LAW_SOFTENED, eps2=1e-6)
+    with gpu.Context() as ctx:
+        ctx.upload_bodies(b)
+        e = ctx.energy(p)
+        ref = ctx.system_energy(p)[0]
+        again = ctx.energy(p)
+    assert abs(e["potential"] - ref[1]) <= 1e-7 * abs(ref[1]), (e["potential"], ref[1])
+    assert e["potential"] == again["potential"]
