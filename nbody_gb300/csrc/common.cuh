@@ -114,6 +114,23 @@ namespace nbg
         return y;
     }
 
+    // Whether an FP64 value is normal, positive and finite (an integer test of its high word).
+    __device__ __forceinline__ bool normal_positive(const double x)
+    {
+        return static_cast<unsigned>(__double2hiint(x) - 0x100000) < 0x7fe00000u;
+    }
+
+    // An approximate FP64 reciprocal square root y of a normal positive x: 21 significant bits
+    // (the low word is zero), so that y^2, and y times a float, are exact, and
+    // |1 - x y^2| < 2^-19 (2^-19.04 measured over 6.7e7 arguments in [1, 4)). The FP32
+    // instruction with the exponents moved by integer operations, 24 bits, took the same time.
+    __device__ __forceinline__ double rsqrt_approx64(const double x)
+    {
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        return y;
+    }
+
     __device__ __forceinline__ float2 f2(const float a) { return make_float2(a, a); }
     __device__ __forceinline__ float2 add2(const float2 a, const float2 b) { return __fadd2_rn(a, b); }
     __device__ __forceinline__ float2 mul2(const float2 a, const float2 b) { return __fmul2_rn(a, b); }

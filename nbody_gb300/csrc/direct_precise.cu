@@ -14,6 +14,7 @@
 // FP64 form: the whole pair sum in FP64 (positions promoted exactly from the FP32 offsets
 // plus the FP64 origin, or from the float positions when no split state exists).
 #include <algorithm>
+#include <climits>
 
 #include "common.cuh"
 #include "context.cuh"
@@ -325,6 +326,17 @@ namespace nbg
     // --------------------------------------------------------------------------------------
     // FP64 direct sum (sources staged as double4 tiles)
     // --------------------------------------------------------------------------------------
+    // Bound by the FP64 pipe (2 lanes per clock and SM), so by FP64 instructions a pair: 16
+    // here (3 differences, 3 for r^2, 7 for m / r^3, 3 sums), with the comparisons on the
+    // integer pipe; the pipe is 91 % busy at n = 40,000. With rsqrt(), its cube formed after
+    // it, and FP64 compares there were 24: n = 12,289 took 5.87 ms, 4.60 ms now (5.19 ms of
+    // them before plan_split64).
+    //
+    // m / r^3 from an approximation y of 1 / r with 21 significant bits, so that y^2 and m y (m
+    // a float) are exact: with e = 1 - r^2 y^2, r^-3 = y^3 (1 - e)^(-3/2)
+    // = y^3 (1 + 3/2 e + 15/8 e^2 + 35/16 e^3 + ...). |e| < 2^-19, so what is left out is below
+    // 2^-55 of the result, which has a rounding of y^2 (1 + ...) and one of the product with m y: within
+    // 2.1 units of 2^-53 over 6.7e7 arguments, where the cube of rsqrt() is within 4.9.
     template <int BLOCK, int LAW>
     __global__ void __launch_bounds__(BLOCK)
     direct_fp64_kernel(const double4* __restrict__ src, const float* __restrict__ radius2, const int* __restrict__ tlist,
@@ -356,7 +368,8 @@ namespace nbg
         if (tid == 0)
             for (int s = 0; s < kStages && s < ntiles; ++s)
                 issue(s, s);
-        double px[T], py[T], pz[T], lim[T], ax[T], ay[T], az[T];
+        double px[T], py[T], pz[T], ax[T], ay[T], az[T];
+        long long lim[T];       // the cutoff radius^2's bit pattern; of a NaN, above every r^2
 #pragma unroll
         for (int k = 0; k < T; ++k)
         {
@@ -366,7 +379,8 @@ namespace nbg
             px[k] = x.x;
             py[k] = x.y;
             pz[k] = x.z;
-            lim[k] = (LAW == NBODY_LAW_CUTOFF) ? (double)radius2[i] : eps2;
+            const double r2 = (LAW == NBODY_LAW_CUTOFF) ? static_cast<double>(radius2[i]) : 0.0;
+            lim[k] = isnan(r2) ? LLONG_MAX : __double_as_longlong(r2);
             ax[k] = ay[k] = az[k] = 0.0;
         }
         int failed_at = -1;
@@ -394,15 +408,20 @@ namespace nbg
                 for (int k = 0; k < T; ++k)
                 {
                     const double dx = s.x - px[k], dy = s.y - py[k], dz = s.z - pz[k];
-                    double r2 = (LAW == NBODY_LAW_SOFTENED) ? fma(dx, dx, lim[k]) : dx * dx;
+                    double r2 = (LAW == NBODY_LAW_SOFTENED) ? fma(dx, dx, eps2) : dx * dx;
                     r2 = fma(dy, dy, r2);
                     r2 = fma(dz, dz, r2);
-                    double inv = rsqrt(r2);
+                    const double y = rsqrt_approx64(r2);
+                    const double y2 = y * y;
+                    const double e = fma(-r2, y2, 1.0);
+                    const double g = fma(y2, e * fma(e, 1.875, 1.5), y2);
+                    // no force where r^2 is 0 (massless padding at the origin, the body itself),
+                    // infinite or NaN, nor within the cutoff; non-negative doubles order as
+                    // their bit patterns do
+                    bool apply = normal_positive(r2);
                     if (LAW == NBODY_LAW_CUTOFF)
-                        inv = r2 > lim[k] ? inv : 0.0;
-                    if (!(r2 > 0.0))
-                        inv = 0.0;      // massless padding at the origin / self at d = 0
-                    const double f = s.w * inv * inv * inv;
+                        apply = apply && __double_as_longlong(r2) > lim[k];
+                    const double f = apply ? (s.w * y) * g : 0.0;
                     ax[k] = fma(dx, f, ax[k]);
                     ay[k] = fma(dy, f, ay[k]);
                     az[k] = fma(dz, f, az[k]);
@@ -646,6 +665,22 @@ namespace nbg
             return p;
         }
 
+        // The FP64 form's split. A CTA's share of the SM's two FP64 lanes is long even for one
+        // tile (256 targets x 128 sources: 0.1 ms), so the split is by balance alone: about 24
+        // CTAs per SM, down to one tile a chunk, up to 512 chunks (sampled sums have few target
+        // blocks). Split into one wave of four CTAs per SM, n = 12,289 left some SMs three and
+        // others four: 5.19 against 4.60 ms.
+        Split plan_split64(const size_t nt, const size_t n, const int per_cta, const int tile, const int sms)
+        {
+            Split p;
+            p.tb = static_cast<int>(std::max<size_t>(1, (nt + per_cta - 1) / per_cta));
+            const size_t tiles = (n + tile - 1) / tile;
+            const size_t js = std::min<size_t>({ (static_cast<size_t>(sms) * 24 + p.tb - 1) / p.tb, tiles, 512 });
+            p.chunk = static_cast<int>((tiles + js - 1) / js * tile);
+            p.js = static_cast<int>((n + p.chunk - 1) / p.chunk);
+            return p;
+        }
+
         int sms_of(const nbody_cuda* ctx)
         {
             int sms = 0;
@@ -666,7 +701,7 @@ namespace nbg
             const bool fp64 = p->precision == NBODY_PREC_FP64;
             const int sms = sms_of(ctx);
             constexpr int kT = 4, kB = 256, kB64 = 128;
-            const Split sp = fp64 ? plan_split(nt, n, kB64 * 2, kTile64, sms * 4)
+            const Split sp = fp64 ? plan_split64(nt, n, kB64 * 2, kTile64, sms)
                                   : plan_split(nt, n, kB * kT, kTileC, sms * 2);
             // scratch: partials (js * nt double4) + radius^2 (n floats)
             const size_t part_bytes = static_cast<size_t>(sp.js) * nt * sizeof(double4);

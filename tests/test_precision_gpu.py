@@ -190,3 +190,30 @@ def test_bh_with_compensated_integration(gpu):
             outs.append(ctx.download_bodies())
     assert np.all(np.isfinite(outs[1]))
     assert np.abs(outs[0][:, :3] - outs[1][:, :3]).max() < 1e-4
+
+
+@pytest.mark.parametrize("scale_pos", [1.0, 1e-15, 1e15], ids=["unit", "tiny", "huge"])
+@pytest.mark.parametrize("n", [1, 2, 127, 128, 129, 257, 4097])
+@pytest.mark.parametrize("law", [0, 1], ids=["cutoff", "softened"])
+def test_fp64_sizes_and_ranges(gpu, law, n, scale_pos):
+    """The FP64 form at the edges of its tiles and target blocks, over distances 30 decades
+    apart, with coincident bodies, massless ones and, under the cutoff law, radii that cut off
+    all, none and some pairs. The file's bar: a sum of n terms of a few roundings each is
+    within (n + 8) 2^-53 < 1e-12 of sum_j |a_ij|."""
+    from nbody_gb300 import scenes
+    b = scenes.uniform_cube(n, seed=5 + n)
+    b[:, :3] *= np.float32(scale_pos)
+    b[n // 2:n // 2 + 3, :3] = b[0, :3]
+    b[n // 3, 7] = 0.0
+    b[::3, 3] = np.float32(0.05 * scale_pos)
+    b[1::7, 3] = np.inf
+    eps2 = float(np.float32(1e-4)) * float(scale_pos) ** 2 if law == 1 else 0.0
+    p = gpu.params(law=law, eps2=eps2, precision=gpu.PREC_FP64)
+    with gpu.Context() as ctx:
+        ctx.upload_bodies(b)
+        got = ctx.accel_sampled(p, np.arange(n))
+        few = ctx.accel_sampled(p, np.arange(0, n, 50))
+    ref, scale = f64_ref(b, float(np.float32(eps2)), law)
+    assert np.all(np.isfinite(got))
+    assert np.all(np.linalg.norm(got - ref, axis=1) <= 1e-12 * scale)
+    assert np.all(np.linalg.norm(few - ref[::50], axis=1) <= 1e-12 * scale[::50])
