@@ -85,16 +85,40 @@ namespace nbg
     // so that the origin lies within e/2 of the centre and x - origin is exact by Sterbenz's
     // lemma for a system far from 0 (its whole point). Whatever rounding remains at set-up
     // goes into the compensation term, so origin + offset - compensation == x exactly.
-    __global__ void origin_kernel(const double* __restrict__ part, const int nparts, double* __restrict__ origin)
+    // One block folds the partials (min and max: exact in any order); a lone thread reading
+    // them one after another took 0.21 ms, 5 % of four steps of 50,021 bodies.
+    __global__ void __launch_bounds__(256) origin_kernel(const double* __restrict__ part, const int nparts,
+                                                         double* __restrict__ origin)
     {
-        if (threadIdx.x || blockIdx.x)
-            return;
+        __shared__ double red[6][8];
         double lo[3] = { INFINITY, INFINITY, INFINITY }, hi[3] = { -INFINITY, -INFINITY, -INFINITY };
-        for (int k = 0; k < nparts; ++k)
+        for (int k = threadIdx.x; k < nparts; k += 256)
             for (int a = 0; a < 3; ++a)
             {
                 lo[a] = fmin(lo[a], part[k * 6 + a]);
                 hi[a] = fmax(hi[a], part[k * 6 + 3 + a]);
+            }
+        for (int a = 0; a < 3; ++a)
+        {
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                lo[a] = fmin(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+                hi[a] = fmax(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+            }
+            if ((threadIdx.x & 31) == 0)
+            {
+                red[a][threadIdx.x >> 5] = lo[a];
+                red[3 + a][threadIdx.x >> 5] = hi[a];
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x)
+            return;
+        for (int w = 1; w < 8; ++w)
+            for (int a = 0; a < 3; ++a)
+            {
+                lo[a] = fmin(lo[a], red[a][w]);
+                hi[a] = fmax(hi[a], red[3 + a][w]);
             }
         double ext = 0.0;
         for (int a = 0; a < 3; ++a)
@@ -625,7 +649,7 @@ namespace nbg
             int stride = 1;
             const float4* src = body_src(ctx, &stride);
             minmax_kernel<<<kBboxBlocks, 256, 0, ctx->stream>>>(src, stride, static_cast<int>(n), s.part);
-            origin_kernel<<<1, 32, 0, ctx->stream>>>(s.part, kBboxBlocks, s.origin);
+            origin_kernel<<<1, 256, 0, ctx->stream>>>(s.part, kBboxBlocks, s.origin);
             to_offsets_kernel<<<ceil_div(n, 256), 256, 0, ctx->stream>>>(src, stride, static_cast<int>(n), s.origin,
                                                                          s.off, s.cx, s.cv);
             ctx->launches += 3;
