@@ -27,19 +27,18 @@
 //      as its deepest cell: that is the node kept. Each node lists its <= 8 children
 //      (cells or single bodies); cells at the Morton limit (identical codes) are buckets
 //      whose bodies are applied one by one when opened;
-//   7. traverse_pairs_kernel (the default; traverse_kernel is its one-target-per-lane
-//      form): a warp walks the tree for 128 Morton-consecutive targets, four per lane as
-//      two packed pairs, with one shared stack of (node, lane mask per target slot)
-//      entries. Every target evaluates the reference test itself -- accept when
-//      |com - x|^2 > size^2 * theta^2 (bhtree.cpp:117-125), leaves always applied,
-//      massless nodes skipped -- and a node is opened only for the targets that rejected
-//      it, so each target sums exactly the nodes the reference's traversal would, in a
-//      different order (the same order in every walk width, so the sums agree bit for
-//      bit).
+//   7. traverse_kernel: a warp walks the tree for 32 to 128 Morton-consecutive targets, opening
+//      one cell at a time for the targets that rejected it. Every target applies the
+//      reference test -- accept when |com - x|^2 > size^2 * theta^2 (bhtree.cpp:117-125), leaves
+//      always applied, massless nodes skipped -- most often decided for all of them at once by
+//      their bounding boxes, exactly; so each target sums exactly the nodes the reference's
+//      traversal would, in an order that depends on the target alone (the sums agree bit for
+//      bit whatever the walk's width).
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "bh.cuh"
 #include "common.cuh"
@@ -53,11 +52,14 @@ namespace nbg
     {
         constexpr int kMortonBits = 21;
         constexpr int kMaxLevel = 21;
-        constexpr int kTravWarps = 8;
-        // warps per CTA of the walk with Q packed pairs per lane: its stack entries carry 2Q
-        // lane masks, and the stacks of one CTA stay within 48 KB of static shared memory
-        __host__ __device__ constexpr int pair_warps(const int q) { return q > 2 ? 4 : kTravWarps; }
-        constexpr int kStack = 192;
+        // warps per CTA of the walk with H targets per lane: its stack entries carry H lane masks,
+        // and the stacks of one CTA stay within 48 KB of static shared memory
+        __host__ __device__ constexpr int trav_warps(const int h) { return h > 4 ? 4 : 8; }
+        // and CTAs per SM: two targets a lane fit 64 registers (a million bodies: 3 to 7 % over
+        // three CTAs of 80; one and four targets a lane were slower so)
+        __host__ __device__ constexpr int trav_ctas(const int h) { return h > 4 || h == 2 ? 4 : 3; }
+        // cells stacked by a walk: at most 7 stay per level (8 are pushed, 1 is popped), 22 levels
+        constexpr int kStack = 164;
         // group walk: warps per CTA, list entries and stacked parent cells per warp (the
         // stack grows by at most 28 parents per tree level, 22 levels: 616 < 768)
         constexpr int kListWarps = 4;
@@ -1150,7 +1152,7 @@ namespace nbg
     template <int LAW>
     __device__ __forceinline__ void apply(const float px, const float py, const float pz, const float lim,
                                           const float sx, const float sy, const float sz, const float m,
-                                          float& ax, float& ay, float& az)
+                                          const bool take, float& ax, float& ay, float& az)
     {
         const float dx = sx - px, dy = sy - py, dz = sz - pz;
         float r2 = (LAW == NBODY_LAW_SOFTENED) ? fmaf(dx, dx, lim) : dx * dx;
@@ -1159,157 +1161,11 @@ namespace nbg
         float inv = rsqrt_sfu(r2);
         if (LAW == NBODY_LAW_CUTOFF)
             inv = r2 > lim ? inv : 0.f;     // physics.h:38-39
-        const float s = m * inv * inv * inv;
+        float s = m * inv * inv * inv;
+        s = take ? s : 0.f;
         ax = fmaf(dx, s, ax);
         ay = fmaf(dy, s, ay);
         az = fmaf(dz, s, az);
-    }
-
-    template <int LAW>
-    __global__ void __launch_bounds__(kTravWarps * 32, 4) traverse_kernel(
-        const OctNode* __restrict__ nodes, const float4* __restrict__ spm, const float* __restrict__ srad,
-        const uint32_t* __restrict__ order, const int n, const float G, const float eps2,
-        float4* __restrict__ acc, float* __restrict__ body_out, unsigned* __restrict__ err,
-        unsigned long long* __restrict__ stats)
-    {
-        // one 8-byte entry per stacked cell: {cell index, mask of the lanes that opened it}
-        __shared__ int2 stk[kTravWarps][kStack];
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const unsigned lt = (1u << lane) - 1u;
-        unsigned inter = 0, visits = 0;
-
-        // 32-target tiles are handed out in order by a counter (stats[3], zeroed with the
-        // statistics at every build), so warps that drew cheap tiles take more of them
-        auto next_tile = [&]() {
-            unsigned long long t = 0;
-            if (lane == 0)
-                t = atomicAdd(&stats[3], 1ull);
-            return static_cast<int>(__shfl_sync(0xffffffffu, t, 0));
-        };
-        for (int tile = next_tile(); static_cast<long long>(tile) * 32 < n; tile = next_tile())
-        {
-            const int k = tile * 32 + lane;
-            const bool valid = k < n;
-            const float4 me = spm[valid ? k : n - 1];
-            const float rad = srad[valid ? k : n - 1];
-            const float lim = (LAW == NBODY_LAW_CUTOFF) ? rad * rad : eps2;
-            float ax = 0.f, ay = 0.f, az = 0.f;
-            const unsigned valid_mask = __ballot_sync(0xffffffffu, valid);
-            if (lane == 0)
-                stk[warp][0] = make_int2(0, static_cast<int>(valid_mask));
-            int sp = 1;
-            __syncwarp();
-            // Each cell is reached from its one parent, so a warp pops at most one entry
-            // per cell (< n). The bound only trips on a malformed tree: it records the
-            // error and stops this warp instead of spinning.
-            int guard = 0;
-            const int guard_limit = n + 64;
-            while (sp > 0)
-            {
-                if (++guard > guard_limit)
-                {
-                    if (lane == 0)
-                        atomicOr(err, DEV_ERR_BOUNDS);
-                    break;
-                }
-                --sp;
-                const int2 top = stk[warp][sp];
-                __syncwarp();
-                const int nd = top.x;
-                const unsigned mask = static_cast<unsigned>(top.y);
-                ++visits;
-                const OctNode* cell = nodes + nd;
-                // the three loads of a visit issue together: centre of mass + mass;
-                // open_r2, nchild, first, last; this lane's child slot
-                const float4 cm = cell->com_mass;
-                const int4 meta = *reinterpret_cast<const int4*>(&cell->open_r2);
-                const int cslot = cell->child[lane & 7];
-                if (cm.w == 0.f)
-                    continue;       // bhtree.cpp:109-113: empty nodes are skipped
-                const bool in = (mask >> lane) & 1u;
-                // bhtree.cpp:117-125, evaluated in the reference's operation order
-                const float dx = __fsub_rn(cm.x, me.x), dy = __fsub_rn(cm.y, me.y), dz = __fsub_rn(cm.z, me.z);
-                const float dist_sq = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-                const bool accept = in && dist_sq > __int_as_float(meta.x);
-                if (accept)
-                {
-                    apply<LAW>(me.x, me.y, me.z, lim, cm.x, cm.y, cm.z, cm.w, ax, ay, az);
-                    ++inter;
-                }
-                const unsigned open = mask & ~__ballot_sync(0xffffffffu, accept);
-                if (!open)
-                    continue;
-                const bool mine = (open >> lane) & 1u;
-                const int nchild = meta.y;
-                if (nchild < 0)
-                {
-                    for (int b = meta.z; b <= meta.w; ++b)
-                    {
-                        const float4 s = spm[b];
-                        if (mine)
-                        {
-                            apply<LAW>(me.x, me.y, me.z, lim, s.x, s.y, s.z, s.w, ax, ay, az);
-                            ++inter;
-                        }
-                    }
-                    continue;
-                }
-                const int c = lane < nchild ? cslot : 0;
-                const bool is_cell = lane < nchild && c >= 0;
-                const bool is_leaf = lane < nchild && c < 0;
-                // each child lane fetches its own leaf body, so the leaf loop below only
-                // broadcasts registers
-                const float4 leaf = is_leaf ? spm[~c] : make_float4(0.f, 0.f, 0.f, 0.f);
-                const unsigned cells = __ballot_sync(0xffffffffu, is_cell);
-                unsigned leaves = __ballot_sync(0xffffffffu, is_leaf && leaf.w != 0.f);
-                if (is_cell)
-                {
-                    const int at = sp + __popc(cells & lt);
-                    if (at < kStack)
-                        stk[warp][at] = make_int2(c, static_cast<int>(open));
-                    else
-                        atomicOr(err, DEV_ERR_BOUNDS);
-                }
-                sp = min(kStack, sp + __popc(cells));
-                __syncwarp();
-                while (leaves)
-                {
-                    const int l = __ffs(leaves) - 1;
-                    leaves &= leaves - 1;
-                    const float sx = __shfl_sync(0xffffffffu, leaf.x, l);
-                    const float sy = __shfl_sync(0xffffffffu, leaf.y, l);
-                    const float sz = __shfl_sync(0xffffffffu, leaf.z, l);
-                    const float sw = __shfl_sync(0xffffffffu, leaf.w, l);
-                    if (mine)
-                    {
-                        apply<LAW>(me.x, me.y, me.z, lim, sx, sy, sz, sw, ax, ay, az);
-                        ++inter;
-                    }
-                }
-            }
-            if (valid)
-            {
-                const uint32_t i = order[k];
-                if (body_out)
-                {
-                    float* o = body_out + static_cast<size_t>(i) * 12 + 8;
-                    o[0] = G * ax;
-                    o[1] = G * ay;
-                    o[2] = G * az;
-                }
-                else
-                    acc[i] = make_float4(G * ax, G * ay, G * az, 0.f);
-            }
-        }
-        // per-warp totals
-        unsigned long long total = inter;
-        for (int o = 16; o > 0; o >>= 1)
-            total += __shfl_down_sync(0xffffffffu, total, o);
-        if (lane == 0)
-        {
-            atomicAdd(&stats[0], total);
-            atomicAdd(&stats[1], static_cast<unsigned long long>(visits));
-        }
     }
 
     // Two targets per lane: the packed form of apply(). Both halves run the scalar
@@ -1339,26 +1195,135 @@ namespace nbg
         az = fma2(dz, sc, az);
     }
 
-    // The walk of traverse_kernel for 64 Q Morton-consecutive targets per warp: lane l holds
-    // targets 64 Q t + 32 h + l for h < 2Q, as Q packed pairs (halves 2p and 2p + 1), and a
-    // stack entry carries one lane mask per target slot h. Each target still decides every
-    // node itself with the reference test, and its accepted nodes come in the same
-    // depth-first order, so its sum is the one traverse_kernel forms; one walk now serves
-    // 2Q times the targets and every interaction is a packed pair.
-    template <int LAW, int Q>
-    __global__ void __launch_bounds__(pair_warps(Q) * 32, 2 * kTravWarps / pair_warps(Q)) traverse_pairs_kernel(
+    // The bounding boxes of a warp's targets, split into NSG runs at the NSG - 1 largest Morton
+    // jumps between neighbours (lane l holds targets 32 h + l, h < H, of the nvalid ones from
+    // t0): run[h] is the run of the lane's target h, and lo / hi receive, on every lane, the box
+    // of run `mine` (an empty run's box is inverted, +inf to -inf).
+    template <int H, int NSG>
+    __device__ __forceinline__ void run_boxes(const uint64_t* __restrict__ codes, const int t0, const int nvalid,
+                                              const int lane, const float3 (&pos)[H], const int mine, int (&run)[H],
+                                              float3& lo, float3& hi)
+    {
+        unsigned key[H];    // (common prefix bits << 8 | position); 0xffffffff: no boundary
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+        {
+            const int b = 32 * h + lane;        // boundary between positions b - 1 and b
+            key[h] = 0xffffffffu;
+            if (b > 0 && b < nvalid)
+                key[h] = (static_cast<unsigned>(__clzll(static_cast<long long>(codes[t0 + b - 1] ^ codes[t0 + b]))) << 8)
+                         | static_cast<unsigned>(b);
+            run[h] = 0;
+        }
+#pragma unroll
+        for (int s = 0; s < NSG - 1; ++s)
+        {
+            unsigned m = key[0];
+#pragma unroll
+            for (int h = 1; h < H; ++h)
+                m = min(m, key[h]);
+            m = __reduce_min_sync(0xffffffffu, m);
+            const int split = m == 0xffffffffu ? 32 * H : static_cast<int>(m & 0xffu);
+#pragma unroll
+            for (int h = 0; h < H; ++h)
+            {
+                run[h] += 32 * h + lane >= split ? 1 : 0;
+                if (key[h] == m)
+                    key[h] = 0xffffffffu;
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < NSG; ++g)
+        {
+            float3 l = make_float3(INFINITY, INFINITY, INFINITY), u = make_float3(-INFINITY, -INFINITY, -INFINITY);
+#pragma unroll
+            for (int h = 0; h < H; ++h)
+                if (32 * h + lane < nvalid && run[h] == g)
+                {
+                    l = make_float3(fminf(l.x, pos[h].x), fminf(l.y, pos[h].y), fminf(l.z, pos[h].z));
+                    u = make_float3(fmaxf(u.x, pos[h].x), fmaxf(u.y, pos[h].y), fmaxf(u.z, pos[h].z));
+                }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                l.x = fminf(l.x, __shfl_xor_sync(0xffffffffu, l.x, o));
+                l.y = fminf(l.y, __shfl_xor_sync(0xffffffffu, l.y, o));
+                l.z = fminf(l.z, __shfl_xor_sync(0xffffffffu, l.z, o));
+                u.x = fmaxf(u.x, __shfl_xor_sync(0xffffffffu, u.x, o));
+                u.y = fmaxf(u.y, __shfl_xor_sync(0xffffffffu, u.y, o));
+                u.z = fmaxf(u.z, __shfl_xor_sync(0xffffffffu, u.z, o));
+            }
+            if (g == mine)
+            {
+                lo = l;
+                hi = u;
+            }
+        }
+    }
+
+    // Who takes the (up to eight) sources of a cell's children: H bits per source.
+    template <int H>
+    struct TakeBits
+    {
+        using Word = typename std::conditional<(H > 4), uint64_t, uint32_t>::type;
+        static constexpr Word kOnes = H == 8 ? Word(0x0101010101010101ull) : (H == 4 ? Word(0x11111111u)
+                                      : (H == 2 ? Word(0x5555u) : Word(0xffu)));   // the first bit of each
+        static __device__ __forceinline__ Word first(const int n)      // the bits of the first n sources
+        {
+            return n * H >= 8 * static_cast<int>(sizeof(Word)) ? ~Word(0) : (Word(1) << (n * H)) - 1;
+        }
+        static __device__ __forceinline__ unsigned count(const Word w)
+        {
+            return H > 4 ? __popcll(w) : __popc(static_cast<unsigned>(w));
+        }
+    };
+
+    // |d|^2 in the reference's operation order (bhtree.cpp:117-125), every operation rounded on
+    // its own
+    __device__ __forceinline__ float dist2_rn(const float dx, const float dy, const float dz)
+    {
+        return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+    }
+
+    // The per-target walk for 32 H Morton-consecutive targets per warp: lane l holds targets
+    // 32 H t + 32 h + l for h < H, as packed pairs (2p, 2p + 1) when H > 1. Every target sums
+    // exactly the nodes that the reference's test accepts for it.
+    //
+    // The walk opens one cell at a time, for the targets that opened it, and decides most of
+    // its up to eight children for the whole warp at once: lane l tests child l % 8 against
+    // the bounding box of run l / 8 of the targets. The nearest point of a box gives the least
+    // distance any of its targets can have, the farthest corner the greatest -- exactly, in the
+    // very roundings of the targets' own test, since each operation of it is monotone in the
+    // distance per axis. A child beyond its opening distance of every run's nearest point is
+    // taken by all who opened the parent; one within it of every run's farthest corner is
+    // opened by all of them; only the others are tested target by target.
+    //
+    // The order of a target's sum: at each cell it opens, the leaves, then the children it
+    // takes, both in child order; then the children it opens, the last first, each with its
+    // subtree. That depends on the target alone, not on the others of its warp, so every H
+    // gives the same bits.
+    //
+    // Bound by instruction issue and the latency of its short chains (IPC 2.6 of 4 at a million
+    // bodies). The walk before it popped one cell at a time and tested all the warp's targets
+    // against it. Walk alone, before and now: 4M disk + halo bodies, theta 0.5: 1.45 -> 1.00 ms,
+    // theta 2: 22.5 -> 16.8 ms; a 1M-body disk under the cutoff law, theta 0.5:
+    // 0.256 -> 0.197 ms; two Plummer spheres of 10,000 bodies, theta 0.5: 70 -> 41 us.
+    template <int LAW, int H>
+    __global__ void __launch_bounds__(trav_warps(H) * 32, trav_ctas(H)) traverse_kernel(
         const OctNode* __restrict__ nodes, const float4* __restrict__ spm, const float* __restrict__ srad,
-        const uint32_t* __restrict__ order, const int n, const float G, const float eps2,
-        float4* __restrict__ acc, float* __restrict__ body_out, unsigned* __restrict__ err,
+        const uint64_t* __restrict__ codes, const uint32_t* __restrict__ order, const int n, const float G,
+        const float eps2, float4* __restrict__ acc, float* __restrict__ body_out, unsigned* __restrict__ err,
         unsigned long long* __restrict__ stats)
     {
-        constexpr int H = 2 * Q;                    // target slots per lane
-        constexpr int TW = 32 * H;                  // targets per warp walk
-        constexpr int W = pair_warps(Q);
-        __shared__ int stk_cell[W][kStack];
-        __shared__ unsigned stk_mask[W][kStack][H];     // lanes of each slot that opened it
+        using Takes = typename TakeBits<H>::Word;
+        constexpr int P = (H + 1) / 2;              // target pairs per lane (H = 1: one scalar target)
+        constexpr int TW = 32 * H;                  // targets per warp
+        constexpr int W = trav_warps(H);
+        __shared__ float4 src_mem[W][8];            // the children's (com, mass), or a leaf's (x, m)
+        __shared__ int stk_cell[W][kStack];         // cells to be opened
+        __shared__ uint8_t stk_mine[W][kStack][32]; // by which of each lane's targets, a bit per slot
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const unsigned lt = (1u << lane) - 1u;
+        float4* const srcs = src_mem[warp];
         unsigned inter = 0, visits = 0;
 
         // tiles are handed out in order by a counter (stats[3], zeroed with the statistics at
@@ -1372,195 +1337,274 @@ namespace nbg
         };
         for (int tile = next_tile(); static_cast<long long>(tile) * TW < n; tile = next_tile())
         {
-            float2 npx[Q], npy[Q], npz[Q], lim[Q], ax[Q], ay[Q], az[Q];
-            unsigned m0[H];
-#pragma unroll
-            for (int q = 0; q < Q; ++q)
+            const int t0 = tile * TW;
+            const int nvalid = static_cast<int>(min(static_cast<long long>(TW), static_cast<long long>(n) - t0));
+            float2 npx[P], npy[P], npz[P], lim[P], ax[P], ay[P], az[P];     // negated positions
+            float3 lo, hi;      // the box of run lane / 8
+            unsigned runs = 0;  // the run of the lane's target h, in bits 4 h
             {
-                float v[2][4];
+                float3 pos[H];
+                int run[H];
+                bool finite = true;
 #pragma unroll
-                for (int e = 0; e < 2; ++e)
+                for (int p = 0; p < P; ++p)
                 {
-                    const int k = tile * TW + (2 * q + e) * 32 + lane;
-                    const bool valid = k < n;
-                    m0[2 * q + e] = __ballot_sync(0xffffffffu, valid);
-                    const float4 pk = spm[valid ? k : n - 1];
-                    v[e][0] = -pk.x;
-                    v[e][1] = -pk.y;
-                    v[e][2] = -pk.z;
-                    if (LAW == NBODY_LAW_CUTOFF)
+                    float v[2][4];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
                     {
-                        const float r = srad[valid ? k : n - 1];
-                        v[e][3] = r * r;
+                        const int h = 2 * p + e < H ? 2 * p + e : H - 1;
+                        const int k = min(t0 + 32 * h + lane, n - 1);
+                        const float4 pk = spm[k];
+                        pos[h] = make_float3(pk.x, pk.y, pk.z);
+                        finite = finite && isfinite(pk.x) && isfinite(pk.y) && isfinite(pk.z);
+                        v[e][0] = -pk.x;
+                        v[e][1] = -pk.y;
+                        v[e][2] = -pk.z;
+                        const float r = LAW == NBODY_LAW_CUTOFF ? srad[k] : 0.f;
+                        v[e][3] = LAW == NBODY_LAW_CUTOFF ? r * r : eps2;
                     }
-                    else
-                        v[e][3] = eps2;
+                    npx[p] = make_float2(v[0][0], v[1][0]);
+                    npy[p] = make_float2(v[0][1], v[1][1]);
+                    npz[p] = make_float2(v[0][2], v[1][2]);
+                    lim[p] = make_float2(v[0][3], v[1][3]);
+                    ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
                 }
-                npx[q] = make_float2(v[0][0], v[1][0]);
-                npy[q] = make_float2(v[0][1], v[1][1]);
-                npz[q] = make_float2(v[0][2], v[1][2]);
-                lim[q] = make_float2(v[0][3], v[1][3]);
-                ax[q] = ay[q] = az[q] = make_float2(0.f, 0.f);
-            }
-            if (lane == 0)
-            {
-                stk_cell[warp][0] = 0;
+                run_boxes<H, kRuns>(codes, t0, nvalid, lane, pos, lane >> 3, run, lo, hi);
+                if (!__all_sync(0xffffffffu, finite))
+                {
+                    // min and max pass over a NaN: a box that decides nothing, so that every
+                    // target decides for itself
+                    lo = make_float3(-INFINITY, -INFINITY, -INFINITY);
+                    hi = make_float3(INFINITY, INFINITY, INFINITY);
+                }
 #pragma unroll
                 for (int h = 0; h < H; ++h)
-                    stk_mask[warp][0][h] = m0[h];
+                    runs |= static_cast<unsigned>(run[h]) << (4 * h);
             }
-            int sp = 1;
-            __syncwarp();
-            // Each cell is reached from its one parent, so a warp pops at most one entry
-            // per cell (< n). The bound only trips on a malformed tree: it records the
-            // error and stops this warp instead of spinning.
+            // the lane's targets that opened the cell at hand, one bit per slot h; at first all, for
+            // a parent of the root
+            unsigned all = 0;
+#pragma unroll
+            for (int h = 0; h < H; ++h)
+                all |= 32 * h + lane < nvalid ? 1u << h : 0u;
+            unsigned mine = all;
+            bool full = true;               // all of the warp's targets
+            int sp = 0;
+            int kid = 0, nchild = 1;        // the lane's child l % 8 of the cell at hand: at first the root
+            int next = 0, last = -1;        // bodies of the bucket at hand (identical codes) still to come
+            // Each cell is opened at most once, from its one parent (cells < n). The bound only
+            // trips on a malformed tree: it records the error and ends this tile.
             int guard = 0;
             const int guard_limit = n + 64;
-            while (sp > 0)
+            for (;;)
             {
-                if (++guard > guard_limit)
+                // --- the children of the cell at hand ---
+                // runs that are empty, or have no target among those that opened it, decide nothing
+                bool idle = lo.x > hi.x;
+                if (!full)
+                {
+                    unsigned active = 0;
+#pragma unroll
+                    for (int h = 0; h < H; ++h)
+                        active |= (mine >> h) & 1u ? 1u << ((runs >> (4 * h)) & 7u) : 0u;
+                    active = __reduce_or_sync(0xffffffffu, active);     // every lane's, idle or not
+                    idle = idle || !((active >> (lane >> 3)) & 1u);
+                }
+                const bool has = (lane & 7) < nchild;
+                float4 src = make_float4(0.f, 0.f, 0.f, 0.f);
+                float open_r2 = 0.f;
+                if (has)
+                {
+                    src = kid < 0 ? spm[~kid] : nodes[kid].com_mass;
+                    open_r2 = kid < 0 ? 0.f : nodes[kid].open_r2;
+                }
+                const float ax0 = __fsub_rn(lo.x, src.x), ax1 = __fsub_rn(src.x, hi.x);
+                const float ay0 = __fsub_rn(lo.y, src.y), ay1 = __fsub_rn(src.y, hi.y);
+                const float az0 = __fsub_rn(lo.z, src.z), az1 = __fsub_rn(src.z, hi.z);
+                const float near2 = dist2_rn(fmaxf(fmaxf(ax0, ax1), 0.f), fmaxf(fmaxf(ay0, ay1), 0.f),
+                                             fmaxf(fmaxf(az0, az1), 0.f));
+                const float far2 = dist2_rn(fmaxf(fabsf(ax0), fabsf(ax1)), fmaxf(fabsf(ay0), fabsf(ay1)),
+                                            fmaxf(fabsf(az0), fabsf(az1)));
+                unsigned beyond = __ballot_sync(0xffffffffu, idle || near2 > open_r2);
+                unsigned within = __ballot_sync(0xffffffffu, idle || !(far2 > open_r2));
+                unsigned cells = __ballot_sync(0xffffffffu, has && kid >= 0) & 0xffu;
+                // a source that is not finite (or a target: its tile's boxes are not), by far2 of run
+                // 0, which is never empty
+                const bool odd = (__ballot_sync(0xffffffffu, !(far2 < INFINITY)) & 0xffu) != 0u;
+                // massless nodes are skipped (bhtree.cpp:109-113)
+                const unsigned mass = __ballot_sync(0xffffffffu, src.w != 0.f) & 0xffu;
+                beyond &= beyond >> 16;
+                beyond &= beyond >> 8;
+                within &= within >> 16;
+                within &= within >> 8;
+                // the children that are applied, in the order of the sums: leaves, then cells taken
+                // or tested
+                const unsigned leaves = mass & ~cells;
+                visits += static_cast<unsigned>(__popc(cells));
+                cells &= mass;
+                unsigned push = cells & within & ~beyond;
+                const unsigned tested = cells & ~beyond & ~within;
+                const unsigned applied = cells & ~push;
+                const int nleaf = __popc(leaves), count = nleaf + __popc(applied);
+                const unsigned below = (1u << (lane & 7)) - 1u;
+                const int at = kid < 0 ? __popc(leaves & below) : nleaf + __popc(applied & below);
+                if (lane < 8 && ((leaves | applied) >> lane) & 1u)
+                    srcs[at] = src;
+                __syncwarp();
+                // who takes each of them: H bits per source, all who opened the parent unless tested
+                Takes takes = static_cast<Takes>(mine) * TakeBits<H>::kOnes;
+                Takes opens = 0;            // who opens each tested child
+                for (unsigned t = tested; t; t &= t - 1)
+                {
+                    const int b = __ffs(t) - 1, e = __shfl_sync(0xffffffffu, at, b);
+                    const float r2 = __shfl_sync(0xffffffffu, open_r2, b);
+                    const float4 s = srcs[e];
+                    unsigned take = 0;
+                    if (H == 1)
+                        take = dist2_rn(__fadd_rn(s.x, npx[0].x), __fadd_rn(s.y, npy[0].x), __fadd_rn(s.z, npz[0].x)) > r2
+                                   ? 1u : 0u;
+                    else
+                    {
+#pragma unroll
+                        for (int p = 0; p < P; ++p)
+                        {
+                            // sq2 forms the squares so that none is contracted into the sum
+                            const float2 dx = add2(f2(s.x), npx[p]), dy = add2(f2(s.y), npy[p]), dz = add2(f2(s.z), npz[p]);
+                            const float2 ds = add2(add2(sq2(dx), sq2(dy)), sq2(dz));
+                            take |= (ds.x > r2 ? 1u : 0u) << (2 * p) | (ds.y > r2 ? 2u : 0u) << (2 * p);
+                        }
+                    }
+                    const unsigned rest = mine & ~take;
+                    takes &= ~(static_cast<Takes>(rest) << (H * e));
+                    opens |= static_cast<Takes>(rest) << (H * b);
+                    push |= __any_sync(0xffffffffu, rest != 0u) ? 1u << b : 0u;
+                }
+                takes &= TakeBits<H>::first(count);
+                inter += TakeBits<H>::count(takes);
+                if (odd)
+                {
+                    // one target at a time: zero times an infinity, in the half of a pair that
+                    // does not take the source, is not zero
+                    for (int e = 0; e < count; ++e)
+                    {
+                        const float4 s = srcs[e];
+#pragma unroll
+                        for (int h = 0; h < H; ++h)
+                            if ((takes >> (H * e + h)) & 1u)
+                            {
+                                const int p = h / 2;
+                                apply<LAW>(-(h & 1 ? npx[p].y : npx[p].x), -(h & 1 ? npy[p].y : npy[p].x),
+                                           -(h & 1 ? npz[p].y : npz[p].x), h & 1 ? lim[p].y : lim[p].x, s.x, s.y, s.z,
+                                           s.w, true, h & 1 ? ax[p].y : ax[p].x, h & 1 ? ay[p].y : ay[p].x,
+                                           h & 1 ? az[p].y : az[p].x);
+                            }
+                    }
+                }
+                else if (full && !tested)
+                {
+#pragma unroll 4
+                    for (int e = 0; e < count; ++e)
+                    {
+                        const float4 s = srcs[e];
+                        if (H == 1)
+                            apply<LAW>(-npx[0].x, -npy[0].x, -npz[0].x, lim[0].x, s.x, s.y, s.z, s.w, true, ax[0].x,
+                                       ay[0].x, az[0].x);
+                        else
+#pragma unroll
+                            for (int p = 0; p < P; ++p)
+                                apply2<LAW>(npx[p], npy[p], npz[p], lim[p], s.x, s.y, s.z, s.w, true, true, ax[p],
+                                            ay[p], az[p]);
+                    }
+                }
+                else
+                {
+                    // pair by pair: the lanes that take nothing with either target sit out the loop
+#pragma unroll
+                    for (int p = 0; p < P; ++p)
+                    {
+                        Takes t = takes >> (2 * p);
+                        if (t & (H == 1 ? TakeBits<H>::kOnes : static_cast<Takes>(3 * TakeBits<H>::kOnes)))
+#pragma unroll 4
+                            for (int e = 0; e < count; ++e, t >>= H)
+                            {
+                                const float4 s = srcs[e];
+                                if (H == 1)
+                                    apply<LAW>(-npx[0].x, -npy[0].x, -npz[0].x, lim[0].x, s.x, s.y, s.z, s.w, t & 1u,
+                                               ax[0].x, ay[0].x, az[0].x);
+                                else
+                                    apply2<LAW>(npx[p], npy[p], npz[p], lim[p], s.x, s.y, s.z, s.w, t & 1u, t & 2u,
+                                                ax[p], ay[p], az[p]);
+                            }
+                    }
+                }
+                __syncwarp();               // the sources, and the entry popped last, have been read
+                if (sp + 8 > kStack)
                 {
                     if (lane == 0)
                         atomicOr(err, DEV_ERR_BOUNDS);
                     break;
                 }
-                --sp;
-                const int nd = stk_cell[warp][sp];
-                unsigned mask[H];
-#pragma unroll
-                for (int h = 0; h < H; ++h)
-                    mask[h] = stk_mask[warp][sp][h];
+                for (unsigned t = push; t; t &= t - 1)
+                {
+                    const int b = __ffs(t) - 1;
+                    const unsigned by = (tested >> b) & 1u ? static_cast<unsigned>(opens >> (H * b)) : mine;
+                    stk_mine[warp][sp][lane] = static_cast<uint8_t>(by & ((1u << H) - 1u));
+                    if (lane == b)
+                        stk_cell[warp][sp] = kid;
+                    ++sp;
+                }
                 __syncwarp();
-                ++visits;
-                const OctNode* cell = nodes + nd;
-                const float4 cm = cell->com_mass;
-                const int4 meta = *reinterpret_cast<const int4*>(&cell->open_r2);
-                const int cslot = cell->child[lane & 7];
-                if (cm.w == 0.f)
-                    continue;       // bhtree.cpp:109-113: empty nodes are skipped
-                const float open_r2 = __int_as_float(meta.x);
-                bool take[H];
-                unsigned open_any = 0;
-                unsigned open[H];
-#pragma unroll
-                for (int q = 0; q < Q; ++q)
+                // --- the next cell to be opened, or eight more bodies of a bucket ---
+                if (next > last)
                 {
-                    // bhtree.cpp:117-125, evaluated in the reference's operation order with
-                    // every operation rounded on its own (packed, two targets at a time). A
-                    // contracted multiply-add has one rounding less, which flips borderline
-                    // acceptances; sq2 forms the squares so that none can be contracted.
-                    const float2 dx = add2(f2(cm.x), npx[q]), dy = add2(f2(cm.y), npy[q]), dz = add2(f2(cm.z), npz[q]);
-                    const float2 ds = add2(add2(sq2(dx), sq2(dy)), sq2(dz));
-                    const float ds0 = ds.x, ds1 = ds.y;
-                    take[2 * q] = ((mask[2 * q] >> lane) & 1u) && ds0 > open_r2;
-                    take[2 * q + 1] = ((mask[2 * q + 1] >> lane) & 1u) && ds1 > open_r2;
-                    if (take[2 * q] || take[2 * q + 1])
+                    if (sp == 0)
+                        break;
+                    if (++guard > guard_limit)
                     {
-                        apply2<LAW>(npx[q], npy[q], npz[q], lim[q], cm.x, cm.y, cm.z, cm.w, take[2 * q],
-                                    take[2 * q + 1], ax[q], ay[q], az[q]);
-                        inter += static_cast<unsigned>(take[2 * q]) + static_cast<unsigned>(take[2 * q + 1]);
+                        if (lane == 0)
+                            atomicOr(err, DEV_ERR_BOUNDS);
+                        break;
+                    }
+                    --sp;
+                    const OctNode* const node = nodes + stk_cell[warp][sp];
+                    const int4 meta = *reinterpret_cast<const int4*>(&node->open_r2);   // open_r2, nchild, first, last
+                    kid = node->child[lane & 7];
+                    mine = stk_mine[warp][sp][lane];
+                    full = __all_sync(0xffffffffu, mine == all);
+                    nchild = meta.y;
+                    if (nchild < 0)
+                    {
+                        next = meta.z;
+                        last = meta.w;
                     }
                 }
-#pragma unroll
-                for (int h = 0; h < H; ++h)
+                if (next <= last)
                 {
-                    open[h] = mask[h] & ~__ballot_sync(0xffffffffu, take[h]);
-                    open_any |= open[h];
-                }
-                if (!open_any)
-                    continue;
-                bool mine[H], mine_any = false;
-#pragma unroll
-                for (int h = 0; h < H; ++h)
-                {
-                    mine[h] = (open[h] >> lane) & 1u;
-                    mine_any |= mine[h];
-                }
-                const int nchild = meta.y;
-                if (nchild < 0)
-                {
-                    for (int b = meta.z; b <= meta.w; ++b)
-                    {
-                        const float4 sb = spm[b];
-                        if (mine_any)
-                        {
-#pragma unroll
-                            for (int q = 0; q < Q; ++q)
-                                if (mine[2 * q] || mine[2 * q + 1])
-                                {
-                                    apply2<LAW>(npx[q], npy[q], npz[q], lim[q], sb.x, sb.y, sb.z, sb.w, mine[2 * q],
-                                                mine[2 * q + 1], ax[q], ay[q], az[q]);
-                                    inter += static_cast<unsigned>(mine[2 * q]) + static_cast<unsigned>(mine[2 * q + 1]);
-                                }
-                        }
-                    }
-                    continue;
-                }
-                const int c = lane < nchild ? cslot : 0;
-                const bool is_cell = lane < nchild && c >= 0;
-                const bool is_leaf = lane < nchild && c < 0;
-                // each child lane fetches its own leaf body, so the leaf loop below only
-                // broadcasts registers
-                const float4 leaf = is_leaf ? spm[~c] : make_float4(0.f, 0.f, 0.f, 0.f);
-                const unsigned cells = __ballot_sync(0xffffffffu, is_cell);
-                unsigned leaves = __ballot_sync(0xffffffffu, is_leaf && leaf.w != 0.f);
-                if (is_cell)
-                {
-                    const int at = sp + __popc(cells & lt);
-                    if (at < kStack)
-                    {
-                        stk_cell[warp][at] = c;
-#pragma unroll
-                        for (int h = 0; h < H; ++h)
-                            stk_mask[warp][at][h] = open[h];
-                    }
-                    else
-                        atomicOr(err, DEV_ERR_BOUNDS);
-                }
-                sp = min(kStack, sp + __popc(cells));
-                __syncwarp();
-                while (leaves)
-                {
-                    const int l = __ffs(leaves) - 1;
-                    leaves &= leaves - 1;
-                    const float sx = __shfl_sync(0xffffffffu, leaf.x, l);
-                    const float sy = __shfl_sync(0xffffffffu, leaf.y, l);
-                    const float sz = __shfl_sync(0xffffffffu, leaf.z, l);
-                    const float sw = __shfl_sync(0xffffffffu, leaf.w, l);
-                    if (mine_any)
-                    {
-#pragma unroll
-                        for (int q = 0; q < Q; ++q)
-                            if (mine[2 * q] || mine[2 * q + 1])
-                            {
-                                apply2<LAW>(npx[q], npy[q], npz[q], lim[q], sx, sy, sz, sw, mine[2 * q], mine[2 * q + 1],
-                                            ax[q], ay[q], az[q]);
-                                inter += static_cast<unsigned>(mine[2 * q]) + static_cast<unsigned>(mine[2 * q + 1]);
-                            }
-                    }
+                    kid = ~(next + (lane & 7));
+                    nchild = min(8, last - next + 1);
+                    next += 8;
                 }
             }
 #pragma unroll
-            for (int q = 0; q < Q; ++q)
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
+            for (int h = 0; h < H; ++h)
+            {
+                const int k = t0 + 32 * h + lane;
+                if (k >= n)
+                    continue;
+                const uint32_t i = order[k];
+                const float2 sx = ax[h / 2], sy = ay[h / 2], sz = az[h / 2];
+                const float gx = G * (h & 1 ? sx.y : sx.x), gy = G * (h & 1 ? sy.y : sy.x), gz = G * (h & 1 ? sz.y : sz.x);
+                if (body_out)
                 {
-                    const int k = tile * TW + (2 * q + e) * 32 + lane;
-                    if (k >= n)
-                        continue;
-                    const uint32_t i = order[k];
-                    const float gx = G * (e ? ax[q].y : ax[q].x), gy = G * (e ? ay[q].y : ay[q].x);
-                    const float gz = G * (e ? az[q].y : az[q].x);
-                    if (body_out)
-                    {
-                        float* o = body_out + static_cast<size_t>(i) * 12 + 8;
-                        o[0] = gx;
-                        o[1] = gy;
-                        o[2] = gz;
-                    }
-                    else
-                        acc[i] = make_float4(gx, gy, gz, 0.f);
+                    float* o = body_out + static_cast<size_t>(i) * 12 + 8;
+                    o[0] = gx;
+                    o[1] = gy;
+                    o[2] = gz;
                 }
+                else
+                    acc[i] = make_float4(gx, gy, gz, 0.f);
+            }
         }
         // per-warp totals
         unsigned long long total = inter;
@@ -2210,67 +2254,47 @@ namespace nbg
             const cudaError_t eg = cudaGetLastError();
             return eg == cudaSuccess ? NBODY_OK : ctx_cuda_fail(ctx, eg, "group tree walk");
         }
-        // Targets per warp walk: 128 (traverse_pairs_kernel, 4 per lane) while the tiles
-        // outnumber the resident warps, then 64 (2 per lane) while they are at least half of
-        // them, then 32 (traverse_kernel): a narrower walk visits more cells but keeps more
-        // warps busy. At 262,144 bodies the 64-target walk is 9 % faster than the 128 one.
-        // NBODY_CUDA_BH_TARGETS (32, 64, 128 or 256) overrides; all give the same sums.
+        // Targets per warp: 128 once there are three such tiles a resident warp, 64 once there is
+        // one, else 32. A wider walk opens fewer cells in all but leaves fewer tiles to balance,
+        // and each takes longer. Walk in ms at 32 / 64 / 128 targets: 20,000 bodies (two Plummer
+        // spheres), theta 2: 0.47 / 0.70 / 1.05; 262,144: 1.60 / 1.59 / 1.62, theta 0.5: 0.086 /
+        // 0.088 / 0.113; 1M disk, theta 0.5: 0.213 / 0.197 / 0.244; 4M disk + halo, theta 2:
+        // 24.9 / 17.6 / 16.8. NBODY_CUDA_BH_TARGETS (32, 64, 128 or 256) overrides; all give the
+        // same sums.
         const char* tsel = std::getenv("NBODY_CUDA_BH_TARGETS");
-        int per_warp = tsel ? std::atoi(tsel) : 0;
+        const int per_warp = tsel ? std::atoi(tsel) : 0;
+        const bool soft = p->law == NBODY_LAW_SOFTENED;
+        using Walk = void (*)(const OctNode*, const float4*, const float*, const uint64_t*, const uint32_t*, int,
+                              float, float, float4*, float*, unsigned*, unsigned long long*);
+        // targets per warp 32, 64, 128, 256
+        const Walk fns[4] = {
+            soft ? traverse_kernel<NBODY_LAW_SOFTENED, 1> : traverse_kernel<NBODY_LAW_CUTOFF, 1>,
+            soft ? traverse_kernel<NBODY_LAW_SOFTENED, 2> : traverse_kernel<NBODY_LAW_CUTOFF, 2>,
+            soft ? traverse_kernel<NBODY_LAW_SOFTENED, 4> : traverse_kernel<NBODY_LAW_CUTOFF, 4>,
+            soft ? traverse_kernel<NBODY_LAW_SOFTENED, 8> : traverse_kernel<NBODY_LAW_CUTOFF, 8>,
+        };
+        auto per_sm = [&](const int i) {
+            int per = 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fns[i], trav_warps(1 << i) * 32, 0) != cudaSuccess || per < 1)
+                per = 1;
+            return per;
+        };
+        int fi = 0;
+        while (fi < 3 && per_warp > (32 << fi))
+            ++fi;
         if (!per_warp)
         {
-            auto resident_warps = [&](auto fn) {
-                int per = 0;
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kTravWarps * 32, 0) != cudaSuccess || per < 1)
-                    per = 1;
-                return static_cast<long long>(per) * sms * kTravWarps;
-            };
-            const bool soft = p->law == NBODY_LAW_SOFTENED;
-            const long long w128 = resident_warps(soft ? traverse_pairs_kernel<NBODY_LAW_SOFTENED, 2>
-                                                       : traverse_pairs_kernel<NBODY_LAW_CUTOFF, 2>);
-            const long long w64 = resident_warps(soft ? traverse_pairs_kernel<NBODY_LAW_SOFTENED, 1>
-                                                      : traverse_pairs_kernel<NBODY_LAW_CUTOFF, 1>);
-            const long long nn = static_cast<long long>(ni);
-            per_warp = nn >= 128 * w128 ? 128 : (2 * nn >= 64 * w64 ? 64 : 32);
+            auto resident = [&](const int i) { return static_cast<long long>(per_sm(i)) * sms * trav_warps(1 << i); };
+            fi = ni >= 3 * 128 * resident(2) ? 2 : (ni >= 64 * resident(1) ? 1 : 0);
         }
-        if (per_warp == 64 || per_warp == 128 || per_warp == 256)
-        {
-            const bool soft = p->law == NBODY_LAW_SOFTENED;
-            using Walk = void (*)(const OctNode*, const float4*, const float*, const uint32_t*, int, float, float,
-                                  float4*, float*, unsigned*, unsigned long long*);
-            Walk fn;
-            int warps = kTravWarps;
-            if (per_warp == 256)
-            {
-                fn = soft ? traverse_pairs_kernel<NBODY_LAW_SOFTENED, 4> : traverse_pairs_kernel<NBODY_LAW_CUTOFF, 4>;
-                warps = pair_warps(4);
-            }
-            else if (per_warp == 128)
-                fn = soft ? traverse_pairs_kernel<NBODY_LAW_SOFTENED, 2> : traverse_pairs_kernel<NBODY_LAW_CUTOFF, 2>;
-            else
-                fn = soft ? traverse_pairs_kernel<NBODY_LAW_SOFTENED, 1> : traverse_pairs_kernel<NBODY_LAW_CUTOFF, 1>;
-            // one resident wave of CTAs, each warp drawing tiles until none are left
-            int per = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, warps * 32, 0) != cudaSuccess || per < 1)
-                per = 1;
-            const int tiles2 = (ni + per_warp - 1) / per_warp;
-            const int grid2 = std::min((tiles2 + warps - 1) / warps, sms * per);
-            fn<<<grid2, warps * 32, 0, s>>>(b.nodes, b.spm, b.srad, b.order, ni, p->G, p->eps2, acc, body_out,
-                                             ctx->dev_error, b.stats);
-            ++ctx->launches;
-            if (timed)
-                b.timed = cudaEventRecord(b.ev[2], s) == cudaSuccess;
-            const cudaError_t e2 = cudaGetLastError();
-            return e2 == cudaSuccess ? NBODY_OK : ctx_cuda_fail(ctx, e2, "tree traversal");
-        }
-        const int tiles = (ni + 31) / 32;
-        const int grid = std::min((tiles + kTravWarps - 1) / kTravWarps, sms * 8);
-        if (p->law == NBODY_LAW_SOFTENED)
-            traverse_kernel<NBODY_LAW_SOFTENED><<<grid, kTravWarps * 32, 0, s>>>(
-                b.nodes, b.spm, b.srad, b.order, ni, p->G, p->eps2, acc, body_out, ctx->dev_error, b.stats);
-        else
-            traverse_kernel<NBODY_LAW_CUTOFF><<<grid, kTravWarps * 32, 0, s>>>(
-                b.nodes, b.spm, b.srad, b.order, ni, p->G, p->eps2, acc, body_out, ctx->dev_error, b.stats);
+        // one resident wave of CTAs, each warp drawing tiles until none are left
+        const int warps = trav_warps(1 << fi);
+        const int tiles = (ni + (32 << fi) - 1) / (32 << fi);
+        int grid = std::min((tiles + warps - 1) / warps, sms * per_sm(fi));
+        if (grid > 3 * sms)
+            grid = grid / sms * sms;    // as many CTAs on every SM
+        fns[fi]<<<grid, warps * 32, 0, s>>>(b.nodes, b.spm, b.srad, b.codes, b.order, ni, p->G, p->eps2, acc, body_out,
+                                            ctx->dev_error, b.stats);
         ++ctx->launches;
         if (timed)
             b.timed = cudaEventRecord(b.ev[2], s) == cudaSuccess;

@@ -610,3 +610,38 @@ def test_bh_softened_config5_sampled(gpu):
         assert np.median(diff) <= 1e-5 and np.mean(diff > 1e-4) <= 0.02, stats
         assert abs(np.median(e_gpu) - np.median(e_ex)) <= 0.05 * np.median(e_ex), stats
         assert abs(np.percentile(e_gpu, 99) - np.percentile(e_ex, 99)) <= 0.05 * np.percentile(e_ex, 99), stats
+
+
+@pytest.mark.parametrize("theta", [0.5, 2.0])
+@pytest.mark.parametrize("n", [2, 3, 5, 31, 33, 35, 63, 65, 67, 127, 129, 131, 259])
+def test_walk_tail_tiles(gpu, n, theta, monkeypatch):
+    """Last tiles with few targets (fewer than the runs of a warp's boxes, one lane of a slot,
+    one slot of several), coincident bodies (a bucket), massless ones and a body that is not a
+    number: every width gives the bits of the 32-target walk and the same interactions, and the
+    finite targets' accelerations are the oracle octree's to the file's bar."""
+    from nbody_gb300 import scenes
+    b = scenes.plummer(n, seed=n)
+    b[:, 3] = np.float32(1e-3)
+    if n > 30:
+        b[7:10, :3] = b[3, :3]
+        b[11, 7] = 0.0
+    kw = dict(theta=theta, law=0, size=0.0, tree_box=1)
+    for nan in (False, True):
+        if nan:
+            b[n - 1, 0] = np.nan
+        out = []
+        for width in ("32", "64", "128", "256", None):
+            if width:
+                monkeypatch.setenv("NBODY_CUDA_BH_TARGETS", width)
+            else:
+                monkeypatch.delenv("NBODY_CUDA_BH_TARGETS")
+            out.append(bh_accel(gpu, b, **kw))
+        for a, s in out[1:]:
+            assert np.array_equal(a.view(np.uint32), out[0][0].view(np.uint32))
+            assert s["interactions"] == out[0][1]["interactions"]
+        if not nan and n <= 30:
+            ref, _ = O.barnes_hut(b, 64.0, theta, 1.0)
+            monkeypatch.setenv("NBODY_CUDA_BH_TARGETS", "32")
+            a, _ = bh_accel(gpu, b, theta=theta, law=0, size=64.0)
+            monkeypatch.delenv("NBODY_CUDA_BH_TARGETS")
+            assert np.all(np.linalg.norm(a - ref[:, 8:11], axis=1) <= TOL * term_scale(b))
