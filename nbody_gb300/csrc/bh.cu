@@ -436,21 +436,6 @@ namespace nbg
         }
     }
 
-    // Copies a full sort's result back into the buffers the build reads, when *run_if is set.
-    __global__ void __launch_bounds__(256) copy_back_kernel(const uint64_t* __restrict__ ks,
-                                                            const uint32_t* __restrict__ vs, uint64_t* __restrict__ kd,
-                                                            uint32_t* __restrict__ vd, const int n,
-                                                            const unsigned* __restrict__ run_if)
-    {
-        if (!*run_if)
-            return;
-        for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256)
-        {
-            kd[i] = ks[i];
-            vd[i] = vs[i];
-        }
-    }
-
     // ------------------------------------------------------------------------------------
     // 4. Morton-ordered copies and the fixed-point cell sums
     // ------------------------------------------------------------------------------------
@@ -2092,23 +2077,15 @@ namespace nbg
         if (n > 1)
         {
             // runs of equal top bits into order; a run too long for that sorts everything
-            // again by all bits, from the current order (its ties are in index order too), and
-            // copies the result back, so that the sorted pairs are where the passes left them
+            // again by all bits, from the current order (its ties are in index order too)
             const int cur = in_alt ? 1 : 0;
             unsigned* full = reinterpret_cast<unsigned*>(b.stats + 4);
             run_sort_kernel<<<ceil_div(n, 256), 256, 0, s>>>(b.keys[cur], b.vals[cur], ni, full);
             ++L;
-            bool alt2 = false;
-            e = radix_sort_pairs(b.keys[cur], b.vals[cur], b.keys[1 - cur], b.vals[1 - cur], n, 0, 63, b.temp, s, &L,
-                                 &alt2, ctx->dev_error, full, (63 - kRunShift + 8) / 9);
+            e = radix_sort_if(b.keys[cur], b.vals[cur], b.keys[1 - cur], b.vals[1 - cur], n, 0, 63, b.temp,
+                              (63 - kRunShift + 8) / 9, s, &L, ctx->dev_error, full);
             if (e != cudaSuccess)
                 return ctx_cuda_fail(ctx, e, "radix sort");
-            if (alt2)
-            {
-                copy_back_kernel<<<1024, 256, 0, s>>>(b.keys[1 - cur], b.vals[1 - cur], b.keys[cur], b.vals[cur], ni,
-                                                         full);
-                ++L;
-            }
         }
         const uint64_t* keys = b.keys[in_alt ? 1 : 0];
         const uint32_t* order = b.vals[in_alt ? 1 : 0];

@@ -38,7 +38,7 @@ namespace nbg
         constexpr int kDigits = 1 << kBits;
         constexpr unsigned kMask = kDigits - 1;
         constexpr int kPer = kDigits / kThreads;      // digits per thread in the per-digit steps
-        constexpr int kMaxPasses = 16;      // over the calls that share one set of temporaries
+        constexpr int kMaxPasses = 16;      // of the two sorts that share one set of temporaries
         constexpr int kHistThreads = 1024;
 
         // A tile's published count for one digit: flag in bits 62-63, the pass's epoch
@@ -54,7 +54,7 @@ namespace nbg
 
         struct TempLayout
         {
-            uint32_t* tickets;      // kMaxPasses tile tickets
+            uint32_t* tickets;      // kMaxPasses tile tickets, then the whole sort's barrier count
             uint32_t* ghist;        // kMaxPasses x kDigits global digit counts
             uint64_t* status;       // tiles x kDigits published counts
             size_t zero_bytes;      // everything above is zeroed before a sort
@@ -77,20 +77,16 @@ namespace nbg
         }
     }
 
-    // Histograms of the digits of all passes, in one read of the keys.
-    __global__ void __launch_bounds__(kHistThreads) digit_hist_kernel(const uint64_t* __restrict__ keys, const int n,
-                                                                      const int shift0, const int passes,
-                                                                      uint32_t* __restrict__ ghist,
-                                                                      const unsigned* __restrict__ run_if)
+    // Histograms of the digits of all passes, in one read of the keys by the whole grid; hist
+    // holds passes * kDigits counters of shared memory.
+    __device__ __forceinline__ void histogram(uint32_t* hist, const uint64_t* __restrict__ keys, const int n,
+                                              const int shift0, const int passes, uint32_t* __restrict__ ghist)
     {
-        if (run_if && !*run_if)
-            return;
-        __shared__ uint32_t hist[kMaxPasses * kDigits];
-        for (int d = threadIdx.x; d < passes * kDigits; d += kHistThreads)
+        for (int d = threadIdx.x; d < passes * kDigits; d += blockDim.x)
             hist[d] = 0;
         __syncthreads();
-        const int stride = gridDim.x * kHistThreads;
-        int i = blockIdx.x * kHistThreads + threadIdx.x;
+        const int stride = gridDim.x * blockDim.x;
+        int i = blockIdx.x * blockDim.x + threadIdx.x;
         // four keys in flight per thread
         for (; static_cast<long long>(i) + 3 * stride < n; i += 4 * stride)
         {
@@ -110,9 +106,17 @@ namespace nbg
                 atomicAdd(&hist[p * kDigits + static_cast<int>((k >> (shift0 + p * kBits)) & kMask)], 1u);
         }
         __syncthreads();
-        for (int d = threadIdx.x; d < passes * kDigits; d += kHistThreads)
+        for (int d = threadIdx.x; d < passes * kDigits; d += blockDim.x)
             if (hist[d])
                 atomicAdd(&ghist[d], hist[d]);
+    }
+
+    __global__ void __launch_bounds__(kHistThreads) digit_hist_kernel(const uint64_t* __restrict__ keys, const int n,
+                                                                      const int shift0, const int passes,
+                                                                      uint32_t* __restrict__ ghist)
+    {
+        __shared__ uint32_t hist[kMaxPasses * kDigits];
+        histogram(hist, keys, n, shift0, passes, ghist);
     }
 
     __device__ __forceinline__ uint64_t load_relaxed(const uint64_t* p)
@@ -158,18 +162,23 @@ namespace nbg
         }
     }
 
-    // PERSIST: a CTA takes tiles until none is left (launched with one CTA per resident slot);
-    // otherwise one tile per CTA (launched with one CTA per tile)
-    template <bool PERSIST>
-    __global__ void __launch_bounds__(kThreads, 3) digit_pass_kernel(
-        const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t* __restrict__ keys_out,
-        uint32_t* __restrict__ vals_out, const int n, const int shift, const int pass,
-        const uint32_t* __restrict__ ghist, uint64_t* __restrict__ status, uint32_t* __restrict__ ticket,
-        unsigned* __restrict__ err, const unsigned* __restrict__ run_if)
+    // A load that may be served by L1, or (L2) one that sees what other SMs wrote in this launch.
+    template <bool L2, typename T>
+    __device__ __forceinline__ T fetch(const T* p)
     {
-        if (run_if && !*run_if)
-            return;
-        extern __shared__ __align__(16) unsigned char smem[];
+        return L2 ? __ldcg(p) : *p;
+    }
+
+    // One pass over the tiles that this CTA takes: until none is left when PERSIST, else one.
+    // smem: kPassSmem bytes.
+    template <bool PERSIST>
+    __device__ __forceinline__ void digit_pass(unsigned char* smem, const uint64_t* __restrict__ keys,
+                                               const uint32_t* __restrict__ vals, uint64_t* __restrict__ keys_out,
+                                               uint32_t* __restrict__ vals_out, const int n, const int shift,
+                                               const int pass, const uint32_t* __restrict__ ghist,
+                                               uint64_t* __restrict__ status, uint32_t* __restrict__ ticket,
+                                               unsigned* __restrict__ err)
+    {
         uint64_t* stage_k = reinterpret_cast<uint64_t*>(smem);                     // kTile
         uint32_t* stage_v = reinterpret_cast<uint32_t*>(stage_k + kTile);          // kTile
         uint32_t* warp_cnt2 = stage_v + kTile;                                     // kWarps * kDigits / 2
@@ -204,7 +213,7 @@ namespace nbg
             for (int r = 0; r < kRounds; ++r)
             {
                 const int i = base + r * 32 + lane;
-                key[r] = i < n ? keys[i] : 0ull;
+                key[r] = i < n ? fetch<PERSIST>(&keys[i]) : 0ull;
             }
 #pragma unroll
             for (int r = 0; r < kRounds; ++r)
@@ -258,7 +267,7 @@ namespace nbg
                 block_exclusive(total, start, warp_sum[0]);
 #pragma unroll
                 for (int q = 0; q < kPer; ++q)
-                    gcount[q] = ghist[threadIdx.x * kPer + q];
+                    gcount[q] = fetch<PERSIST>(&ghist[threadIdx.x * kPer + q]);
                 block_exclusive(gcount, gstart, warp_sum[1]);
 #pragma unroll
                 for (int q = 0; q < kPer; ++q)
@@ -279,7 +288,7 @@ namespace nbg
                 const unsigned d = static_cast<unsigned>((key[r] >> shift) & kMask);
                 const uint32_t pos = digit_start[d] + warp_cnt[warp * kDigits + d] + rank[r];
                 stage_k[pos] = key[r];
-                stage_v[pos] = vals[i];
+                stage_v[pos] = fetch<PERSIST>(&vals[i]);
             }
             // decoupled look-back: sum the earlier tiles' counts of each digit, four tiles per
             // step, back to the nearest tile that has published an inclusive count
@@ -357,16 +366,108 @@ namespace nbg
         }
     }
 
+    __global__ void __launch_bounds__(kThreads, 3) digit_pass_kernel(
+        const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t* __restrict__ keys_out,
+        uint32_t* __restrict__ vals_out, const int n, const int shift, const int pass,
+        const uint32_t* __restrict__ ghist, uint64_t* __restrict__ status, uint32_t* __restrict__ ticket,
+        unsigned* __restrict__ err)
+    {
+        extern __shared__ __align__(16) unsigned char smem[];
+        digit_pass<false>(smem, keys, vals, keys_out, vals_out, n, shift, pass, ghist, status, ticket, err);
+    }
+
+    // Every CTA of the grid arrives, then goes on; *count counts arrivals over all barriers and
+    // `upto` is what it reaches here. Every CTA must be resident (a cooperative launch). Returns
+    // false, and records the error, when the wait gives up. What the grid wrote before is read
+    // after it.
+    __device__ __forceinline__ bool grid_barrier(uint32_t* count, const uint32_t upto, unsigned* err)
+    {
+        __shared__ int ok;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            ok = 1;
+            atomicAdd(count, 1u);
+            const uint64_t t0 = globaltimer();
+            while (*reinterpret_cast<volatile uint32_t*>(count) < upto)
+            {
+                if (globaltimer() - t0 > kWaitLimitNs)
+                {
+                    atomicOr(err, DEV_ERR_TIMEOUT);
+                    ok = 0;
+                    break;
+                }
+                __nanosleep(200);
+            }
+            __threadfence();
+        }
+        __syncthreads();
+        return ok != 0;
+    }
+
+    // A whole sort in one launch, when *run_if is set: the histogram and every pass by a grid of
+    // resident CTAs, a grid-wide barrier between them. As nine launches of the kernels above
+    // that return at once when the flag is clear -- the usual case -- it cost a step of 262,144
+    // bodies (a replayed graph) 16 of 250 us more, an eager build 35 of 227. The result ends in keys / vals. Between barriers each buffer is either read
+    // or written, never both; plain loads may find lines of an earlier pass in L1, so the
+    // inputs are read around it (ld.cg).
+    __global__ void __launch_bounds__(kThreads, 3) whole_sort_kernel(
+        uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, const int n, const int begin_bit,
+        const int passes, const int pass_base, uint32_t* ghist, uint64_t* status, uint32_t* tickets,
+        uint32_t* barrier_count, unsigned* err, const unsigned* __restrict__ run_if)
+    {
+        if (!*run_if)
+            return;
+        extern __shared__ __align__(16) unsigned char smem[];
+        histogram(reinterpret_cast<uint32_t*>(smem), keys, n, begin_bit, passes, ghist + pass_base * kDigits);
+        uint32_t upto = 0;
+        for (int p = 0; p < passes; ++p)
+        {
+            if (!grid_barrier(barrier_count, upto += gridDim.x, err))
+                return;
+            const int q = pass_base + p;
+            if (p & 1)
+                digit_pass<true>(smem, keys_alt, vals_alt, keys, vals, n, begin_bit + p * kBits, q, ghist + q * kDigits,
+                                 status, tickets + q, err);
+            else
+                digit_pass<true>(smem, keys, vals, keys_alt, vals_alt, n, begin_bit + p * kBits, q, ghist + q * kDigits,
+                                 status, tickets + q, err);
+        }
+        if (!(passes & 1) || !grid_barrier(barrier_count, upto += gridDim.x, err))
+            return;
+        for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
+        {
+            keys[i] = __ldcg(&keys_alt[i]);
+            vals[i] = __ldcg(&vals_alt[i]);
+        }
+    }
+
     size_t sort_temp_bytes(const size_t n)
     {
         const size_t tiles = (n + kTile - 1) / kTile;
         return zero_bytes(tiles) + 256;
     }
 
+    namespace
+    {
+        int sm_count()
+        {
+            int dev = 0, sms = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            return std::max(1, sms);
+        }
+
+        cudaError_t allow_smem(const void* fn)
+        {
+            return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPassSmem));
+        }
+    }
+
     cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt,
                                  const size_t n, const int begin_bit, const int end_bit, void* temp,
-                                 cudaStream_t stream, uint64_t* launches, bool* in_alt, unsigned* err,
-                                 const unsigned* run_if, const int pass_base)
+                                 cudaStream_t stream, uint64_t* launches, bool* in_alt, unsigned* err)
     {
         *in_alt = false;
         if (n <= 1)
@@ -374,69 +475,72 @@ namespace nbg
         if (n > 0x7fffffffu)
             return cudaErrorInvalidValue;
         const int passes = (end_bit - begin_bit + kBits - 1) / kBits;
-        if (passes < 1 || pass_base < 0 || pass_base + passes > kMaxPasses)
+        if (passes < 1 || passes > kMaxPasses)
             return cudaErrorInvalidValue;
-        static const cudaError_t attr = [] {
-            const cudaError_t a = cudaFuncSetAttribute(digit_pass_kernel<false>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       static_cast<int>(kPassSmem));
-            return a != cudaSuccess ? a
-                                    : cudaFuncSetAttribute(digit_pass_kernel<true>,
-                                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           static_cast<int>(kPassSmem));
-        }();
+        static const cudaError_t attr = allow_smem(reinterpret_cast<const void*>(digit_pass_kernel));
         if (attr != cudaSuccess)
             return attr;
         const int tiles = static_cast<int>((n + kTile - 1) / kTile);
         const TempLayout t = layout(temp, static_cast<size_t>(tiles));
-        // a call that may do nothing (run_if) launches persistent passes, one CTA per
-        // resident slot, so that a pass with nothing to do costs few CTAs; otherwise one CTA
-        // per tile
-        static const int per_sm = [] {
-            int b = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, digit_pass_kernel<true>, kThreads, kPassSmem);
-            return std::max(1, b);
-        }();
-        // the first call zeroes the tickets, histograms and published counts of every pass;
-        // a later call's passes have their own tickets and histograms, and their counts carry
-        // other epochs
-        cudaError_t e = pass_base == 0 ? cudaMemsetAsync(temp, 0, t.zero_bytes, stream) : cudaSuccess;
+        // the tickets, histograms and published counts of every pass, a later sort_if's too
+        cudaError_t e = cudaMemsetAsync(temp, 0, t.zero_bytes, stream);
         if (e != cudaSuccess)
             return e;
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int hist_grid = std::max(1, std::min((static_cast<int>(n) + kHistThreads - 1) / kHistThreads, 2 * sms));
-        const int pass_grid = std::min(tiles, per_sm * sms);
-        digit_hist_kernel<<<hist_grid, kHistThreads, 0, stream>>>(keys, static_cast<int>(n), begin_bit, passes,
-                                                                  t.ghist + pass_base * kDigits, run_if);
+        const int hist_grid = std::max(1, std::min((static_cast<int>(n) + kHistThreads - 1) / kHistThreads, 2 * sm_count()));
+        digit_hist_kernel<<<hist_grid, kHistThreads, 0, stream>>>(keys, static_cast<int>(n), begin_bit, passes, t.ghist);
         ++*launches;
         e = cudaGetLastError();
-        if (e != cudaSuccess)
-            return e;
         uint64_t* kin = keys;
         uint32_t* vin = vals;
         uint64_t* kout = keys_alt;
         uint32_t* vout = vals_alt;
-        for (int p = 0; p < passes; ++p)
+        for (int p = 0; p < passes && e == cudaSuccess; ++p)
         {
-            const int q = pass_base + p;
-            if (run_if)
-                digit_pass_kernel<true><<<pass_grid, kThreads, kPassSmem, stream>>>(
-                    kin, vin, kout, vout, static_cast<int>(n), begin_bit + p * kBits, q, t.ghist + q * kDigits,
-                    t.status, t.tickets + q, err, run_if);
-            else
-                digit_pass_kernel<false><<<tiles, kThreads, kPassSmem, stream>>>(
-                    kin, vin, kout, vout, static_cast<int>(n), begin_bit + p * kBits, q, t.ghist + q * kDigits,
-                    t.status, t.tickets + q, err, run_if);
+            digit_pass_kernel<<<tiles, kThreads, kPassSmem, stream>>>(kin, vin, kout, vout, static_cast<int>(n),
+                                                                      begin_bit + p * kBits, p, t.ghist + p * kDigits,
+                                                                      t.status, t.tickets + p, err);
             ++*launches;
             e = cudaGetLastError();
-            if (e != cudaSuccess)
-                return e;
             std::swap(kin, kout);
             std::swap(vin, vout);
             *in_alt = !*in_alt;
         }
-        return cudaSuccess;
+        return e;
+    }
+
+    cudaError_t radix_sort_if(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, const size_t n,
+                              const int begin_bit, const int end_bit, void* temp, const int pass_base,
+                              cudaStream_t stream, uint64_t* launches, unsigned* err, const unsigned* run_if)
+    {
+        if (n <= 1)
+            return cudaSuccess;
+        if (n > 0x7fffffffu)
+            return cudaErrorInvalidValue;
+        const int passes = (end_bit - begin_bit + kBits - 1) / kBits;
+        if (passes < 1 || pass_base < 0 || pass_base + passes > kMaxPasses)
+            return cudaErrorInvalidValue;
+        static const cudaError_t attr = allow_smem(reinterpret_cast<const void*>(whole_sort_kernel));
+        if (attr != cudaSuccess)
+            return attr;
+        static const int per_sm = [] {
+            int b = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, whole_sort_kernel, kThreads, kPassSmem);
+            return std::max(1, b);
+        }();
+        const int tiles = static_cast<int>((n + kTile - 1) / kTile);
+        const TempLayout t = layout(temp, static_cast<size_t>(tiles));
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(static_cast<unsigned>(std::min(tiles, per_sm * sm_count())));
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = kPassSmem;
+        cfg.stream = stream;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        ++*launches;
+        return cudaLaunchKernelEx(&cfg, whole_sort_kernel, keys, vals, keys_alt, vals_alt, static_cast<int>(n), begin_bit,
+                                  passes, pass_base, t.ghist, t.status, t.tickets, t.tickets + kMaxPasses, err, run_if);
     }
 }
