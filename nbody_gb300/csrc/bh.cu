@@ -94,8 +94,9 @@ namespace nbg
         int2* child = nullptr;          // binary children: >= 0 internal, < 0 ~leaf
         int2* range = nullptr;          // [first, last] of each internal node
         int* prefix = nullptr;          // common-prefix bits of each internal node
-        uint32_t* octflag = nullptr;
-        uint32_t* octidx = nullptr;
+        uint8_t* octflag = nullptr;     // 1 for a binary node that is an octree node
+        uint32_t* octidx = nullptr;     // octree nodes before each binary node; kIsOct set on one
+        uint64_t* numbering = nullptr;  // number_kernel's tile counts (after a ticket word)
         Int64x4* psum = nullptr;        // N + 1 fixed-point sums of {m x, m y, m z, m} over the
                                         // sorted bodies before x within x's cell-sum tile
         OctNode* nodes = nullptr;
@@ -103,6 +104,7 @@ namespace nbg
         size_t temp_bytes = 0;
         BoxParams* box = nullptr;
         float* bbox_part = nullptr;
+        unsigned* box_ticket = nullptr; // blocks that have left their bounds; 0 between builds
         unsigned long long* stats = nullptr;   // [0] interactions, [1] node visits, [2] octree nodes,
                                                // [3] the traversal's tile counter, [4] the Morton
                                                // sort's full-sort flag (as unsigned)
@@ -118,71 +120,6 @@ namespace nbg
     // ------------------------------------------------------------------------------------
     // 1. root box
     // ------------------------------------------------------------------------------------
-    // Per block: the box's min and max per axis, and the largest finite |m| and |x| (over
-    // all axes), which fix the fixed-point scale of the cell sums. Min and max are exact,
-    // so the float fold equals a double one; the partials are widened at the end.
-    __global__ void __launch_bounds__(256) bbox_partial_kernel(const float4* __restrict__ src, const int stride,
-                                                               const int n, float* __restrict__ part)
-    {
-        float v[kBboxVals] = { INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, 0.f, 0.f };
-        auto fold = [&](const float4 p, const float m) {
-            const float x[3] = { p.x, p.y, p.z };
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-            {
-                v[a] = fminf(v[a], x[a]);
-                v[3 + a] = fmaxf(v[3 + a], x[a]);
-                if (isfinite(x[a]))
-                    v[7] = fmaxf(v[7], fabsf(x[a]));
-            }
-            if (isfinite(m))
-                v[6] = fmaxf(v[6], fabsf(m));
-        };
-        const int step = gridDim.x * blockDim.x;
-        int i = blockIdx.x * blockDim.x + threadIdx.x;
-        // four bodies in flight per thread
-        for (; static_cast<long long>(i) + 3 * step < n; i += 4 * step)
-        {
-            float4 p[4];
-            float m[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-            {
-                const size_t k = static_cast<size_t>(i + u * step);
-                p[u] = src[k * stride];
-                m[u] = stride == 3 ? src[k * 3 + 1].w : p[u].w;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                fold(p[u], m[u]);
-        }
-        for (; i < n; i += step)
-        {
-            const float4 p = src[static_cast<size_t>(i) * stride];
-            fold(p, stride == 3 ? src[static_cast<size_t>(i) * 3 + 1].w : p.w);
-        }
-        __shared__ float red[kBboxVals][256];
-#pragma unroll
-        for (int a = 0; a < kBboxVals; ++a)
-            red[a][threadIdx.x] = v[a];
-        __syncthreads();
-        for (int s = blockDim.x / 2; s > 0; s >>= 1)
-        {
-            if (threadIdx.x < s)
-            {
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-                    red[a][threadIdx.x] = fminf(red[a][threadIdx.x], red[a][threadIdx.x + s]);
-#pragma unroll
-                for (int a = 3; a < kBboxVals; ++a)
-                    red[a][threadIdx.x] = fmaxf(red[a][threadIdx.x], red[a][threadIdx.x + s]);
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x < kBboxVals)
-            part[blockIdx.x * kBboxVals + threadIdx.x] = red[threadIdx.x][0];
-    }
-
     // The exponent e with 0 <= v < 2^e for a finite float v >= 0 (v = M 2^(E - 150) with
     // M < 2^24, so v < 2^(E - 126); subnormals and zero lie below 2^-126).
     __device__ __forceinline__ int bound_exp(const float v)
@@ -191,20 +128,18 @@ namespace nbg
         return (E ? static_cast<int>(E) : 1) - 126;
     }
 
-    __global__ void __launch_bounds__(256) box_final_kernel(const float* __restrict__ part, const int nparts,
-                                                            const int n, const int mode, const float size,
-                                                            BoxParams* __restrict__ box)
+    // One block of 256 threads folds the blocks' partials (a strided pass, then a tree), in float:
+    // min and max are exact.
+    __device__ void finish_box(const float* part, const int nparts, const int n, const int mode, const float size,
+                               float (&red)[kBboxVals][256], BoxParams* __restrict__ box)
     {
-        // one block folds the per-block partials (a strided pass, then a tree), in float:
-        // min and max are exact
-        __shared__ float red[kBboxVals][256];
         float v[kBboxVals] = { INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, 0.f, 0.f };
         for (int k = threadIdx.x; k < nparts; k += blockDim.x)
         {
             for (int a = 0; a < 3; ++a)
-                v[a] = fminf(v[a], part[k * kBboxVals + a]);
+                v[a] = fminf(v[a], __ldcg(&part[k * kBboxVals + a]));
             for (int a = 3; a < kBboxVals; ++a)
-                v[a] = fmaxf(v[a], part[k * kBboxVals + a]);
+                v[a] = fmaxf(v[a], __ldcg(&part[k * kBboxVals + a]));
         }
         for (int a = 0; a < kBboxVals; ++a)
             red[a][threadIdx.x] = v[a];
@@ -293,6 +228,95 @@ namespace nbg
         b.exact = exact ? 1 : 0;
         b.edge_f = static_cast<float>(b.edge);
         *box = b;
+    }
+
+    // Per block: the box's min and max per axis, and the largest finite |m| and |x| (over
+    // all axes), which fix the fixed-point scale of the cell sums. Min and max are exact,
+    // so the float fold equals a double one; the partials are widened at the end.
+    // The last block to leave its partials folds them into the root box. The grid also zeroes
+    // what the kernels after it count in (zero_a and zero_b, in 16-byte units), which as
+    // memsets were two more launches.
+    __global__ void __launch_bounds__(256) bbox_kernel(const float4* __restrict__ src, const int stride, const int n,
+                                                       const int mode, const float size, float* part,
+                                                       unsigned* __restrict__ ticket, uint4* __restrict__ zero_a,
+                                                       const size_t count_a, uint4* __restrict__ zero_b,
+                                                       const size_t count_b, BoxParams* __restrict__ box)
+    {
+        for (size_t k = blockIdx.x * 256u + threadIdx.x; k < count_a; k += gridDim.x * 256u)
+            zero_a[k] = make_uint4(0u, 0u, 0u, 0u);
+        for (size_t k = blockIdx.x * 256u + threadIdx.x; k < count_b; k += gridDim.x * 256u)
+            zero_b[k] = make_uint4(0u, 0u, 0u, 0u);
+        float v[kBboxVals] = { INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, 0.f, 0.f };
+        auto fold = [&](const float4 p, const float m) {
+            const float x[3] = { p.x, p.y, p.z };
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+            {
+                v[a] = fminf(v[a], x[a]);
+                v[3 + a] = fmaxf(v[3 + a], x[a]);
+                if (isfinite(x[a]))
+                    v[7] = fmaxf(v[7], fabsf(x[a]));
+            }
+            if (isfinite(m))
+                v[6] = fmaxf(v[6], fabsf(m));
+        };
+        const int step = gridDim.x * blockDim.x;
+        int i = blockIdx.x * blockDim.x + threadIdx.x;
+        // four bodies in flight per thread
+        for (; static_cast<long long>(i) + 3 * step < n; i += 4 * step)
+        {
+            float4 p[4];
+            float m[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                const size_t k = static_cast<size_t>(i + u * step);
+                p[u] = src[k * stride];
+                m[u] = stride == 3 ? src[k * 3 + 1].w : p[u].w;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                fold(p[u], m[u]);
+        }
+        for (; i < n; i += step)
+        {
+            const float4 p = src[static_cast<size_t>(i) * stride];
+            fold(p, stride == 3 ? src[static_cast<size_t>(i) * 3 + 1].w : p.w);
+        }
+        __shared__ float red[kBboxVals][256];
+#pragma unroll
+        for (int a = 0; a < kBboxVals; ++a)
+            red[a][threadIdx.x] = v[a];
+        __syncthreads();
+        for (int s = blockDim.x / 2; s > 0; s >>= 1)
+        {
+            if (threadIdx.x < s)
+            {
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    red[a][threadIdx.x] = fminf(red[a][threadIdx.x], red[a][threadIdx.x + s]);
+#pragma unroll
+                for (int a = 3; a < kBboxVals; ++a)
+                    red[a][threadIdx.x] = fmaxf(red[a][threadIdx.x], red[a][threadIdx.x + s]);
+            }
+            __syncthreads();
+        }
+        __shared__ bool last;
+        if (threadIdx.x < kBboxVals)
+        {
+            part[blockIdx.x * kBboxVals + threadIdx.x] = red[threadIdx.x][0];
+            __threadfence();
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (!last)
+            return;
+        __threadfence();
+        if (threadIdx.x == 0)
+            *ticket = 0;        // for the next build
+        finish_box(part, gridDim.x, n, mode, size, red, box);
     }
 
     // ------------------------------------------------------------------------------------
@@ -499,6 +523,38 @@ namespace nbg
         return Int64x4{ a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w };
     }
 
+    // dl[k] = the common prefix of keys k and k + 1 for k < n - 1: 1 .. 95, one byte (64 + the
+    // bits that their indices share when they are equal), and smp[k] = the key at 64 k for
+    // 64 k < n - 1: those of k0 .. k0 + 3 (k0 a multiple of 4). For sorted keys the common
+    // prefix of keys i < j is the least of dl[i .. j - 1].
+    __device__ __forceinline__ void adjacent_prefixes(const uint64_t* __restrict__ keys, const int n, const int k0,
+                                                      uint8_t* __restrict__ dl, uint64_t* __restrict__ smp)
+    {
+        if (k0 >= n - 1)
+            return;
+        uint64_t a[5];
+#pragma unroll
+        for (int u = 0; u < 5; ++u)
+            a[u] = keys[min(k0 + u, n - 1)];
+        if ((k0 & 63) == 0)
+            smp[k0 >> 6] = a[0];        // every 64th key, for the far nodes' coarse searches
+        uint32_t packed = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const int k = k0 + u;
+            const uint32_t v = a[u] != a[u + 1]
+                                   ? static_cast<uint32_t>(__clzll(static_cast<long long>(a[u] ^ a[u + 1])))
+                                   : 64u + static_cast<uint32_t>(__clz(k ^ (k + 1)));
+            packed |= (k < n - 1 ? v : 0u) << (8 * u);
+        }
+        if (k0 + 4 <= n - 1)
+            *reinterpret_cast<uint32_t*>(dl + k0) = packed;
+        else
+            for (int u = 0; k0 + u < n - 1; ++u)
+                dl[k0 + u] = static_cast<uint8_t>(packed >> (8 * u));
+    }
+
     // Bodies into Morton order (pos_mass, and the radius when srad is given: only the cutoff
     // law reads it), and the fixed-point prefix sums within each tile of kMomTile sorted
     // bodies: part[x] = the sum of the terms of the bodies of x's tile before x, for
@@ -507,12 +563,15 @@ namespace nbg
     // of all bodies before x is then tile_prefix[x / kMomTile] + part[x], with tile_prefix
     // the exclusive scan of the totals (a tile past the last has total 0). Tiles need not
     // wait for one another. Four consecutive bodies per thread; every random read is issued
-    // before any is used (indices past the end read the last body and are not stored).
+    // before any is used (indices past the end read the last body and are not stored). The
+    // adjacent prefixes of the sorted keys, which the radix tree is found from, are formed here
+    // too: they depend on the same sort and nothing else.
     __global__ void __launch_bounds__(kMomThreads) gather_sum_kernel(
         const float4* __restrict__ src, const int stride, const float4* __restrict__ vel_radius,
         const uint32_t* __restrict__ order, const int n, const BoxParams* __restrict__ box,
         float4* __restrict__ spm, float* __restrict__ srad, Int64x4* __restrict__ part,
-        Int64x4* __restrict__ tile_sum)
+        Int64x4* __restrict__ tile_sum, const uint64_t* __restrict__ keys, uint8_t* __restrict__ dl,
+        uint64_t* __restrict__ smp)
     {
         using Op = ScanOps<Int64x4>;
         if (n <= 0)
@@ -556,6 +615,8 @@ namespace nbg
                 r[k] = vel_radius ? vel_radius[i].w : 0.f;
             }
         }
+        // the radix tree's prefix bytes, while those reads are in flight
+        adjacent_prefixes(keys, n, base, dl, smp);
         // the thread's total here; its bodies' terms are formed again for the prefixes below
         // (cheaper than holding four more Int64x4 through the scan)
         Int64x4 run{ 0, 0, 0, 0 };
@@ -642,38 +703,6 @@ namespace nbg
 
     __device__ __forceinline__ int level_of(const int prefix) { return min(kMaxLevel, prefix / 3); }
 
-    // dl[k] = delta(k, k + 1) for k < n - 1: 1 .. 95, one byte, and smp[k] = the key at 64 k
-    // for 64 k < n - 1. Four per thread. For sorted keys the common prefix of keys i < j is
-    // the least of dl[i .. j - 1].
-    __global__ void __launch_bounds__(256) adjacent_prefix_kernel(const uint64_t* __restrict__ keys, const int n,
-                                                                  uint8_t* __restrict__ dl, uint64_t* __restrict__ smp)
-    {
-        const int k0 = (blockIdx.x * 256 + threadIdx.x) * 4;
-        if (k0 >= n - 1)
-            return;
-        uint64_t a[5];
-#pragma unroll
-        for (int u = 0; u < 5; ++u)
-            a[u] = keys[min(k0 + u, n - 1)];
-        if ((k0 & 63) == 0)
-            smp[k0 >> 6] = a[0];        // every 64th key, for the far nodes' coarse searches
-        uint32_t packed = 0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-        {
-            const int k = k0 + u;
-            const uint32_t v = a[u] != a[u + 1]
-                                   ? static_cast<uint32_t>(__clzll(static_cast<long long>(a[u] ^ a[u + 1])))
-                                   : 64u + static_cast<uint32_t>(__clz(k ^ (k + 1)));
-            packed |= (k < n - 1 ? v : 0u) << (8 * u);
-        }
-        if (k0 + 4 <= n - 1)
-            *reinterpret_cast<uint32_t*>(dl + k0) = packed;
-        else
-            for (int u = 0; k0 + u < n - 1; ++u)
-                dl[k0 + u] = static_cast<uint8_t>(packed >> (8 * u));
-    }
-
     // one bit per byte of four 0x00 / 0xff bytes, byte 0 to bit 0
     __device__ __forceinline__ uint32_t movemask4(const uint32_t m) { return ((m & 0x80808080u) * 0x00204081u) >> 28; }
 
@@ -708,14 +737,14 @@ namespace nbg
     __device__ __forceinline__ void write_radix_node(const int i, const int lo, const int hi, const int gamma,
                                                      const int dnode, const int dmin, const int dfar,
                                                      int2* __restrict__ child, int2* __restrict__ range,
-                                                     int* __restrict__ prefix, uint32_t* __restrict__ flag)
+                                                     int* __restrict__ prefix, uint8_t* __restrict__ flag)
     {
         child[i] = make_int2(lo == gamma ? ~gamma : gamma, hi == gamma + 1 ? ~(gamma + 1) : gamma + 1);
         range[i] = make_int2(lo, hi);
         const int pre = dnode - 1;      // codes are 63-bit: the top key bit is always shared
         prefix[i] = pre;
         const int up = max(dmin, dfar) - 1;
-        flag[i] = (i == 0 || level_of(pre) > level_of(up)) ? 1u : 0u;
+        flag[i] = (i == 0 || level_of(pre) > level_of(up)) ? 1 : 0;
     }
 
     // Radix-tree nodes whose ranges end within about kNearScan keys (97.5 % of them at 16.8M
@@ -735,7 +764,7 @@ namespace nbg
     __device__ __forceinline__ bool near_node(const uint64_t* __restrict__ keys, const uint8_t* __restrict__ dl,
                                               const int n, const int i, int2* __restrict__ child,
                                               int2* __restrict__ range, int* __restrict__ prefix,
-                                              uint32_t* __restrict__ flag, unsigned* __restrict__ err)
+                                              uint8_t* __restrict__ flag, unsigned* __restrict__ err)
     {
         const int dr = dl[i];
         const int dlf = i > 0 ? static_cast<int>(dl[i - 1]) : -1;
@@ -821,12 +850,58 @@ namespace nbg
         return false;
     }
 
+    // The exclusive scan of the cell sums' tile totals by one block of 256 threads: the octree
+    // records need it and the radix tree does not, so one block of that kernel has it done
+    // before its others end (at 16.8M bodies, 8193 totals).
+    __device__ void scan_totals(const Int64x4* __restrict__ in, Int64x4* __restrict__ out, const int count)
+    {
+        using Op = ScanOps<Int64x4>;
+        __shared__ Int64x4 warp_tot[8];
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        Int64x4 carry{ 0, 0, 0, 0 };        // all earlier chunks'
+        for (int base = 0; base < count; base += 256)
+        {
+            const int i = base + threadIdx.x;
+            Int64x4 incl = i < count ? in[i] : Int64x4{ 0, 0, 0, 0 };
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1)
+            {
+                const Int64x4 o = Op::shfl_up(incl, d);
+                if (lane >= d)
+                    incl = add4(incl, o);
+            }
+            if (lane == 31)
+                warp_tot[warp] = incl;
+            __syncthreads();
+            Int64x4 off = Op::shfl_up(incl, 1);
+            if (lane == 0)
+                off = Int64x4{ 0, 0, 0, 0 };
+            off = add4(off, carry);
+#pragma unroll 1
+            for (int w = 0; w < 8; ++w)
+            {
+                if (w < warp)
+                    off = add4(off, warp_tot[w]);
+                carry = add4(carry, warp_tot[w]);
+            }
+            if (i < count)
+                out[i] = off;
+            __syncthreads();
+        }
+    }
+
     __global__ void __launch_bounds__(256) radix_near_kernel(
         const uint64_t* __restrict__ keys, const uint8_t* __restrict__ dl, const int n, int2* __restrict__ child,
-        int2* __restrict__ range, int* __restrict__ prefix, uint32_t* __restrict__ flag, int* __restrict__ far_list,
-        unsigned* __restrict__ far_count, unsigned* __restrict__ err)
+        int2* __restrict__ range, int* __restrict__ prefix, uint8_t* __restrict__ flag, int* __restrict__ far_list,
+        unsigned* __restrict__ far_count, const Int64x4* __restrict__ tile_sum, Int64x4* __restrict__ tile_prefix,
+        const int tiles, unsigned* __restrict__ err)
     {
-        const int i = blockIdx.x * 256 + threadIdx.x;
+        if (blockIdx.x == 0)
+        {
+            scan_totals(tile_sum, tile_prefix, tiles);
+            return;
+        }
+        const int i = (blockIdx.x - 1) * 256 + threadIdx.x;
         const bool far = i < n - 1 && near_node(keys, dl, n, i, child, range, prefix, flag, err);
         // a warp's far nodes take consecutive slots of far_list: one global atomic a warp
         const unsigned fm = __ballot_sync(0xffffffffu, far);
@@ -950,7 +1025,7 @@ namespace nbg
                                                             const int* __restrict__ far_list,
                                                             const unsigned* __restrict__ far_count,
                                                             int2* __restrict__ child, int2* __restrict__ range,
-                                                            int* __restrict__ prefix, uint32_t* __restrict__ flag,
+                                                            int* __restrict__ prefix, uint8_t* __restrict__ flag,
                                                             unsigned* __restrict__ err)
     {
         const int count = static_cast<int>(*far_count);
@@ -980,6 +1055,118 @@ namespace nbg
     // ------------------------------------------------------------------------------------
     // 6. octree records
     // ------------------------------------------------------------------------------------
+    constexpr uint32_t kIsOct = 0x80000000u;
+    constexpr int kNumTile = 4096;      // binary nodes per CTA of the numbering
+
+    // A tile's published count of octree nodes: its own, or with all earlier tiles'.
+    constexpr uint64_t kCountOwn = 1ull << 62, kCountAll = 2ull << 62;
+
+    // octidx[i] = the octree nodes among binary nodes 0 .. i - 1, with kIsOct set when node i is one
+    // itself (its index in the record array is then octidx[i] without it). One launch: tiles of
+    // 4096 nodes taken in ticket order, the earlier tiles' count found by decoupled look-back,
+    // 32 tiles at a time (the waits are bounded and on CTAs that are running, as in the radix
+    // sort). status[0] is the ticket, status[1 + t] tile t's count, all zero before. A wait that
+    // gives up counts nothing before its tile: indices stay in range.
+    __global__ void __launch_bounds__(1024) number_kernel(const uint8_t* __restrict__ flag, const int m,
+                                                          uint32_t* __restrict__ octidx, uint64_t* __restrict__ status,
+                                                          unsigned* __restrict__ err)
+    {
+        __shared__ uint32_t warp_tot[32];
+        __shared__ uint32_t before_s;
+        __shared__ int tile_s;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        if (threadIdx.x == 0)
+            tile_s = static_cast<int>(atomicAdd(reinterpret_cast<unsigned*>(status), 1u));
+        __syncthreads();
+        const int tile = tile_s;
+        const int base = tile * kNumTile + threadIdx.x * 4;
+        uint32_t f = 0;     // a byte per node
+        if (base + 4 <= m)
+            f = *reinterpret_cast<const uint32_t*>(flag + base);
+        else
+            for (int k = 0; k < 4; ++k)
+                f |= base + k < m ? static_cast<uint32_t>(flag[base + k]) << (8 * k) : 0u;
+        const uint32_t mine = __popc(f);
+        uint32_t incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+        {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d)
+                incl += o;
+        }
+        if (lane == 31)
+            warp_tot[warp] = incl;
+        __syncthreads();
+        if (warp == 0)
+        {
+            const uint32_t w = warp_tot[lane];
+            uint32_t wi = w;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1)
+            {
+                const uint32_t o = __shfl_up_sync(0xffffffffu, wi, d);
+                if (lane >= d)
+                    wi += o;
+            }
+            warp_tot[lane] = wi - w;        // before each warp
+            const uint32_t total = __shfl_sync(0xffffffffu, wi, 31);
+            if (lane == 0)
+                store_relaxed(&status[1 + tile], (tile ? kCountOwn : kCountAll) | total);
+            uint32_t before = 0;
+            uint64_t t0 = 0;
+            for (int j = tile - 1; j >= 0;)
+            {
+                const uint64_t v = j - lane >= 0 ? load_relaxed(&status[1 + j - lane]) : kCountAll;
+                const unsigned missing = __ballot_sync(0xffffffffu, !(v >> 62));
+                const unsigned all = __ballot_sync(0xffffffffu, (v >> 62) == 2);
+                // the lanes before the first missing word, up to and with the first that counts all
+                const unsigned stop = all & (0u - all);
+                const unsigned use = all ? (stop << 1) - 1u : 0xffffffffu;
+                if (missing & use)
+                {
+                    if (!t0)
+                        t0 = globaltimer();
+                    else if (globaltimer() - t0 > kWaitLimitNs)
+                    {
+                        if (lane == 0)
+                            atomicOr(err, DEV_ERR_TIMEOUT);
+                        before = 0;
+                        break;
+                    }
+                    __nanosleep(100);
+                    continue;
+                }
+                before += __reduce_add_sync(0xffffffffu, (use >> lane) & 1u ? static_cast<uint32_t>(v) : 0u);
+                if (all)
+                    break;
+                j -= 32;
+            }
+            if (lane == 0)
+            {
+                if (tile)
+                    store_relaxed(&status[1 + tile], kCountAll | (before + total));
+                before_s = before;
+            }
+        }
+        __syncthreads();
+        uint32_t at = before_s + warp_tot[warp] + incl - mine;
+        uint32_t out[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+        {
+            const uint32_t is = (f >> (8 * k)) & 1u;
+            out[k] = at | (is ? kIsOct : 0u);
+            at += is;
+        }
+        if (base + 4 <= m)
+            *reinterpret_cast<uint4*>(octidx + base) = make_uint4(out[0], out[1], out[2], out[3]);
+        else
+            for (int k = 0; k < 4; ++k)
+                if (base + k < m)
+                    octidx[base + k] = out[k];
+    }
+
     // The children of a cell: walking down through the binary nodes of the cell's own level
     // (at most three splits below it), every leaf body and every node of a deeper level is
     // one child. Right subtrees first, which is the order the traversal has always used.
@@ -996,13 +1183,13 @@ namespace nbg
 
     template <int DEPTH>
     __device__ __forceinline__ void collect_children(const int c, const int2* __restrict__ child,
-                                                     const uint32_t* __restrict__ flag,
                                                      const uint32_t* __restrict__ octidx, int (&kid)[8],
                                                      int& nc, unsigned* __restrict__ err)
     {
-        if (c < 0 || flag[c])
+        const uint32_t w = c < 0 ? 0u : octidx[c];
+        if (c < 0 || (w & kIsOct))
         {
-            emit_child(kid, nc, c < 0 ? c : static_cast<int>(octidx[c]), err);
+            emit_child(kid, nc, c < 0 ? c : static_cast<int>(w & ~kIsOct), err);
             return;
         }
         if (DEPTH == 0)
@@ -1011,8 +1198,8 @@ namespace nbg
             return;
         }
         const int2 ch = child[c];
-        collect_children<DEPTH ? DEPTH - 1 : 0>(ch.y, child, flag, octidx, kid, nc, err);
-        collect_children<DEPTH ? DEPTH - 1 : 0>(ch.x, child, flag, octidx, kid, nc, err);
+        collect_children<DEPTH ? DEPTH - 1 : 0>(ch.y, child, octidx, kid, nc, err);
+        collect_children<DEPTH ? DEPTH - 1 : 0>(ch.x, child, octidx, kid, nc, err);
     }
 
     // position of the r-th set bit (from 0) of v, for r < popc(v)
@@ -1051,8 +1238,7 @@ namespace nbg
     // (ballots; about 40 % are flagged) and its lanes then take them in turn, instead of
     // idling on unflagged ones; and full occupancy (32 registers) beats fewer spills.
     __global__ void __launch_bounds__(256, 8) octnode_kernel(const int2* __restrict__ child, const int2* __restrict__ range,
-                                   const int* __restrict__ prefix, const uint32_t* __restrict__ flag,
-                                   const uint32_t* __restrict__ octidx, const Int64x4* __restrict__ part,
+                                   const int* __restrict__ prefix, const uint32_t* __restrict__ octidx, const Int64x4* __restrict__ part,
                                    const Int64x4* __restrict__ tile_prefix, const int m,
                                    const BoxParams* __restrict__ box, const float theta,
                                    OctNode* __restrict__ nodes, unsigned* __restrict__ err,
@@ -1060,7 +1246,7 @@ namespace nbg
     {
         const int gt = blockIdx.x * blockDim.x + threadIdx.x;
         if (gt == 0)
-            atomicAdd(&stats[2], static_cast<unsigned long long>(octidx[m - 1] + flag[m - 1]));
+            atomicAdd(&stats[2], static_cast<unsigned long long>((octidx[m - 1] & ~kIsOct) + (octidx[m - 1] >> 31)));
         const int lane = threadIdx.x & 31;
         const int first = (gt >> 5) * (32 * kOctSpan);
         if (first >= m)
@@ -1071,7 +1257,7 @@ namespace nbg
         for (int u = 0; u < kOctSpan; ++u)
         {
             const int i = first + u * 32 + lane;
-            mask[u] = __ballot_sync(0xffffffffu, i < m && flag[i] != 0u);
+            mask[u] = __ballot_sync(0xffffffffu, i < m && (octidx[i] & kIsOct));
             total += __popc(mask[u]);
         }
         const int shift = box->mass_shift - box->mom_shift;
@@ -1097,7 +1283,7 @@ namespace nbg
             const Int64x4 hi = add4(tile_prefix[(rg.y + 1) / kMomTile], part[rg.y + 1]);
             const Int64x4 lo = add4(tile_prefix[rg.x / kMomTile], part[rg.x]);
             const long long ms = hi.w - lo.w;   // exact: the cell's own terms
-            OctNode* out = nodes + octidx[i];
+            OctNode* out = nodes + (octidx[i] & ~kIsOct);
             float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
             if (ms > 0)
             {
@@ -1119,8 +1305,8 @@ namespace nbg
             else
             {
                 const int2 ch = child[i];
-                collect_children<2>(ch.y, child, flag, octidx, kid, nc, err);
-                collect_children<2>(ch.x, child, flag, octidx, kid, nc, err);
+                collect_children<2>(ch.y, child, octidx, kid, nc, err);
+                collect_children<2>(ch.x, child, octidx, kid, nc, err);
                 nc = min(nc, 8);
             }
             out->com_mass = cm;
@@ -1972,6 +2158,13 @@ namespace nbg
             return cudaMallocAsync(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T), s);
         }
 
+        // The words a build counts in: statistics, the numbering's ticket and a word per tile.
+        size_t count_bytes(const size_t n)
+        {
+            const size_t words = kStatsWords + 1 + (n + kNumTile - 1) / kNumTile;
+            return (words + 1) / 2 * 16;
+        }
+
         int reserve_bh(nbody_cuda* ctx, const size_t n)
         {
             if (!ctx->bh)
@@ -1984,7 +2177,9 @@ namespace nbg
                     e = cudaMallocAsync(reinterpret_cast<void**>(&b.bbox_part), kBboxBlocks * kBboxVals * sizeof(float),
                                         ctx->stream);
                 if (e == cudaSuccess)
-                    e = cudaMallocAsync(reinterpret_cast<void**>(&b.stats), kStatsWords * sizeof(unsigned long long), ctx->stream);
+                    e = cudaMallocAsync(reinterpret_cast<void**>(&b.box_ticket), sizeof(unsigned), ctx->stream);
+                if (e == cudaSuccess)
+                    e = cudaMemsetAsync(b.box_ticket, 0, sizeof(unsigned), ctx->stream);
                 if (e != cudaSuccess)
                     return ctx_cuda_fail(ctx, e, "tree allocation");
             }
@@ -1994,12 +2189,8 @@ namespace nbg
                 return st;
             const size_t cap = std::max(n, b.cap + b.cap / 2);
             const size_t tiles = (cap + kMomTile - 1) / kMomTile;
-            // the sort's temporaries; later the cell sums' tile totals and tile prefixes, and
-            // after them the scans' temporaries (the tile totals' and the octree compaction's)
-            const size_t tb = std::max(sort_temp_bytes(cap),
-                                       2 * (tiles + 1) * sizeof(Int64x4)
-                                           + std::max(scan_temp_elems(tiles + 1) * sizeof(Int64x4),
-                                                      scan_temp_elems(cap) * sizeof(uint32_t)));
+            // the sort's temporaries; later the cell sums' tile totals and tile prefixes
+            const size_t tb = std::max(sort_temp_bytes(cap), 2 * (tiles + 1) * sizeof(Int64x4));
             cudaError_t e = cudaSuccess;
             cudaStream_t s = ctx->stream;
             for (int k = 0; k < 2 && e == cudaSuccess; ++k)
@@ -2015,6 +2206,9 @@ namespace nbg
             if (e == cudaSuccess) e = grow(&b.prefix, cap, s);
             if (e == cudaSuccess) e = grow(&b.octflag, cap, s);
             if (e == cudaSuccess) e = grow(&b.octidx, cap, s);
+            // the statistics, then the numbering's ticket and tile counts: zeroed together
+            if (e == cudaSuccess) e = grow(&b.stats, count_bytes(cap) / sizeof(unsigned long long), s);
+            b.numbering = reinterpret_cast<uint64_t*>(b.stats) + kStatsWords;
             if (e == cudaSuccess) e = grow(&b.psum, cap + 1, s);
             if (e == cudaSuccess) e = grow(&b.nodes, cap, s);
             if (e == cudaSuccess)
@@ -2058,14 +2252,12 @@ namespace nbg
         const int ni = static_cast<int>(n);
         uint64_t& L = ctx->launches;
 
-        if (const cudaError_t me = cudaMemsetAsync(b.stats, 0, kStatsWords * sizeof(unsigned long long), s))
-            return ctx_cuda_fail(ctx, me, "tree statistics");
         // tree_box = 0 is the reference's fixed root box; it needs a positive size
         const bool auto_box = p->tree_box != 0 || !(p->size > 0.f);
         // the bounds pass runs for the fixed box too: the cell sums' scale comes from it
-        bbox_partial_kernel<<<kBboxBlocks, 256, 0, s>>>(src, stride, ni, b.bbox_part);
-        ++L;
-        box_final_kernel<<<1, 256, 0, s>>>(b.bbox_part, kBboxBlocks, ni, auto_box ? 1 : 0, p->size, b.box);
+        bbox_kernel<<<std::min<unsigned>(kBboxBlocks, std::max(1u, ceil_div(n, 1024))), 256, 0, s>>>(
+            src, stride, ni, auto_box ? 1 : 0, p->size, b.bbox_part, b.box_ticket, reinterpret_cast<uint4*>(b.stats),
+            count_bytes(n) / 16, static_cast<uint4*>(b.temp), sort_zero_bytes(n) / 16, b.box);
         ++L;
         morton_kernel<<<ceil_div(n, 256 * kMortonItems), 256, 0, s>>>(src, stride, ni, b.box, b.keys[0], b.vals[0]);
         ++L;
@@ -2093,19 +2285,21 @@ namespace nbg
         b.codes = keys;
         const unsigned tiles = std::max(1u, ceil_div(n, kMomTile));
         // temporaries: tile totals and their exclusive scan (tiles + 1 each: the entry past
-        // the last tile gives the sum of all bodies), then the scans' own
+        // the last tile gives the sum of all bodies)
         Int64x4* tile_sum = static_cast<Int64x4*>(b.temp);
         Int64x4* tile_prefix = tile_sum + tiles + 1;
-        void* scan_temp = tile_prefix + tiles + 1;
+        // adjacent prefix lengths, key samples and the far nodes' list live in the sort's
+        // other key and value buffers, free until the next build
+        const int other = in_alt ? 0 : 1;
+        uint8_t* dl = reinterpret_cast<uint8_t*>(b.keys[other]);
+        // (n rounded up to 8 bytes, then n / 64 + 1 keys: within the buffer's 8 n bytes for n >= 2)
+        uint64_t* smp = reinterpret_cast<uint64_t*>(dl + ((n + 7) & ~size_t(7)));
         const bool radius = p->law == NBODY_LAW_CUTOFF;
         gather_sum_kernel<<<tiles, kMomThreads, 0, s>>>(src, stride,
                                                         radius && ctx->layout != NBODY_LAYOUT_AOS ? ctx->vr : nullptr,
                                                         order, ni, b.box, b.spm, radius ? b.srad : nullptr, b.psum,
-                                                        tile_sum);
+                                                        tile_sum, keys, dl, smp);
         ++L;
-        e = exclusive_scan<Int64x4>(tile_sum, tile_prefix, tiles + 1, static_cast<Int64x4*>(scan_temp), s, &L);
-        if (e != cudaSuccess)
-            return ctx_cuda_fail(ctx, e, "cell sums");
         if (n < 2)
         {
             b.built = true;
@@ -2114,30 +2308,20 @@ namespace nbg
             return NBODY_OK;
         }
         const int m = ni - 1;
-        {
-            // adjacent prefix lengths, key samples and the far nodes' list live in the sort's
-            // other key and value buffers, free until the next build
-            const int other = in_alt ? 0 : 1;
-            uint8_t* dl = reinterpret_cast<uint8_t*>(b.keys[other]);
-            // (n rounded up to 8 bytes, then n / 64 + 1 keys: within the buffer's 8 n bytes for n >= 2)
-            uint64_t* smp = reinterpret_cast<uint64_t*>(dl + ((n + 7) & ~size_t(7)));
-            int* far_list = reinterpret_cast<int*>(b.vals[other]);
-            unsigned* far_count = reinterpret_cast<unsigned*>(b.stats + 5);
-            adjacent_prefix_kernel<<<ceil_div(m, 256 * 4), 256, 0, s>>>(keys, ni, dl, smp);
-            ++L;
-            radix_near_kernel<<<ceil_div(m, 256), 256, 0, s>>>(keys, dl, ni, b.child, b.range, b.prefix, b.octflag,
-                                                               far_list, far_count, ctx->dev_error);
-            ++L;
-            radix_far_kernel<<<std::min(ceil_div(m, 256), 2048u), 256, 0, s>>>(keys, dl, smp, ni, far_list, far_count,
-                                                                                  b.child, b.range, b.prefix,
-                                                                                  b.octflag, ctx->dev_error);
-            ++L;
-        }
-        e = exclusive_scan<uint32_t>(b.octflag, b.octidx, m, static_cast<uint32_t*>(scan_temp), s, &L);
-        if (e != cudaSuccess)
-            return ctx_cuda_fail(ctx, e, "octree compaction");
-        octnode_kernel<<<ceil_div(m, 256 * kOctSpan), 256, 0, s>>>(b.child, b.range, b.prefix, b.octflag, b.octidx,
-                                                                    b.psum, tile_prefix, m, b.box, p->theta, b.nodes,
+        int* far_list = reinterpret_cast<int*>(b.vals[other]);
+        unsigned* far_count = reinterpret_cast<unsigned*>(b.stats + 5);
+        radix_near_kernel<<<1 + ceil_div(m, 256), 256, 0, s>>>(keys, dl, ni, b.child, b.range, b.prefix, b.octflag,
+                                                               far_list, far_count, tile_sum, tile_prefix,
+                                                               static_cast<int>(tiles) + 1, ctx->dev_error);
+        ++L;
+        radix_far_kernel<<<std::min(ceil_div(m, 256), 2048u), 256, 0, s>>>(keys, dl, smp, ni, far_list, far_count,
+                                                                              b.child, b.range, b.prefix, b.octflag,
+                                                                              ctx->dev_error);
+        ++L;
+        number_kernel<<<ceil_div(m, kNumTile), 1024, 0, s>>>(b.octflag, m, b.octidx, b.numbering, ctx->dev_error);
+        ++L;
+        octnode_kernel<<<ceil_div(m, 256 * kOctSpan), 256, 0, s>>>(b.child, b.range, b.prefix, b.octidx, b.psum,
+                                                                    tile_prefix, m, b.box, p->theta, b.nodes,
                                                                     ctx->dev_error, b.stats);
         ++L;
         e = cudaGetLastError();
@@ -2307,7 +2491,7 @@ namespace nbg
             cudaFree(b.vals[k]);
         }
         void* ptrs[] = { b.spm, b.srad, b.child, b.range, b.prefix, b.octflag, b.octidx, b.psum,
-                         b.nodes, b.temp, b.box, b.bbox_part, b.stats };
+                         b.nodes, b.temp, b.box, b.bbox_part, b.box_ticket, b.stats };
         for (void* q : ptrs)
             cudaFree(q);
         for (cudaEvent_t ev : b.ev)

@@ -96,6 +96,19 @@ namespace nbg
         }
     }
 
+    // Counts published between CTAs of one launch (decoupled look-back): single 64-bit words.
+    __device__ __forceinline__ uint64_t load_relaxed(const uint64_t* p)
+    {
+        uint64_t v;
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+        return v;
+    }
+
+    __device__ __forceinline__ void store_relaxed(uint64_t* p, const uint64_t v)
+    {
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
+    }
+
     // One-dimensional TMA bulk copy global -> shared, completing on `bar` with a byte
     // count. dst, src and bytes must all be multiples of 16.
     __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, const unsigned bytes,

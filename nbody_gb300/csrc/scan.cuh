@@ -1,5 +1,5 @@
-// Device-wide exclusive prefix sums (uint32 and four int64 lanes), used by the radix sort,
-// the octree compaction and the fixed-point centre-of-mass sums. Three-phase: each CTA scans a 4096-item
+// Device-wide exclusive prefix sums of uint32 (the scene generators' slot counts), and the
+// operations of a scan over uint32 or four int64 lanes. Three-phase: each CTA scans a 4096-item
 // tile and records its total; the totals are scanned (recursively); each tile then adds
 // its offset. All temporaries come from a caller-provided buffer.
 #pragma once
@@ -65,5 +65,4 @@ namespace nbg
     cudaError_t exclusive_scan(const T* in, T* out, size_t n, T* temp, cudaStream_t stream, uint64_t* launches);
 
     extern template cudaError_t exclusive_scan<uint32_t>(const uint32_t*, uint32_t*, size_t, uint32_t*, cudaStream_t, uint64_t*);
-    extern template cudaError_t exclusive_scan<Int64x4>(const Int64x4*, Int64x4*, size_t, Int64x4*, cudaStream_t, uint64_t*);
 }

@@ -57,7 +57,7 @@ namespace nbg
             uint32_t* tickets;      // kMaxPasses tile tickets, then the whole sort's barrier count
             uint32_t* ghist;        // kMaxPasses x kDigits global digit counts
             uint64_t* status;       // tiles x kDigits published counts
-            size_t zero_bytes;      // everything above is zeroed before a sort
+            size_t zero_bytes;      // everything above, zero before a sort
         };
 
         constexpr size_t kGhistOffset = 256;
@@ -117,18 +117,6 @@ namespace nbg
     {
         __shared__ uint32_t hist[kMaxPasses * kDigits];
         histogram(hist, keys, n, shift0, passes, ghist);
-    }
-
-    __device__ __forceinline__ uint64_t load_relaxed(const uint64_t* p)
-    {
-        uint64_t v;
-        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-        return v;
-    }
-
-    __device__ __forceinline__ void store_relaxed(uint64_t* p, const uint64_t v)
-    {
-        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
     }
 
     // Exclusive block-wide scan of kPer consecutive values per thread (the thread's digits).
@@ -443,11 +431,9 @@ namespace nbg
         }
     }
 
-    size_t sort_temp_bytes(const size_t n)
-    {
-        const size_t tiles = (n + kTile - 1) / kTile;
-        return zero_bytes(tiles) + 256;
-    }
+    size_t sort_zero_bytes(const size_t n) { return zero_bytes((n + kTile - 1) / kTile); }
+
+    size_t sort_temp_bytes(const size_t n) { return sort_zero_bytes(n) + 256; }
 
     namespace
     {
@@ -482,14 +468,10 @@ namespace nbg
             return attr;
         const int tiles = static_cast<int>((n + kTile - 1) / kTile);
         const TempLayout t = layout(temp, static_cast<size_t>(tiles));
-        // the tickets, histograms and published counts of every pass, a later sort_if's too
-        cudaError_t e = cudaMemsetAsync(temp, 0, t.zero_bytes, stream);
-        if (e != cudaSuccess)
-            return e;
         const int hist_grid = std::max(1, std::min((static_cast<int>(n) + kHistThreads - 1) / kHistThreads, 2 * sm_count()));
         digit_hist_kernel<<<hist_grid, kHistThreads, 0, stream>>>(keys, static_cast<int>(n), begin_bit, passes, t.ghist);
         ++*launches;
-        e = cudaGetLastError();
+        cudaError_t e = cudaGetLastError();
         uint64_t* kin = keys;
         uint32_t* vin = vals;
         uint64_t* kout = keys_alt;

@@ -11,6 +11,9 @@ namespace nbg
     // Temporary bytes radix_sort_pairs needs for n pairs.
     size_t sort_temp_bytes(size_t n);
 
+    // The bytes at its start (a multiple of 16) that are zero before a sort of n pairs.
+    size_t sort_zero_bytes(size_t n);
+
     // Sort by bits [begin_bit, end_bit) of the key, 9 bits per pass, ping-ponging between
     // (keys, vals) and (keys_alt, vals_alt). *in_alt tells which pair holds the result.
     // n < 2^31. A look-back wait that gives up (it cannot, unless the device is broken) ORs
@@ -22,7 +25,7 @@ namespace nbg
     // The same sort in one launch, done only when *run_if is not 0 on the device (the host
     // need not know); the result is in (keys, vals). For a call after radix_sort_pairs on the
     // same temp and n, with at most pass_base passes: both use the 16 passes' tickets,
-    // histograms and published counts that it zeroed.
+    // histograms and published counts.
     cudaError_t radix_sort_if(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, size_t n,
                               int begin_bit, int end_bit, void* temp, int pass_base, cudaStream_t stream,
                               uint64_t* launches, unsigned* err, const unsigned* run_if);
