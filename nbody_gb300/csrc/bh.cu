@@ -2189,8 +2189,10 @@ namespace nbg
                 return st;
             const size_t cap = std::max(n, b.cap + b.cap / 2);
             const size_t tiles = (cap + kMomTile - 1) / kMomTile;
-            // the sort's temporaries; later the cell sums' tile totals and tile prefixes
-            const size_t tb = std::max(sort_temp_bytes(cap), 2 * (tiles + 1) * sizeof(Int64x4));
+            // the sort's temporaries; later the cell sums' tile totals and tile prefixes, and a
+            // tree export's scan
+            const size_t tb = std::max({ sort_temp_bytes(cap), 2 * (tiles + 1) * sizeof(Int64x4),
+                                         scan_temp_elems(cap) * sizeof(uint32_t) });
             cudaError_t e = cudaSuccess;
             cudaStream_t s = ctx->stream;
             for (int k = 0; k < 2 && e == cudaSuccess; ++k)
@@ -2520,42 +2522,15 @@ namespace nbg
         return (ctx->bh && ctx->bh->built) ? ctx->bh->build_id : 0;
     }
 
-    int bh_download(nbody_cuda* ctx, TreeSnapshot* out)
+    int bh_view(nbody_cuda* ctx, TreeView* out)
     {
-        out->n = 0;
-        out->cells.clear();
-        out->codes.clear();
-        out->bodies.clear();
         if (!ctx->bh || !ctx->bh->built)
             return ctx_fail(ctx, NBODY_ERR_INVALID, "no Barnes-Hut tree has been built");
         BhState& b = *ctx->bh;
-        const size_t n = b.built_n;
-        out->n = n;
-        out->build_id = b.build_id;
-        cudaStream_t s = ctx->stream;
-        out->codes.resize(n);
-        out->bodies.resize(n);
-        unsigned long long st[3] = { 0, 0, 0 };
-        cudaError_t e = cudaMemcpyAsync(out->codes.data(), b.codes, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(out->bodies.data(), b.spm, n * sizeof(float4), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(&out->box, b.box, sizeof(BoxParams), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(st, b.stats, sizeof st, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess)
-            e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess)
-            return ctx_cuda_fail(ctx, e, "tree readback");
-        const size_t cells = n >= 2 ? static_cast<size_t>(st[2]) : 0;
-        out->cells.resize(cells);
-        if (cells)
-        {
-            e = cudaMemcpyAsync(out->cells.data(), b.nodes, cells * sizeof(OctNode), cudaMemcpyDeviceToHost, s);
-            if (e != cudaSuccess)
-                return ctx_cuda_fail(ctx, e, "tree readback");
-        }
-        return check_device_error(ctx);
+        *out = TreeView{ static_cast<int>(b.built_n), b.build_id, b.nodes, b.codes, b.spm, b.box, &b.stats[2],
+                         { b.octidx, reinterpret_cast<uint32_t*>(b.prefix), reinterpret_cast<uint32_t*>(b.child) },
+                         b.temp };
+        return NBODY_OK;
     }
 
     int bh_morton(nbody_cuda* ctx, const nbody_step_params* p, uint64_t* codes, uint32_t* order, double box[4])

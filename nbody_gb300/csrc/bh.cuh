@@ -2,7 +2,6 @@
 #pragma once
 
 #include <cstdint>
-#include <vector>
 #include <cuda_runtime.h>
 
 #include "nbody_cuda.h"
@@ -42,19 +41,23 @@ namespace nbg
     };
     static_assert(sizeof(OctNode) == 64, "OctNode is one 64-byte record");
 
-    // Host copy of the last device tree (tree_export.cu turns it into reference nodes).
-    struct TreeSnapshot
+    // The last device tree where it lies, and scratch that is free until the next build
+    // (tree_export.cu turns it into reference nodes).
+    struct TreeView
     {
-        size_t n = 0;                   // bodies
-        uint64_t build_id = 0;
-        BoxParams box{};
-        std::vector<OctNode> cells;     // cell 0 is the root cell (n >= 2)
-        std::vector<uint64_t> codes;    // sorted Morton codes
-        std::vector<float4> bodies;     // pos + mass in Morton order
+        int n;                          // bodies
+        uint64_t build_id;
+        const OctNode* nodes;           // cell 0 is the root cell (n >= 2)
+        const uint64_t* codes;          // sorted Morton codes
+        const float4* bodies;           // pos + mass in Morton order
+        const BoxParams* box;
+        const unsigned long long* cells;    // how many cells there are
+        uint32_t* words[3];             // n words each
+        void* temp;                     // a scan of n words' temporaries
     };
 
     int bh_build(nbody_cuda* ctx, const nbody_step_params* p);
-    int bh_download(nbody_cuda* ctx, TreeSnapshot* out);
+    int bh_view(nbody_cuda* ctx, TreeView* out);
     uint64_t bh_build_id(const nbody_cuda* ctx);    // 0 before the first build
     int bh_stats(nbody_cuda* ctx, unsigned long long out[3]);
     int bh_stage_ms(nbody_cuda* ctx, float ms[2]);

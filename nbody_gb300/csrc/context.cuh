@@ -87,15 +87,13 @@ struct nbody_cuda
     size_t graph_count = 0;
     cudaStream_t graph_stream = nullptr;
 
-    // The last tree in the reference's node layout (tree_export.cu), and the build it is of.
-    std::vector<unsigned char> tree_export;
-    uint64_t tree_export_id = 0;
-
-    // Ray queries (query.cu): the node array on the device (the exported tree while
-    // query_nodes_id matches its build) and the rays / hits / counts buffers.
+    // Ray queries (query.cu): a node array on the device (the last tree in the reference's node
+    // layout while query_nodes_id matches its build, tree_export.cu; a caller's otherwise) and
+    // the rays / hits / counts buffers.
     void* query_nodes = nullptr;
     size_t query_nodes_cap = 0;
     uint64_t query_nodes_id = 0;
+    size_t query_nodes_count = 0;
     void* query_buf = nullptr;
     size_t query_buf_cap = 0;
 
@@ -165,7 +163,11 @@ namespace nbg
     // query.cu
     int tree_query(nbody_cuda* ctx, const void* nodes, size_t count, const float* rays, size_t nrays, int stop,
                    uint32_t* hits, size_t max_hits, uint32_t* counts);
+    int reserve_query_nodes(nbody_cuda* ctx, size_t bytes);
     void release_query(nbody_cuda* ctx);
+
+    // tree_export.cu: the last Barnes-Hut tree as reference nodes in ctx->query_nodes
+    int tree_on_device(nbody_cuda* ctx, size_t* count);
 
     // scenes.cu
     int scene_disk(nbody_cuda* ctx, const nbody_disk_args* a, size_t begin, size_t num);

@@ -129,6 +129,11 @@ namespace nbg
         }
     }
 
+    int reserve_query_nodes(nbody_cuda* ctx, const size_t bytes)
+    {
+        return grow(ctx, &ctx->query_nodes, &ctx->query_nodes_cap, bytes, "query tree allocation");
+    }
+
     int tree_query(nbody_cuda* ctx, const void* nodes, size_t count, const float* rays, const size_t nrays,
                    const int stop, uint32_t* hits, const size_t max_hits, uint32_t* counts)
     {
@@ -138,15 +143,9 @@ namespace nbg
             return ctx_fail(ctx, NBODY_ERR_INVALID, "null query buffers");
         if (nrays > UINT32_MAX || max_hits > UINT32_MAX || (max_hits && nrays > SIZE_MAX / 4 / max_hits))
             return ctx_fail(ctx, NBODY_ERR_INVALID, "query too large");
-        const void* host_nodes = nodes;
-        uint64_t id = 0;
         if (!nodes)
-        {
-            if (const int st = nbody_cuda_tree_export(ctx, nullptr, 0, &count))
+            if (const int st = tree_on_device(ctx, &count))
                 return st;
-            host_nodes = ctx->tree_export.data();
-            id = ctx->tree_export_id;
-        }
         if (count > UINT32_MAX)
             return ctx_fail(ctx, NBODY_ERR_INVALID, "tree too large");
         if (!nrays)
@@ -157,15 +156,14 @@ namespace nbg
                 counts[q] = 0;
             return NBODY_OK;
         }
-        // the exported tree stays on the device until the next build; a caller's array is
-        // uploaded each call
-        if (!id || id != ctx->query_nodes_id)
+        if (nodes)
         {
-            if (const int st = grow(ctx, &ctx->query_nodes, &ctx->query_nodes_cap, count * 48, "query tree allocation"))
+            // a caller's array is uploaded each call
+            ctx->query_nodes_id = 0;
+            if (const int st = reserve_query_nodes(ctx, count * 48))
                 return st;
-            if (const int st = h2d(ctx, ctx->query_nodes, host_nodes, count * 48))
+            if (const int st = h2d(ctx, ctx->query_nodes, nodes, count * 48))
                 return st;
-            ctx->query_nodes_id = id;
         }
         const size_t ray_bytes = nrays * 24, hit_bytes = nrays * max_hits * 4, count_bytes = nrays * 4;
         const size_t at_hits = (ray_bytes + 255) / 256 * 256, at_counts = at_hits + (hit_bytes + 255) / 256 * 256;

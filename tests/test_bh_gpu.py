@@ -645,3 +645,70 @@ def test_walk_tail_tiles(gpu, n, theta, monkeypatch):
             a, _ = bh_accel(gpu, b, theta=theta, law=0, size=64.0)
             monkeypatch.delenv("NBODY_CUDA_BH_TARGETS")
             assert np.all(np.linalg.norm(a - ref[:, 8:11], axis=1) <= TOL * term_scale(b))
+
+
+def expand_codes(codes, bodies, box):
+    """The exported node array, from its definition: sorted codes, bodies in their order, a block
+    of eight appended when the depth-first walk reaches a split node, octants in reference order.
+    Cells above one body carry no mass here (NaN): their sums are checked elsewhere."""
+    out = []
+
+    def record(level, prefix, nxt):
+        cell = box[3] / 2.0 ** level
+        i = [sum(((prefix >> (3 * k + a)) & 1) << k for k in range(level)) for a in range(3)]
+        return [[np.float32(box[a] + (i[a] + 0.5) * cell) for a in range(3)], np.float32(cell), [0, 0, 0], 0.0, nxt, 0]
+
+    def fill(at, level, prefix, lo, hi):
+        if hi - lo == 0:
+            return
+        if hi - lo == 1:
+            out[at][2], out[at][3] = list(bodies[lo, :3]), bodies[lo, 7]
+            return
+        out[at][2], out[at][3] = [np.nan] * 3, np.nan
+        if level == 21:
+            return
+        block = out[at][5] = len(out)
+        digits = (codes[lo:hi] >> np.uint64(3 * (20 - level))).astype(np.int64) & 7
+        for q in range(8):
+            out.append(record(level + 1, (prefix << 3) | (q ^ 7), block + q + 1 if q < 7 else out[at][4]))
+        for q in range(8):
+            a, b = np.searchsorted(digits, [q ^ 7, (q ^ 7) + 1])
+            fill(block + q, level + 1, (prefix << 3) | (q ^ 7), lo + a, lo + b)
+
+    out.append(record(0, 0, 0))
+    fill(0, 0, 0, 0, len(codes))
+    return out
+
+
+@pytest.mark.parametrize("size,tree_box", [(0.0, 1), (100.0, 0)], ids=["fitted", "fixed"])
+@pytest.mark.parametrize("n", [1, 2, 3, 8, 33, 700])
+def test_tree_export_order(gpu, n, size, tree_box):
+    """Every link, bound and leaf of the exported nodes, in order, with chains of single-child
+    cells (close pairs), coincident bodies (finest-level leaves, alone and as the root) and bodies
+    on the octants' corners."""
+    from nbody_gb300 import scenes
+    b = scenes.plummer(n, seed=n)
+    if n > 3:
+        b[1, :3] = b[0, :3] + np.float32(1e-6)
+        b[2, :3] = b[3, :3]
+        b[n - 1, :3] = 0.0
+    for same in (False, True):
+        if same:
+            b[:, :3] = b[0, :3]
+        with gpu.Context() as ctx:
+            ctx.upload_bodies(b)
+            p = gpu.params(mode=gpu.MODE_NLOGN, theta=0.5, size=size, tree_box=tree_box)
+            codes, order, box = ctx.morton(p)
+            ctx.accelerate(p)
+            nodes = ctx.tree_export()
+        ref = expand_codes(codes, b[order], box)
+        assert len(nodes) == len(ref)
+        assert np.array_equal(nodes["next"], [r[4] for r in ref])
+        assert np.array_equal(nodes["children"], [r[5] for r in ref])
+        assert np.array_equal(nodes["center"], np.array([r[0] for r in ref], np.float32))
+        assert np.array_equal(nodes["size"], np.array([r[1] for r in ref], np.float32))
+        mass = np.array([r[3] for r in ref], np.float32)
+        leaf = ~np.isnan(mass)
+        assert np.array_equal(nodes["mass"][leaf], mass[leaf]) and np.all(nodes["mass"][~leaf] > 0)
+        assert np.array_equal(nodes["com"][leaf], np.array([r[2] for r in ref], np.float32)[leaf])
+        assert not nodes["pad"].any()
