@@ -104,3 +104,18 @@ def test_empty_inputs(gpu):
         assert np.all(c == 0)
         with pytest.raises(gpu.NbodyError):
             ctx.tree_query(np.zeros((1, 6), np.float32), 7, 8, nodes=np.zeros(1, O.NODE_DTYPE))
+
+
+@pytest.mark.parametrize("stop", [0, 1])
+def test_few_and_many_rays_agree(gpu, stop):
+    """A ray's lanes depend on how many rays there are: the same rays, alone and among more than
+    the GPU holds at eight lanes each, meet the same nodes in the same order."""
+    b = scenes.plummer(3000, seed=5)
+    rays = random_rays(513, seed=9)
+    with gpu.Context() as ctx:
+        ctx.upload_bodies(b)
+        ctx.accelerate(gpu.params(mode=gpu.MODE_NLOGN, theta=0.5, law=gpu.LAW_SOFTENED, eps2=1e-4, size=0.0,
+                                  tree_box=1))
+        few, nfew = ctx.tree_query(rays, stop, 64)
+        many, nmany = ctx.tree_query(np.tile(rays, (100, 1)), stop, 64)
+    assert np.array_equal(np.tile(few, (100, 1)), many) and np.array_equal(np.tile(nfew, 100), nmany)
