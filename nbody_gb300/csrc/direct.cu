@@ -74,30 +74,10 @@ namespace nbg
                                               const float2 nz, const float2 lim, float2& ax,
                                               float2& ay, float2& az)
     {
-        if (!PACKED)
-        {
+        if (PACKED)
+            interact_pair<LAW>(sx, sy, sz, sm, nx, ny, nz, lim, ax, ay, az);
+        else
             interact2_scalar<LAW>(sx, sy, sz, sm, nx, ny, nz, lim, ax, ay, az);
-            return;
-        }
-        const float2 dx = add2(sx, nx);
-        const float2 dy = add2(sy, ny);
-        const float2 dz = add2(sz, nz);
-        float2 r2 = (LAW == NBODY_LAW_SOFTENED) ? fma2(dx, dx, lim) : mul2(dx, dx);
-        r2 = fma2(dy, dy, r2);
-        r2 = fma2(dz, dz, r2);
-        float2 inv = make_float2(rsqrt_sfu(r2.x), rsqrt_sfu(r2.y));
-        if (LAW == NBODY_LAW_CUTOFF)
-        {
-            // physics.h:38-39: nothing when |d|^2 <= radius^2 (lim holds radius^2)
-            inv.x = r2.x > lim.x ? inv.x : 0.f;
-            inv.y = r2.y > lim.y ? inv.y : 0.f;
-        }
-        const float2 inv2 = mul2(inv, inv);
-        const float2 mi = mul2(sm, inv);
-        const float2 s = mul2(mi, inv2);
-        ax = fma2(dx, s, ax);
-        ay = fma2(dy, s, ay);
-        az = fma2(dz, s, az);
     }
 
     // Fold one tile's FP32 sums t (two targets) into the thread's (S, C) pair, kept at
@@ -445,6 +425,21 @@ namespace nbg
     DirectPlan plan_direct(const size_t n, const int law, const bool aos, const int force_variant)
     {
         DirectPlan plan{};
+        if (force_variant < 0 && n <= kSmallDirect)
+        {
+            plan.small = true;
+            plan.variant = -1;
+            plan.T = n <= kSmallPair ? 2 : 4;
+            plan.block = kSmallBlock;
+            plan.tile = 32;
+            plan.fold = 1;
+            plan.jsplit = 1;
+            plan.chunk = static_cast<int>(n);
+            plan.grid_x = static_cast<int>(ceil_div(n, 32 * static_cast<size_t>(plan.T))) * kSmallSplit;
+            plan.law = law;
+            plan.aos = aos;
+            return plan;
+        }
         int nv = 0;
         const Variant* vs = variants(&nv);
         const int li = law == NBODY_LAW_SOFTENED ? 1 : 0;
@@ -505,6 +500,7 @@ namespace nbg
         const size_t js = std::max<size_t>(1, (n + chunk - 1) / chunk);
 
         plan.variant = chosen;
+        plan.small = false;
         plan.T = v.T;
         plan.block = v.block;
         plan.tile = kTile;
@@ -524,6 +520,9 @@ namespace nbg
     {
         if (n <= 0)
             return cudaSuccess;
+        if (plan.small)
+            return launch_direct_small(plan, src, vel_radius, acc, plan.aos ? body_out : nullptr, n, G, eps2, stream,
+                                       launches);
         int nv = 0;
         const Variant* vs = variants(&nv);
         const Variant& v = vs[plan.variant];

@@ -9,10 +9,44 @@
 
 namespace nbg
 {
+    // One source (sx, sy, sz, sm) applied to two targets held as negated positions; lim is
+    // their cutoff radius^2, or eps2.
+    template <int LAW>
+    __device__ __forceinline__ void interact_pair(const float2 sx, const float2 sy, const float2 sz, const float2 sm,
+                                                  const float2 nx, const float2 ny, const float2 nz, const float2 lim,
+                                                  float2& ax, float2& ay, float2& az)
+    {
+        const float2 dx = add2(sx, nx);
+        const float2 dy = add2(sy, ny);
+        const float2 dz = add2(sz, nz);
+        float2 r2 = (LAW == NBODY_LAW_SOFTENED) ? fma2(dx, dx, lim) : mul2(dx, dx);
+        r2 = fma2(dy, dy, r2);
+        r2 = fma2(dz, dz, r2);
+        float2 inv = make_float2(rsqrt_sfu(r2.x), rsqrt_sfu(r2.y));
+        if (LAW == NBODY_LAW_CUTOFF)
+        {
+            // physics.h:38-39: nothing when |d|^2 <= radius^2 (lim holds radius^2)
+            inv.x = r2.x > lim.x ? inv.x : 0.f;
+            inv.y = r2.y > lim.y ? inv.y : 0.f;
+        }
+        const float2 inv2 = mul2(inv, inv);
+        const float2 mi = mul2(sm, inv);
+        const float2 s = mul2(mi, inv2);
+        ax = fma2(dx, s, ax);
+        ay = fma2(dy, s, ay);
+        az = fma2(dz, s, az);
+    }
+
+    // Systems small enough for direct_small.cu, and for two targets a lane there (see the kernel).
+    constexpr size_t kSmallDirect = 8192, kSmallPair = 2048;
+    constexpr int kSmallBlock = 256;
+    constexpr int kSmallSplit = 8;      // CTAs a cluster: they share targets and split the sources
+
     // Launch shape of one direct-sum accelerate.
     struct DirectPlan
     {
-        int variant;    // index into the instantiated (targets/thread, block) table
+        int variant;    // index into the instantiated (targets/thread, block) table; -1 when small
+        bool small;     // direct_small.cu's kernel: no scratch, one launch
         int T;          // targets per thread
         int block;      // threads per CTA
         int tile;       // sources per shared-memory tile
@@ -110,6 +144,11 @@ namespace nbg
                               float4* acc, float* body_out, float4* scratch, int n, float G,
                               float eps2, unsigned* err, cudaStream_t stream, uint64_t* launches,
                               bool reduce = true);
+
+    // The same for a plan with small set (direct_small.cu).
+    cudaError_t launch_direct_small(const DirectPlan& plan, const float4* src, const float4* vel_radius, float4* acc,
+                                    float* body_out, int n, float G, float eps2, cudaStream_t stream,
+                                    uint64_t* launches);
 
     cudaError_t launch_reduce(const float4* scratch, int jsplit, int n, float G, float4* acc,
                               float* body_out, cudaStream_t stream, uint64_t* launches);

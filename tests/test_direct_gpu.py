@@ -348,3 +348,44 @@ def test_plain_relative_bar_config1(gpu):
     rel = np.linalg.norm(out[:, 8:11] - a64, axis=1) / np.linalg.norm(a64, axis=1)
     assert np.median(rel) <= 1e-5 and np.percentile(rel, 99) <= 1e-5, (np.median(rel), np.percentile(rel, 99),
                                                                           rel.max())
+
+
+@pytest.mark.parametrize("law", [0, 1], ids=["cutoff", "softened"])
+@pytest.mark.parametrize("layout", [0, 1], ids=["soa", "aos"])
+@pytest.mark.parametrize("n", [1, 2, 31, 63, 64, 65, 127, 129, 500, 2047, 2048, 2049, 4097, 8191, 8192, 8193])
+def test_small_systems(gpu, n, layout, law):
+    """The small systems' kernel at the edges of its slices (64 of them), target blocks (64 and
+    128) and range, and the first size beyond it, against FP64 with the file's bar; repeats are
+    identical, and the accelerate-only and caller-buffer calls give the same bits."""
+    from nbody_gb300 import scenes
+    import torch
+    b = scenes.uniform_cube(n, seed=n)
+    b[:, 3] = np.float32(0.01)
+    b[n // 2, 7] = 0.0
+    if n > 40:
+        b[7, :3] = b[3, :3]
+    eps2 = 1e-6 if law == gpu.LAW_SOFTENED else 0.0
+    p = gpu.params(law=law, eps2=eps2, G=1.5)
+    with gpu.Context(layout) as ctx:
+        ctx.upload_bodies(b)
+        ctx.accelerate(p)
+        out = ctx.download_bodies()
+        ctx.accelerate(p)
+        again = ctx.download_bodies()
+        dev = torch.from_numpy(b).cuda()
+        if layout == gpu.LAYOUT_AOS:
+            ctx.dev_accel_aos(dev.data_ptr(), n, p)
+            ctx.synchronize()
+            mine = dev.cpu().numpy()[:, 8:11]
+        else:
+            pm, vr = dev[:, [0, 1, 2, 7]].contiguous(), dev[:, [4, 5, 6, 3]].contiguous()
+            acc = torch.full_like(pm, 7.0)
+            torch.cuda.synchronize()
+            ctx.dev_accel_soa(pm.data_ptr(), vr.data_ptr(), acc.data_ptr(), n, p)
+            ctx.synchronize()
+            assert not acc[:, 3].any()
+            mine = acc.cpu().numpy()[:, :3]
+    assert np.array_equal(out, again) and np.array_equal(out[:, 8:11], mine)
+    assert np.array_equal(out[:, :8], b[:, :8])
+    err = scaled_err(out[:, 8:11] / np.float32(1.5), b, law, eps2=eps2)
+    assert err.max() <= TOL_MAX and np.median(err) <= TOL_MEDIAN
