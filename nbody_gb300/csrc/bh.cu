@@ -242,6 +242,7 @@ namespace nbg
                                                        const size_t count_a, uint4* __restrict__ zero_b,
                                                        const size_t count_b, BoxParams* __restrict__ box)
     {
+        after_previous();
         for (size_t k = blockIdx.x * 256u + threadIdx.x; k < count_a; k += gridDim.x * 256u)
             zero_a[k] = make_uint4(0u, 0u, 0u, 0u);
         for (size_t k = blockIdx.x * 256u + threadIdx.x; k < count_b; k += gridDim.x * 256u)
@@ -385,6 +386,7 @@ namespace nbg
                                                          const int n, const BoxParams* __restrict__ box,
                                                          uint64_t* __restrict__ keys, uint32_t* __restrict__ vals)
     {
+        after_previous();
         const int base = blockIdx.x * (256 * kMortonItems) + threadIdx.x;
         float4 p[kMortonItems];
 #pragma unroll
@@ -428,6 +430,7 @@ namespace nbg
     __global__ void __launch_bounds__(256) run_sort_kernel(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                                            const int n, unsigned* __restrict__ full)
     {
+        after_previous();
         const int i = blockIdx.x * 256 + threadIdx.x;
         if (i >= n)
             return;
@@ -573,6 +576,7 @@ namespace nbg
         Int64x4* __restrict__ tile_sum, const uint64_t* __restrict__ keys, uint8_t* __restrict__ dl,
         uint64_t* __restrict__ smp)
     {
+        after_previous();
         using Op = ScanOps<Int64x4>;
         if (n <= 0)
             return;
@@ -896,6 +900,7 @@ namespace nbg
         unsigned* __restrict__ far_count, const Int64x4* __restrict__ tile_sum, Int64x4* __restrict__ tile_prefix,
         const int tiles, unsigned* __restrict__ err)
     {
+        after_previous();
         if (blockIdx.x == 0)
         {
             scan_totals(tile_sum, tile_prefix, tiles);
@@ -1028,6 +1033,7 @@ namespace nbg
                                                             int* __restrict__ prefix, uint8_t* __restrict__ flag,
                                                             unsigned* __restrict__ err)
     {
+        after_previous();
         const int count = static_cast<int>(*far_count);
         for (int q = blockIdx.x * 256 + threadIdx.x; q < count; q += gridDim.x * 256)
         {
@@ -1071,6 +1077,7 @@ namespace nbg
                                                           uint32_t* __restrict__ octidx, uint64_t* __restrict__ status,
                                                           unsigned* __restrict__ err)
     {
+        after_previous();
         __shared__ uint32_t warp_tot[32];
         __shared__ uint32_t before_s;
         __shared__ int tile_s;
@@ -1244,6 +1251,7 @@ namespace nbg
                                    OctNode* __restrict__ nodes, unsigned* __restrict__ err,
                                    unsigned long long* __restrict__ stats)
     {
+        after_previous();
         const int gt = blockIdx.x * blockDim.x + threadIdx.x;
         if (gt == 0)
             atomicAdd(&stats[2], static_cast<unsigned long long>((octidx[m - 1] & ~kIsOct) + (octidx[m - 1] >> 31)));
@@ -1486,6 +1494,7 @@ namespace nbg
         const float eps2, float4* __restrict__ acc, float* __restrict__ body_out, unsigned* __restrict__ err,
         unsigned long long* __restrict__ stats)
     {
+        after_previous();
         using Takes = typename TakeBits<H>::Word;
         constexpr int P = (H + 1) / 2;              // target pairs per lane (H = 1: one scalar target)
         constexpr int TW = 32 * H;                  // targets per warp
@@ -1859,6 +1868,7 @@ namespace nbg
         const float eps2, float4* __restrict__ acc, float* __restrict__ body_out, unsigned* __restrict__ err,
         unsigned long long* __restrict__ stats)
     {
+        after_previous();
         constexpr int H = 2 * Q;                    // target slots per lane
         constexpr int TW = 32 * H;                  // targets per group
         static_assert(NSG >= 1 && NSG <= 32, "runs per group");
@@ -2242,6 +2252,18 @@ namespace nbg
         }
     }
 
+    // Launches overlap with the end of the kernel before (launch_after) for up to 2^19 bodies (an
+    // eager build of 262,144 went from 163 to 147 us; of a million, whose kernels fill the GPU,
+    // from 256 to 265), and not in a captured graph: replays of its linear chain were slower so
+    // (a step of 65,536 bodies 178 against 155 us).
+    static bool launch_early(cudaStream_t s, const size_t n)
+    {
+        if (n > (1u << 19))
+            return false;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        return cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    }
+
     int bh_build(nbody_cuda* ctx, const nbody_step_params* p)
     {
         const size_t n = ctx->count;
@@ -2254,18 +2276,19 @@ namespace nbg
         const int ni = static_cast<int>(n);
         uint64_t& L = ctx->launches;
 
+        const bool early = launch_early(s, n);
         // tree_box = 0 is the reference's fixed root box; it needs a positive size
         const bool auto_box = p->tree_box != 0 || !(p->size > 0.f);
         // the bounds pass runs for the fixed box too: the cell sums' scale comes from it
-        bbox_kernel<<<std::min<unsigned>(kBboxBlocks, std::max(1u, ceil_div(n, 1024))), 256, 0, s>>>(
+        launch_after(early, bbox_kernel, std::min<unsigned>(kBboxBlocks, std::max(1u, ceil_div(n, 1024))), 256, 0, s, 
             src, stride, ni, auto_box ? 1 : 0, p->size, b.bbox_part, b.box_ticket, reinterpret_cast<uint4*>(b.stats),
             count_bytes(n) / 16, static_cast<uint4*>(b.temp), sort_zero_bytes(n) / 16, b.box);
         ++L;
-        morton_kernel<<<ceil_div(n, 256 * kMortonItems), 256, 0, s>>>(src, stride, ni, b.box, b.keys[0], b.vals[0]);
+        launch_after(early, morton_kernel, ceil_div(n, 256 * kMortonItems), 256, 0, s, src, stride, ni, b.box, b.keys[0], b.vals[0]);
         ++L;
         bool in_alt = false;
         cudaError_t e = radix_sort_pairs(b.keys[0], b.vals[0], b.keys[1], b.vals[1], n, kRunShift, 63, b.temp, s, &L,
-                                         &in_alt, ctx->dev_error);
+                                         &in_alt, ctx->dev_error, early);
         if (e != cudaSuccess)
             return ctx_cuda_fail(ctx, e, "radix sort");
         if (n > 1)
@@ -2274,7 +2297,7 @@ namespace nbg
             // again by all bits, from the current order (its ties are in index order too)
             const int cur = in_alt ? 1 : 0;
             unsigned* full = reinterpret_cast<unsigned*>(b.stats + 4);
-            run_sort_kernel<<<ceil_div(n, 256), 256, 0, s>>>(b.keys[cur], b.vals[cur], ni, full);
+            launch_after(early, run_sort_kernel, ceil_div(n, 256), 256, 0, s, b.keys[cur], b.vals[cur], ni, full);
             ++L;
             e = radix_sort_if(b.keys[cur], b.vals[cur], b.keys[1 - cur], b.vals[1 - cur], n, 0, 63, b.temp,
                               (63 - kRunShift + 8) / 9, s, &L, ctx->dev_error, full);
@@ -2297,7 +2320,7 @@ namespace nbg
         // (n rounded up to 8 bytes, then n / 64 + 1 keys: within the buffer's 8 n bytes for n >= 2)
         uint64_t* smp = reinterpret_cast<uint64_t*>(dl + ((n + 7) & ~size_t(7)));
         const bool radius = p->law == NBODY_LAW_CUTOFF;
-        gather_sum_kernel<<<tiles, kMomThreads, 0, s>>>(src, stride,
+        launch_after(early, gather_sum_kernel, tiles, kMomThreads, 0, s, src, stride,
                                                         radius && ctx->layout != NBODY_LAYOUT_AOS ? ctx->vr : nullptr,
                                                         order, ni, b.box, b.spm, radius ? b.srad : nullptr, b.psum,
                                                         tile_sum, keys, dl, smp);
@@ -2312,17 +2335,17 @@ namespace nbg
         const int m = ni - 1;
         int* far_list = reinterpret_cast<int*>(b.vals[other]);
         unsigned* far_count = reinterpret_cast<unsigned*>(b.stats + 5);
-        radix_near_kernel<<<1 + ceil_div(m, 256), 256, 0, s>>>(keys, dl, ni, b.child, b.range, b.prefix, b.octflag,
+        launch_after(early, radix_near_kernel, 1 + ceil_div(m, 256), 256, 0, s, keys, dl, ni, b.child, b.range, b.prefix, b.octflag,
                                                                far_list, far_count, tile_sum, tile_prefix,
                                                                static_cast<int>(tiles) + 1, ctx->dev_error);
         ++L;
-        radix_far_kernel<<<std::min(ceil_div(m, 256), 2048u), 256, 0, s>>>(keys, dl, smp, ni, far_list, far_count,
+        launch_after(early, radix_far_kernel, std::min(ceil_div(m, 256), 2048u), 256, 0, s, keys, dl, smp, ni, far_list, far_count,
                                                                               b.child, b.range, b.prefix, b.octflag,
                                                                               ctx->dev_error);
         ++L;
-        number_kernel<<<ceil_div(m, kNumTile), 1024, 0, s>>>(b.octflag, m, b.octidx, b.numbering, ctx->dev_error);
+        launch_after(early, number_kernel, ceil_div(m, kNumTile), 1024, 0, s, b.octflag, m, b.octidx, b.numbering, ctx->dev_error);
         ++L;
-        octnode_kernel<<<ceil_div(m, 256 * kOctSpan), 256, 0, s>>>(b.child, b.range, b.prefix, b.octidx, b.psum,
+        launch_after(early, octnode_kernel, ceil_div(m, 256 * kOctSpan), 256, 0, s, b.child, b.range, b.prefix, b.octidx, b.psum,
                                                                     tile_prefix, m, b.box, p->theta, b.nodes,
                                                                     ctx->dev_error, b.stats);
         ++L;
@@ -2343,6 +2366,7 @@ namespace nbg
         // stage timing: three events on the stream, except while it is captured into a graph
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         bool timed = cudaStreamIsCapturing(ctx->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+        const bool early = launch_early(ctx->stream, n);
         for (int k = 0; k < 3 && timed; ++k)
             timed = ctx->bh->ev[k] || cudaEventCreate(&ctx->bh->ev[k]) == cudaSuccess;
         ctx->bh->timed = false;
@@ -2409,7 +2433,7 @@ namespace nbg
             const Walk fn = fns[gi][long_list ? 1 : 0];
             const int per = per_sm(fn);
             const int grid = std::min((groups + kListWarps - 1) / kListWarps, sms * per);
-            fn<<<grid, kListWarps * 32, 0, s>>>(b.nodes, b.spm, b.srad, b.codes, b.order, ni, p->G, p->eps2, acc,
+            launch_after(early, fn, grid, kListWarps * 32, 0, s, b.nodes, b.spm, b.srad, b.codes, b.order, ni, p->G, p->eps2, acc,
                                                 body_out, ctx->dev_error, b.stats);
             ++ctx->launches;
             if (timed)
@@ -2456,7 +2480,7 @@ namespace nbg
         int grid = std::min((tiles + warps - 1) / warps, sms * per_sm(fi));
         if (grid > 3 * sms)
             grid = grid / sms * sms;    // as many CTAs on every SM
-        fns[fi]<<<grid, warps * 32, 0, s>>>(b.nodes, b.spm, b.srad, b.codes, b.order, ni, p->G, p->eps2, acc, body_out,
+        launch_after(early, fns[fi], grid, warps * 32, 0, s, b.nodes, b.spm, b.srad, b.codes, b.order, ni, p->G, p->eps2, acc, body_out,
                                             ctx->dev_error, b.stats);
         ++ctx->launches;
         if (timed)

@@ -109,6 +109,16 @@ namespace nbg
         asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
     }
 
+    // Programmatic dependent launch: the first statement of every kernel that launch_after
+    // starts. The next kernel of the stream may be made ready as soon as all of this one's CTAs
+    // have begun, and this one goes on once every kernel before it has ended and its writes
+    // are visible: nothing is read or written before that, so only launch latency overlaps.
+    __device__ __forceinline__ void after_previous()
+    {
+        asm volatile("griddepcontrol.launch_dependents;");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+
     // One-dimensional TMA bulk copy global -> shared, completing on `bar` with a byte
     // count. dst, src and bytes must all be multiples of 16.
     __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, const unsigned bytes,
@@ -179,6 +189,24 @@ namespace nbg
         s = add2(a, b);
         const float2 bb = sub2(s, a);
         e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+    }
+
+    // Launches a kernel that begins with after_previous(); early = false launches it as any other.
+    template <typename... Params, typename... Args>
+    cudaError_t launch_after(const bool early, void (*kernel)(Params...), const dim3 grid, const dim3 block,
+                             const size_t smem, cudaStream_t stream, Args&&... args)
+    {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+        cfg.attrs = &at;
+        cfg.numAttrs = early ? 1 : 0;
+        return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
     }
 
     inline unsigned ceil_div(const size_t a, const size_t b) { return static_cast<unsigned>((a + b - 1) / b); }

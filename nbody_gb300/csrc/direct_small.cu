@@ -38,6 +38,7 @@ namespace nbg
         const float4* __restrict__ src, const float4* __restrict__ vel_radius, float4* __restrict__ acc,
         float* __restrict__ body_out, const int n, const float G, const float eps2)
     {
+        after_previous();
         namespace cg = cooperative_groups;
         constexpr int P = T / 2;
         constexpr int REC = AOS ? 3 : 1;
@@ -188,9 +189,8 @@ namespace nbg
               { direct_small_kernel<4, NBODY_LAW_SOFTENED, false>, direct_small_kernel<4, NBODY_LAW_SOFTENED, true> } },
         };
         const dim3 grid(static_cast<unsigned>(plan.grid_x / kSmallSplit), kSmallSplit);
-        fns[plan.T == 4 ? 1 : 0][plan.law == NBODY_LAW_SOFTENED ? 1 : 0][plan.aos ? 1 : 0]
-            <<<grid, kSmallBlock, 0, stream>>>(src, vel_radius, acc, body_out, n, G, eps2);
         ++*launches;
-        return cudaGetLastError();
+        return launch_after(true, fns[plan.T == 4 ? 1 : 0][plan.law == NBODY_LAW_SOFTENED ? 1 : 0][plan.aos ? 1 : 0], grid,
+                            kSmallBlock, 0, stream, src, vel_radius, acc, body_out, n, G, eps2);
     }
 }

@@ -34,6 +34,7 @@ namespace nbg
                                          const int js, const int n, const float G, const float dt,
                                          const float size, const int wrap)
     {
+        after_previous();
         const int t = blockIdx.x * blockDim.x + threadIdx.x;
         const int i = t / W, g = t % W;
         if (W == 1 && i >= n)
@@ -70,6 +71,7 @@ namespace nbg
                                          const int js, const int n, const float G, const float dt,
                                          const float size, const int wrap)
     {
+        after_previous();
         const int t = blockIdx.x * blockDim.x + threadIdx.x;
         const int i = t / W, g = t % W;
         if (W == 1 && i >= n)
@@ -146,10 +148,10 @@ namespace nbg
         if (n <= 0)
             return cudaSuccess;
         if (part && combine_width(n, js) == 8)
-            integrate_soa_kernel<8><<<ceil_div(static_cast<size_t>(n) * 8, kBlock), kBlock, 0, stream>>>(
+            launch_after(true, integrate_soa_kernel<8>, ceil_div(static_cast<size_t>(n) * 8, kBlock), kBlock, 0, stream, 
                 pm, vr, acc, part, js, n, G, dt, size, wrap);
         else
-            integrate_soa_kernel<1><<<ceil_div(n, kBlock), kBlock, 0, stream>>>(pm, vr, acc, part, js, n, G, dt, size,
+            launch_after(true, integrate_soa_kernel<1>, ceil_div(n, kBlock), kBlock, 0, stream, pm, vr, acc, part, js, n, G, dt, size,
                                                                              wrap);
         ++*launches;
         return cudaGetLastError();
@@ -162,10 +164,10 @@ namespace nbg
         if (n <= 0)
             return cudaSuccess;
         if (part && combine_width(n, js) == 8)
-            integrate_aos_kernel<8><<<ceil_div(static_cast<size_t>(n) * 8, kBlock), kBlock, 0, stream>>>(
+            launch_after(true, integrate_aos_kernel<8>, ceil_div(static_cast<size_t>(n) * 8, kBlock), kBlock, 0, stream, 
                 bodies, part, js, n, G, dt, size, wrap);
         else
-            integrate_aos_kernel<1><<<ceil_div(n, kBlock), kBlock, 0, stream>>>(bodies, part, js, n, G, dt, size,
+            launch_after(true, integrate_aos_kernel<1>, ceil_div(n, kBlock), kBlock, 0, stream, bodies, part, js, n, G, dt, size,
                                                                              wrap);
         ++*launches;
         return cudaGetLastError();

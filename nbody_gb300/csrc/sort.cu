@@ -115,6 +115,7 @@ namespace nbg
                                                                       const int shift0, const int passes,
                                                                       uint32_t* __restrict__ ghist)
     {
+        after_previous();
         __shared__ uint32_t hist[kMaxPasses * kDigits];
         histogram(hist, keys, n, shift0, passes, ghist);
     }
@@ -360,6 +361,7 @@ namespace nbg
         const uint32_t* __restrict__ ghist, uint64_t* __restrict__ status, uint32_t* __restrict__ ticket,
         unsigned* __restrict__ err)
     {
+        after_previous();
         extern __shared__ __align__(16) unsigned char smem[];
         digit_pass<false>(smem, keys, vals, keys_out, vals_out, n, shift, pass, ghist, status, ticket, err);
     }
@@ -453,7 +455,8 @@ namespace nbg
 
     cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt,
                                  const size_t n, const int begin_bit, const int end_bit, void* temp,
-                                 cudaStream_t stream, uint64_t* launches, bool* in_alt, unsigned* err)
+                                 cudaStream_t stream, uint64_t* launches, bool* in_alt, unsigned* err,
+                                 const bool early)
     {
         *in_alt = false;
         if (n <= 1)
@@ -469,7 +472,7 @@ namespace nbg
         const int tiles = static_cast<int>((n + kTile - 1) / kTile);
         const TempLayout t = layout(temp, static_cast<size_t>(tiles));
         const int hist_grid = std::max(1, std::min((static_cast<int>(n) + kHistThreads - 1) / kHistThreads, 2 * sm_count()));
-        digit_hist_kernel<<<hist_grid, kHistThreads, 0, stream>>>(keys, static_cast<int>(n), begin_bit, passes, t.ghist);
+        launch_after(early, digit_hist_kernel, hist_grid, kHistThreads, 0, stream, keys, static_cast<int>(n), begin_bit, passes, t.ghist);
         ++*launches;
         cudaError_t e = cudaGetLastError();
         uint64_t* kin = keys;
@@ -478,7 +481,7 @@ namespace nbg
         uint32_t* vout = vals_alt;
         for (int p = 0; p < passes && e == cudaSuccess; ++p)
         {
-            digit_pass_kernel<<<tiles, kThreads, kPassSmem, stream>>>(kin, vin, kout, vout, static_cast<int>(n),
+            launch_after(early, digit_pass_kernel, tiles, kThreads, kPassSmem, stream, kin, vin, kout, vout, static_cast<int>(n),
                                                                       begin_bit + p * kBits, p, t.ghist + p * kDigits,
                                                                       t.status, t.tickets + p, err);
             ++*launches;

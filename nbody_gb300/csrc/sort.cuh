@@ -17,10 +17,10 @@ namespace nbg
     // Sort by bits [begin_bit, end_bit) of the key, 9 bits per pass, ping-ponging between
     // (keys, vals) and (keys_alt, vals_alt). *in_alt tells which pair holds the result.
     // n < 2^31. A look-back wait that gives up (it cannot, unless the device is broken) ORs
-    // DEV_ERR_TIMEOUT into *err.
+    // DEV_ERR_TIMEOUT into *err. early: as in launch_after.
     cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt,
                                  size_t n, int begin_bit, int end_bit, void* temp, cudaStream_t stream,
-                                 uint64_t* launches, bool* in_alt, unsigned* err);
+                                 uint64_t* launches, bool* in_alt, unsigned* err, bool early);
 
     // The same sort in one launch, done only when *run_if is not 0 on the device (the host
     // need not know); the result is in (keys, vals). For a call after radix_sort_pairs on the
