@@ -16,7 +16,7 @@
 //   4. gather_sum_kernel: bodies into Morton order, and exact fixed-point (int64) prefix
 //      sums of m and m*x within tiles of sorted bodies, plus a scan of the tile totals:
 //      differences of their sums give each cell's mass and COM;
-//   5. adjacent_prefix_kernel, radix_near_kernel, radix_far_kernel: binary radix tree over
+//   5. radix_tree_kernel, from prefix bytes of gather_sum_kernel: binary radix tree over
 //      the sorted codes (Karras 2012), duplicates separated by index; each internal node's
 //      common-prefix length fixes its octree level floor(prefix / 3) (capped at 21, the
 //      last Morton level), and the node is flagged as an octree node here;
@@ -756,10 +756,11 @@ namespace nbg
     // adjacent prefixes stay above dmin = delta(i, i - d), so its far end is the first byte
     // of dl beyond i (in that direction) that is <= dmin: 16 bytes are compared at a time.
     // Its split is the one position of its range's least prefix, dnode = delta(i, j): the
-    // first byte equal to dnode from the range's low end. A node whose end lies farther goes
-    // to far_list for radix_far_kernel, so that no warp waits on one lane's long search
-    // (Karras's searches for every node took 0.47 ms at 16.8M bodies; these kernels and the
-    // prefix bytes take about 0.37).
+    // first byte equal to dnode from the range's low end. A node whose end lies farther is
+    // found by eight lanes together (radix_tree_kernel): a lane's own search, 40 dependent
+    // loads for the top levels' nodes, cost a second kernel 14 to 20 us at 65,536 to 262,144
+    // bodies. In one kernel with the searches shared a step of 65,536 bodies takes 144 us (155),
+    // of 262,144 203 (217), of 1,000,003 423 (433), of 16.8M 4,550 (4,533).
     constexpr int kNearScan = 64;
     constexpr int kNearChunks = kNearScan / 16 + 1;
 
@@ -894,11 +895,112 @@ namespace nbg
         }
     }
 
-    __global__ void __launch_bounds__(256) radix_near_kernel(
-        const uint64_t* __restrict__ keys, const uint8_t* __restrict__ dl, const int n, int2* __restrict__ child,
-        int2* __restrict__ range, int* __restrict__ prefix, uint8_t* __restrict__ flag, int* __restrict__ far_list,
-        unsigned* __restrict__ far_count, const Int64x4* __restrict__ tile_sum, Int64x4* __restrict__ tile_prefix,
-        const int tiles, unsigned* __restrict__ err)
+    __device__ __forceinline__ int delta_of(const uint64_t a, const int i, const uint64_t b, const int j)
+    {
+        return a != b ? __clzll(static_cast<long long>(a ^ b))
+                      : 64 + __clz(static_cast<int>(static_cast<unsigned>(i) ^ static_cast<unsigned>(j)));
+    }
+
+    // How many of a monotone predicate's values on eight lanes hold: true on the first ones,
+    // false from there. Every lane of the warp calls it.
+    __device__ __forceinline__ int count_leading(const bool t, const int lane)
+    {
+        const unsigned b = ~(__ballot_sync(0xffffffffu, t) >> (lane & 24)) & 0xffu;
+        return b ? __ffs(b) - 1 : 8;
+    }
+
+    // Searches of four nodes by a warp, eight lanes each. For sorted keys dl[ref .. P - 1] > D exactly
+    // when the common prefix of keys ref and P exceeds D, so a coarse search over every 64th key
+    // (the samples, 1/64 of the keys, stay in the caches) finds the last sample P for which it
+    // does: eight powers of two at once, then eight points of the bracket at once. The answer
+    // lies in the 64 bytes after it, which the lanes compare 16 each.
+    //
+    // The first p >= start with dl[p] <= D (n - 1 when none: past the last pair), given
+    // dl[ref .. start - 1] > D and kref = key ref.
+    __device__ __forceinline__ int first_le_up(const uint64_t* __restrict__ smp, const uint8_t* __restrict__ dl,
+                                               const int n, const uint64_t kref, const int ref, const int start,
+                                               const int D, const int lane, unsigned* __restrict__ err)
+    {
+        const int sub = lane & 7, ka = (start >> 6) + 1;
+        auto f = [&](const int k) { return k < (n + 62) / 64 && delta_of(kref, ref, smp[k], 64 * k) > D; };
+        int e = 0;
+        for (bool open = true; __any_sync(0xffffffffu, open);)
+        {
+            const int c = count_leading(open && e + sub < 25 && f(ka + (1 << (e + sub)) - 1), lane);
+            e += open ? c : 0;
+            open = open && c == 8;
+        }
+        int lo = e ? ka + (1 << (e - 1)) - 1 : 0, hi = e ? ka + (1 << e) - 1 : 0;
+        while (__any_sync(0xffffffffu, hi - lo > 1))
+        {
+            const int stride = (hi - lo + 7) / 8, k = lo + (sub + 1) * stride;
+            const int held = count_leading(k < hi && f(k), lane);
+            hi = min(hi, lo + (held + 1) * stride);
+            lo += held * stride;
+        }
+        const int q0 = e ? 64 * lo : start;
+        const int base = (q0 & ~15) + 16 * sub;
+        uint32_t mk = base < n - 1
+                          ? lt_mask16(*reinterpret_cast<const uint4*>(dl + base), static_cast<uint32_t>(D + 1) * 0x01010101u)
+                          : 0u;
+        if (sub == 0)
+            mk &= ~((1u << (q0 & 15)) - 1u);
+        const int past = n - 1 - base;      // bytes from here on are past the last pair
+        if (past < 16)
+            mk |= past <= 0 ? 0xffffu : (0xffffu << past) & 0xffffu;
+        const unsigned any = (__ballot_sync(0xffffffffu, mk != 0u) >> (lane & 24)) & 0xffu;
+        if (!any)
+            atomicOr(err, DEV_ERR_BOUNDS);      // not sorted keys
+        const int p = __shfl_sync(0xffffffffu, base + __ffs(mk) - 1, any ? __ffs(any) - 1 : 0, 8);
+        return any ? p : n - 1;
+    }
+
+    // The last p <= start with dl[p] <= D (-1 when none), given dl[start + 1 .. ref - 1] > D.
+    __device__ __forceinline__ int last_le_down(const uint64_t* __restrict__ smp, const uint8_t* __restrict__ dl,
+                                                const uint64_t kref, const int ref, const int start, const int D,
+                                                const int lane, unsigned* __restrict__ err)
+    {
+        const int sub = lane & 7, ka = start >> 6;
+        auto f = [&](const int k) { return k >= 0 && delta_of(kref, ref, smp[k], 64 * k) > D; };
+        int e = 0;
+        for (bool open = true; __any_sync(0xffffffffu, open);)
+        {
+            const int c = count_leading(open && e + sub < 25 && f(ka - (1 << (e + sub)) + 1), lane);
+            e += open ? c : 0;
+            open = open && c == 8;
+        }
+        int hi = e ? ka - (1 << (e - 1)) + 1 : 0, lo = e ? ka - (1 << e) + 1 : 0;
+        while (__any_sync(0xffffffffu, hi - lo > 1))
+        {
+            const int stride = (hi - lo + 7) / 8, k = hi - (sub + 1) * stride;
+            const int held = count_leading(k > lo && f(k), lane);
+            lo = max(lo, hi - (held + 1) * stride);
+            hi -= held * stride;
+        }
+        const int q0 = e ? 64 * hi - 1 : start;
+        const int base = (q0 & ~15) - 16 * sub;
+        uint32_t mk = 0;
+        if (q0 >= 0 && base >= 0)
+        {
+            mk = lt_mask16(*reinterpret_cast<const uint4*>(dl + base), static_cast<uint32_t>(D + 1) * 0x01010101u);
+            if (sub == 0)
+                mk &= (2u << (q0 & 15)) - 1u;
+        }
+        const unsigned any = (__ballot_sync(0xffffffffu, mk != 0u) >> (lane & 24)) & 0xffu;
+        if (!any && q0 >= 128)
+            atomicOr(err, DEV_ERR_BOUNDS);      // not sorted keys
+        const int p = __shfl_sync(0xffffffffu, base + 31 - __clz(mk), any ? __ffs(any) - 1 : 0, 8);
+        return any ? p : -1;
+    }
+
+    // Block 0 scans the tile sums, the others take 256 nodes each: near ones a lane each, then
+    // the CTA's far ones (six of 256 at 16.8M bodies) four a warp, so that few warps stay for
+    // their dependent loads (each warp searching for its own far nodes took 2 % longer there).
+    __global__ void __launch_bounds__(256) radix_tree_kernel(
+        const uint64_t* __restrict__ keys, const uint8_t* __restrict__ dl, const uint64_t* __restrict__ smp, const int n,
+        int2* __restrict__ child, int2* __restrict__ range, int* __restrict__ prefix, uint8_t* __restrict__ flag,
+        const Int64x4* __restrict__ tile_sum, Int64x4* __restrict__ tile_prefix, const int tiles,
+        unsigned* __restrict__ err)
     {
         after_previous();
         if (blockIdx.x == 0)
@@ -908,153 +1010,49 @@ namespace nbg
         }
         const int i = (blockIdx.x - 1) * 256 + threadIdx.x;
         const bool far = i < n - 1 && near_node(keys, dl, n, i, child, range, prefix, flag, err);
-        // a warp's far nodes take consecutive slots of far_list: one global atomic a warp
+        // the CTA's nodes whose ranges end too far for the byte scans, eight lanes each
+        __shared__ int far_node[256];
+        __shared__ unsigned far_count;
+        const int lane = threadIdx.x & 31;
+        if (threadIdx.x == 0)
+            far_count = 0;
+        __syncthreads();
         const unsigned fm = __ballot_sync(0xffffffffu, far);
-        if (!fm)
-            return;
-        const int lane = threadIdx.x & 31, leader = __ffs(fm) - 1;
-        unsigned base = 0;
-        if (lane == leader)
-            base = atomicAdd(far_count, static_cast<unsigned>(__popc(fm)));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (far)
-            far_list[base + __popc(fm & ((1u << lane) - 1u))] = i;
-    }
-
-    __device__ __forceinline__ int delta_of(const uint64_t a, const int i, const uint64_t b, const int j)
-    {
-        return a != b ? __clzll(static_cast<long long>(a ^ b))
-                      : 64 + __clz(static_cast<int>(static_cast<unsigned>(i) ^ static_cast<unsigned>(j)));
-    }
-
-    // The first p >= start with dl[p] <= D (n - 1 when none: past the last pair), given
-    // dl[ref .. start - 1] > D and kref = key ref. A coarse search over every 64th key finds
-    // the last sampled position P with delta(ref, P) > D, that is dl[ref .. P - 1] > D
-    // (exponential, then binary); the answer lies in the 64 bytes after it, found by the
-    // byte scan. The samples are 1/64 of the keys and stay in the caches.
-    __device__ int first_le_up(const uint64_t* __restrict__ smp, const uint8_t* __restrict__ dl, const int n,
-                               const uint64_t kref, const int ref, const int start, const int D,
-                               unsigned* __restrict__ err)
-    {
-        auto f = [&](const int k) {
-            const int P = 64 * k;
-            return P < n - 1 && delta_of(kref, ref, smp[k], P) > D;
-        };
-        int q0 = start;
-        const int ka = (start >> 6) + 1;
-        if (f(ka))
+        if (fm)
         {
-            int lo = ka, step = 1;
-            while (f(lo + step))
-            {
-                lo += step;
-                step <<= 1;
-            }
-            int hi = lo + step;
-            while (hi - lo > 1)
-            {
-                const int mid = (lo + hi) >> 1;
-                if (f(mid))
-                    lo = mid;
-                else
-                    hi = mid;
-            }
-            q0 = 64 * lo;
+            unsigned at = lane == 0 ? atomicAdd(&far_count, static_cast<unsigned>(__popc(fm))) : 0u;
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (far)
+                far_node[at + __popc(fm & ((1u << lane) - 1u))] = i;
         }
-        const uint32_t lim = static_cast<uint32_t>(D + 1) * 0x01010101u;      // bytes <= D
-        for (int c = 0; c < 8; ++c)
+        __syncthreads();
+        const unsigned count = far_count;
+        for (unsigned q = (threadIdx.x >> 5) * 4; q < count; q += 32)
         {
-            const int base = (q0 & ~15) + 16 * c;
-            uint32_t mk = base < n - 1 ? lt_mask16(*reinterpret_cast<const uint4*>(dl + base), lim) : 0u;
-            if (c == 0)
-                mk &= ~((1u << (q0 & 15)) - 1u);
-            const int past = n - 1 - base;
-            if (past < 16)
-                mk |= past <= 0 ? 0xffffu : (0xffffu << past) & 0xffffu;
-            if (mk)
-                return base + __ffs(mk) - 1;
-        }
-        atomicOr(err, DEV_ERR_BOUNDS);      // not sorted keys
-        return n - 1;
-    }
-
-    // The last p <= start with dl[p] <= D (-1 when none), given dl[start + 1 .. ref - 1] > D;
-    // the same coarse search downward (delta(ref, P) > D means dl[P .. ref - 1] > D).
-    __device__ int last_le_down(const uint64_t* __restrict__ smp, const uint8_t* __restrict__ dl, const uint64_t kref,
-                                const int ref, const int start, const int D, unsigned* __restrict__ err)
-    {
-        auto f = [&](const int k) { return k >= 0 && delta_of(kref, ref, smp[k], 64 * k) > D; };
-        int q0 = start;
-        const int ka = start >> 6;
-        if (f(ka))
-        {
-            int hi = ka, step = 1;
-            while (f(hi - step))
-            {
-                hi -= step;
-                step <<= 1;
-            }
-            int lo = hi - step;
-            while (hi - lo > 1)
-            {
-                const int mid = (lo + hi) >> 1;
-                if (f(mid))
-                    hi = mid;
-                else
-                    lo = mid;
-            }
-            q0 = 64 * hi - 1;
-        }
-        const uint32_t lim = static_cast<uint32_t>(D + 1) * 0x01010101u;
-        for (int c = 0; c < 8; ++c)
-        {
-            const int base = (q0 & ~15) - 16 * c;
-            if (q0 < 0 || base < 0)
-                return -1;
-            uint32_t mk = lt_mask16(*reinterpret_cast<const uint4*>(dl + base), lim);
-            if (c == 0)
-                mk &= (2u << (q0 & 15)) - 1u;
-            if (mk)
-                return base + 31 - __clz(mk);
-        }
-        atomicOr(err, DEV_ERR_BOUNDS);
-        return -1;
-    }
-
-    // The nodes radix_near_kernel passed on, one per thread: the range's far end and the
-    // split by the coarse-then-fine searches above (the top levels' nodes span millions of
-    // keys; their searches over the samples stay in the caches).
-    __global__ void __launch_bounds__(256) radix_far_kernel(const uint64_t* __restrict__ keys,
-                                                            const uint8_t* __restrict__ dl,
-                                                            const uint64_t* __restrict__ smp, const int n,
-                                                            const int* __restrict__ far_list,
-                                                            const unsigned* __restrict__ far_count,
-                                                            int2* __restrict__ child, int2* __restrict__ range,
-                                                            int* __restrict__ prefix, uint8_t* __restrict__ flag,
-                                                            unsigned* __restrict__ err)
-    {
-        after_previous();
-        const int count = static_cast<int>(*far_count);
-        for (int q = blockIdx.x * 256 + threadIdx.x; q < count; q += gridDim.x * 256)
-        {
-            const int i = far_list[q];
-            const uint64_t ki = keys[i];
-            const int dr = dl[i];
-            const int dlf = i > 0 ? static_cast<int>(dl[i - 1]) : -1;
+            // (a group past the last one repeats it, and writes nothing)
+            const bool mine = q + (lane >> 3) < count;
+            const int node = far_node[min(q + (lane >> 3), count - 1)];
+            const int dr = dl[node];
+            const int dlf = node > 0 ? static_cast<int>(dl[node - 1]) : -1;
             const int d = dr - dlf >= 0 ? 1 : -1;
             const int dmin = d > 0 ? dlf : dr;
-            const int j = d > 0 ? first_le_up(smp, dl, n, ki, i, i, dmin, err)
-                                : last_le_down(smp, dl, ki, i, i - 1, dmin, err) + 1;
-            const int lo = min(i, j), hi = max(i, j);
-            const int dnode = delta(keys, n, i, j);
-            const int gamma = first_le_up(smp, dl, n, keys[lo], lo, lo, dnode, err);
-            if (gamma < lo || gamma >= hi)
+            // every lane makes both searches' calls; a group's other one ends at once
+            const uint64_t ki = keys[node];
+            const int up = first_le_up(smp, dl, n, ki, node, node, d > 0 ? dmin : 95, lane, err);
+            const int down = last_le_down(smp, dl, ki, node, node - 1, d > 0 ? 95 : dmin, lane, err) + 1;
+            const int j = d > 0 ? up : down;
+            const int lo = min(node, j), hi = max(node, j);
+            const int dnode = delta(keys, n, node, j);
+            const int gamma = first_le_up(smp, dl, n, keys[lo], lo, lo, dnode, lane, err);
+            if (mine && (lane & 7) == 0)
             {
-                atomicOr(err, DEV_ERR_BOUNDS);
-                continue;
+                const int dfar = d > 0 ? (j < n - 1 ? static_cast<int>(dl[j]) : -1)
+                                       : (j > 0 ? static_cast<int>(dl[j - 1]) : -1);
+                if (gamma < lo || gamma >= hi)
+                    atomicOr(err, DEV_ERR_BOUNDS);
+                else
+                    write_radix_node(node, lo, hi, gamma, dnode, dmin, dfar, child, range, prefix, flag);
             }
-            const int dfar = d > 0 ? (j < n - 1 ? static_cast<int>(dl[j]) : -1) : (j > 0 ? static_cast<int>(dl[j - 1]) : -1);
-            write_radix_node(i, lo, hi, gamma, dnode, dmin, dfar, child, range, prefix, flag);
         }
     }
 
@@ -2333,15 +2331,8 @@ namespace nbg
             return NBODY_OK;
         }
         const int m = ni - 1;
-        int* far_list = reinterpret_cast<int*>(b.vals[other]);
-        unsigned* far_count = reinterpret_cast<unsigned*>(b.stats + 5);
-        launch_after(early, radix_near_kernel, 1 + ceil_div(m, 256), 256, 0, s, keys, dl, ni, b.child, b.range, b.prefix, b.octflag,
-                                                               far_list, far_count, tile_sum, tile_prefix,
-                                                               static_cast<int>(tiles) + 1, ctx->dev_error);
-        ++L;
-        launch_after(early, radix_far_kernel, std::min(ceil_div(m, 256), 2048u), 256, 0, s, keys, dl, smp, ni, far_list, far_count,
-                                                                              b.child, b.range, b.prefix, b.octflag,
-                                                                              ctx->dev_error);
+        launch_after(early, radix_tree_kernel, 1 + ceil_div(m, 256), 256, 0, s, keys, dl, smp, ni, b.child, b.range,
+                     b.prefix, b.octflag, tile_sum, tile_prefix, static_cast<int>(tiles) + 1, ctx->dev_error);
         ++L;
         launch_after(early, number_kernel, ceil_div(m, kNumTile), 1024, 0, s, b.octflag, m, b.octidx, b.numbering, ctx->dev_error);
         ++L;

@@ -712,3 +712,28 @@ def test_tree_export_order(gpu, n, size, tree_box):
         assert np.array_equal(nodes["mass"][leaf], mass[leaf]) and np.all(nodes["mass"][~leaf] > 0)
         assert np.array_equal(nodes["com"][leaf], np.array([r[2] for r in ref], np.float32)[leaf])
         assert not nodes["pad"].any()
+
+
+@pytest.mark.parametrize("n", [65, 66, 129, 193, 1025, 4097])
+def test_tree_of_nodes_with_far_ends(gpu, n):
+    """Binary nodes whose ranges end 64 keys and more away, in either direction and up to the
+    arrays' ends: a tight cluster at the box's low corner, one at its high corner, coincident
+    bodies, and a few strays between. Every link of the exported tree has one right value."""
+    rng = np.random.default_rng(n)
+    from nbody_gb300 import scenes
+    b = scenes.plummer(n, seed=n)
+    third = n // 3
+    b[:, :3] = rng.random((n, 3), dtype=np.float32) * 100
+    b[:third, :3] *= np.float32(1e-3)
+    b[third:2 * third, :3] = np.float32(100) - b[third:2 * third, :3] * np.float32(1e-3)
+    b[2 * third:2 * third + third // 2, :3] = b[2 * third, :3]
+    with gpu.Context() as ctx:
+        ctx.upload_bodies(b)
+        p = gpu.params(mode=gpu.MODE_NLOGN, theta=0.5, size=0.0, tree_box=1)
+        codes, order, box = ctx.morton(p)
+        ctx.accelerate(p)
+        nodes = ctx.tree_export()
+    ref = expand_codes(codes, b[order], box)
+    assert len(nodes) == len(ref)
+    assert np.array_equal(nodes["next"], [r[4] for r in ref])
+    assert np.array_equal(nodes["children"], [r[5] for r in ref])
