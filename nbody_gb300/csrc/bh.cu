@@ -63,12 +63,21 @@ namespace nbg
         // group walk: warps per CTA, list entries and stacked parent cells per warp (the
         // stack grows by at most 28 parents per tree level, 22 levels: 616 < 768)
         constexpr int kListWarps = 4;
-        // interaction-list entries per warp: the long list (8 KB; five CTAs per SM) drains half
-        // as often, the short one (4 KB; six CTAs) keeps more warps resident when the groups
-        // are too few to fill them
+        // interaction-list entries per warp: the long list (8 KB) drains half as often, the short
+        // one (4 KB) keeps more warps resident when the groups are too few to fill them
         constexpr int kListLong = 512;
         constexpr int kListShort = 256;
+        // CTAs per SM of the group walk with Q target pairs per lane: two pairs want 128 registers
+        // for the list's loop (halo of 16.8M bodies: 41.0 ms at five CTAs, 37.8 at four, 40.8 at
+        // three of 168), one pair is fastest with more warps (1M-body disk: 344 us at five, 377 at four)
+        __host__ __device__ constexpr int list_ctas(const int q, const int cap)
+        {
+            return q == 4 ? 3 : (q == 2 ? 4 : (cap > kListShort ? 5 : 6));
+        }
         constexpr int kGroupStack = 768;
+        // parents stacked up to which a round's parents are taken a round ahead: 120 - 1 + 32, and
+        // 616 from there, stay within the stack
+        constexpr int kGroupAhead = 120;
         constexpr int kRuns = 4;            // runs (own acceptance boxes) per group
         constexpr int kBboxBlocks = 1024;
         constexpr int kBboxVals = 8;    // min x y z, max x y z, max |m|, max |x|
@@ -1822,6 +1831,21 @@ namespace nbg
         az = fma2(dz, sc, az);
     }
 
+    // Loads that stay where they are written, ahead of the work that hides them.
+    __device__ __forceinline__ int load_ahead(const int* p)
+    {
+        int v;
+        asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(p));
+        return v;
+    }
+
+    __device__ __forceinline__ float4 load_ahead(const float4* p)
+    {
+        float4 v;
+        asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+        return v;
+    }
+
     // The reference's opening test (bhtree.cpp:117-125) for a box of targets: the cell is
     // accepted when the nearest point of the box lies beyond its opening distance,
     // |com - p|^2 > size^2 * theta^2. Every target in the box is at least that far from the
@@ -1854,13 +1878,20 @@ namespace nbg
     //
     // The walk tests up to 32 cells at a time: it pops up to four opened parent cells from a
     // stack, and lane l tests child l % 8 of parent l / 8. The stack grows by at most 28
-    // parents per tree level (22 levels: 616 < kGroupStack).
+    // parents per tree level (22 levels: 616 < kGroupStack). A round's parents are popped before
+    // the round ahead of it pushes its own, and its cells' records loaded before that one's
+    // list is applied, so that only a nearly empty stack waits for its loads; while more than
+    // kGroupAhead parents are stacked they are popped after the pushes, which bounds the stack
+    // as before. The list's loop is FP32-pipe work (24 instructions a source and two pairs);
+    // unrolled 16 times the pipe waits less between its iterations (2 times: 3 to 20 % longer).
+    // Walk alone, before and now: 16.8M halo bodies, theta 2: 41.6 -> 37.8 ms; 1M: 2.62 -> 2.30;
+    // two Plummer spheres of 131,072 bodies, theta 2: 797 -> 670 us; of 10,000, theta 0.5: 119 -> 78 us.
     //
     // Each target's sources refine the cells the reference's walk accepts for it alone (a
     // cell opened for the group may be one the target would have accepted), so each target
     // is summed at least as finely as in the reference, over more interactions.
     template <int LAW, int Q, int NSG, int CAP>
-    __global__ void __launch_bounds__(kListWarps * 32) traverse_list_kernel(
+    __global__ void __launch_bounds__(kListWarps * 32, list_ctas(Q, CAP)) traverse_list_kernel(
         const OctNode* __restrict__ nodes, const float4* __restrict__ spm, const float* __restrict__ srad,
         const uint64_t* __restrict__ codes, const uint32_t* __restrict__ order, const int n, const float G,
         const float eps2, float4* __restrict__ acc, float* __restrict__ body_out, unsigned* __restrict__ err,
@@ -1995,7 +2026,7 @@ namespace nbg
             // apply the whole list to every target of the group, then empty it
             auto drain = [&]() {
                 __syncwarp();
-#pragma unroll 2
+#pragma unroll 16
                 for (int e = 0; e < ln; ++e)
                 {
                     const float4 s = list[e];
@@ -2057,11 +2088,35 @@ namespace nbg
                 }
             }
             __syncwarp();
+            // the lane's child of the next (up to four) parents off the stack; 0: none (cell 0 is
+            // the root, never a child)
+            auto pop = [&]() {
+                const int slot = lane >> 3;
+                const int c = slot < sp ? load_ahead(&nodes[stk[sp - 1 - slot]].child[lane & 7]) : 0;
+                sp -= min(sp, 4);
+                return c;
+            };
+            float4 src;             // a child's (com, mass), or a leaf's (x, m)
+            float4 meta;            // a cell's open_r2, nchild, first, last
+            auto load = [&](const int c) {
+                src = make_float4(0.f, 0.f, 0.f, 0.f);
+                meta = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (c < 0)
+                    src = load_ahead(spm + ~c);
+                else if (c > 0)
+                {
+                    src = load_ahead(&nodes[c].com_mass);
+                    meta = load_ahead(reinterpret_cast<const float4*>(&nodes[c].open_r2));
+                }
+            };
+            bool more = sp > 0;
+            int c = more ? pop() : 0;
+            load(c);
             // Each cell is pushed at most once per group, so the walk takes at most one
             // round per cell (< n); the bound only trips on a malformed tree.
             int guard = 0;
             const int guard_limit = n + 64;
-            while (sp > 0)
+            while (more)
             {
                 if (++guard > guard_limit)
                 {
@@ -2070,39 +2125,18 @@ namespace nbg
                     break;
                 }
                 ++iters;
-                const int k = min(sp, 4);
-                const int slot = lane >> 3;
-                int c = 0;              // 0: no child (cell 0 is the root, never a child)
-                if (slot < k)
-                    c = nodes[stk[sp - 1 - slot]].child[lane & 7];
+                const bool ahead = sp > 0 && sp <= kGroupAhead;
+                int cn = ahead ? pop() : 0;
+                // empty cells are skipped (bhtree.cpp:109-113); a leaf is always applied
+                // (bhtree.cpp:115-116)
+                const bool cell = c > 0 && src.w != 0.f;
+                const bool taken = cell && accepts(src, meta.x);
+                const bool bucket = cell && !taken && __float_as_int(meta.y) < 0;
+                const bool push = cell && !taken && !bucket;
+                const bool take = c < 0 ? src.w != 0.f : taken;
+                const float4 from = src;
+                const int first = __float_as_int(meta.z), last = __float_as_int(meta.w);
                 __syncwarp();           // every parent read before pushes overwrite its slot
-                sp -= k;
-                bool take = false, push = false, bucket = false;
-                float4 src = make_float4(0.f, 0.f, 0.f, 0.f);
-                int4 meta = make_int4(0, 0, 0, 0);
-                if (c < 0)
-                {
-                    src = spm[~c];      // a leaf: always applied (bhtree.cpp:115-116)
-                    take = src.w != 0.f;
-                }
-                else if (c > 0)
-                {
-                    const float4 cm = nodes[c].com_mass;
-                    meta = *reinterpret_cast<const int4*>(&nodes[c].open_r2);
-                    if (cm.w != 0.f)    // empty cells are skipped (bhtree.cpp:109-113)
-                    {
-                        if (accepts(cm, __int_as_float(meta.x)))
-                        {
-                            src = cm;
-                            take = true;
-                        }
-                        else if (meta.y < 0)
-                            bucket = true;
-                        else
-                            push = true;
-                    }
-                }
-                append(take, src);
                 const unsigned pm = __ballot_sync(0xffffffffu, push);
                 if (push)
                 {
@@ -2113,14 +2147,18 @@ namespace nbg
                         atomicOr(err, DEV_ERR_BOUNDS);
                 }
                 sp = min(kGroupStack, sp + __popc(pm));
+                __syncwarp();
+                more = ahead || sp > 0;
+                c = !ahead && more ? pop() : cn;
+                load(c);
+                append(take, from);
                 unsigned bm = __ballot_sync(0xffffffffu, bucket);
                 while (bm)
                 {
                     const int bl = __ffs(bm) - 1;
                     bm &= bm - 1;
-                    append_range(__shfl_sync(0xffffffffu, meta.z, bl), __shfl_sync(0xffffffffu, meta.w, bl));
+                    append_range(__shfl_sync(0xffffffffu, first, bl), __shfl_sync(0xffffffffu, last, bl));
                 }
-                __syncwarp();
             }
             drain();
 #pragma unroll
@@ -2388,8 +2426,9 @@ namespace nbg
         if (p->walk == NBODY_WALK_GROUP)
         {
             // Group walk: 128 targets per group (4 per lane) while the groups outnumber the
-            // resident warps, else 64. NBODY_CUDA_BH_GROUP (64, 128 or 256) overrides; the
-            // group size changes which cells each target applies, not the bar they meet.
+            // warps of six CTAs an SM (five under the cutoff law), else 64. NBODY_CUDA_BH_GROUP (64,
+            // 128 or 256) overrides; the group size changes which cells each target applies, not the
+            // bar they meet, so the line is fixed and does not follow the kernels' occupancy.
             const bool soft = p->law == NBODY_LAW_SOFTENED;
             using Walk = void (*)(const OctNode*, const float4*, const float*, const uint64_t*, const uint32_t*, int,
                                   float, float, float4*, float*, unsigned*, unsigned long long*);
@@ -2416,7 +2455,7 @@ namespace nbg
             const char* gsel = std::getenv("NBODY_CUDA_BH_GROUP");
             int group = gsel ? std::atoi(gsel) : 0;
             if (group != 64 && group != 128 && group != 256)
-                group = static_cast<long long>(ni) >= 128LL * per_sm(fns[1][0]) * sms * kListWarps ? 128 : 64;
+                group = static_cast<long long>(ni) >= 128LL * (soft ? 6 : 5) * sms * kListWarps ? 128 : 64;
             const int gi = group == 256 ? 2 : (group == 128 ? 1 : 0);
             const int groups = (ni + group - 1) / group;
             // the long list once the groups are at least twice the warps it leaves resident

@@ -189,3 +189,21 @@ def test_unknown_walk_rejected(gpu):
         with pytest.raises(gpu.NbodyError) as e:
             ctx.accelerate(gpu.params(mode=gpu.MODE_NLOGN, walk=7))
         assert e.value.status == gpu.ERR_INVALID
+
+
+@pytest.mark.parametrize("group", [64, 128, 256])
+@pytest.mark.parametrize("n", [31, 65, 257, 2049, 100003])
+def test_group_walk_opens_every_cell(gpu, n, group, monkeypatch):
+    """An opening angle at which no cell is accepted: every group's list is every body, once
+    (the interactions are n * n), at list lengths around the loop's unrolling and with stacks
+    short and long. Each sum is then the direct sum: within n + 16 roundings of the terms."""
+    from nbody_gb300 import scenes
+    monkeypatch.setenv("NBODY_CUDA_BH_GROUP", str(group))
+    rng = np.random.default_rng(n)
+    b = scenes.plummer(n, seed=n)
+    b[:, :3] = rng.random((n, 3), dtype=np.float32) * 10
+    acc, stats = accel(gpu, b, gpu.WALK_GROUP, theta=1e4, law=gpu.LAW_SOFTENED, eps2=1e-4, size=0.0, tree_box=1)
+    assert stats["interactions"] == n * n
+    tg = np.unique(rng.integers(0, n, 200))
+    a64, scale = O.direct_f64(b[:, [0, 1, 2, 7]], 1.0, float(np.float32(1e-4)), O.LAW_SOFTENED, targets=tg, with_scale=True)
+    assert np.all(np.linalg.norm(acc[tg] - a64, axis=1) <= (n + 16) * 2.0**-24 * scale)
