@@ -29,6 +29,7 @@
 //     launch shape (up to a rounding tie of the last fold), and it is more accurate than
 //     one FP32 running sum over all N sources.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 
 #include "common.cuh"
@@ -100,8 +101,14 @@ namespace nbg
 
     // DUP: each landed tile is first rewritten in shared memory as source pairs {x,x,y,y},
     // {z,z,m,m}, so the inner loop reads the packed operands ready-made (two 16-byte loads)
-    // instead of broadcasting each scalar into a register pair.
-    template <int T, int BLOCK, int TILE, int STAGES, int LAW, bool AOS, bool PACKED = true, bool DUP = false>
+    // instead of broadcasting each scalar into a register pair. Body records otherwise are
+    // first gathered to {x, y, z, m}: one load a source in the loop instead of two.
+    // U sources a loop iteration: their chains overlap. Bound by the FP32 pipe (12 packed
+    // instructions a source and pair of targets; 91 % of it at 200,000 bodies). Before, with
+    // two sources an iteration and chunks planned by whole waves, and now: 20,011 bodies softened
+    // 176 -> 166 us, records under the cutoff law 221 -> 192; 32,768: 438 -> 419, 532 -> 450;
+    // 100,003: 3.61 -> 3.52 ms, 4.38 -> 3.95.
+    template <int T, int BLOCK, int TILE, int STAGES, int LAW, bool AOS, bool PACKED, bool DUP, int U>
     __global__ void __launch_bounds__(BLOCK, (T >= 8 ? 2 : 3))
     direct_fp32_kernel(const float4* __restrict__ src,        // pos_mass (SoA) or Body (AoS)
                        const float4* __restrict__ vel_radius, // SoA radius source (CUTOFF)
@@ -112,8 +119,9 @@ namespace nbg
     {
         constexpr int P = T / 2;
         constexpr int REC = Layout<AOS>::kRec;
+        constexpr bool GATHER = AOS && !DUP;
         __shared__ __align__(128) float4 tile[STAGES][TILE * REC];
-        __shared__ __align__(16) float4 pairs[DUP ? 2 * TILE : 1];
+        __shared__ __align__(16) float4 pairs[DUP ? 2 * TILE : (GATHER ? TILE : 1)];
         __shared__ __align__(8) uint64_t bar[STAGES];
         // Each thread's fold of its tile sums (dynamic shared memory, fold_bytes(T, BLOCK)):
         // row 6p + c holds S of component c (x, y, z) of pair p, row 6p + 3 + c its
@@ -209,7 +217,7 @@ namespace nbg
                     pairs[2 * j + 1] = make_float4(s.z, s.z, m, m);
                 }
                 __syncthreads();
-#pragma unroll 2
+#pragma unroll U
                 for (int j = 0; j < TILE; ++j)
                 {
                     const float4 a = pairs[2 * j], b = pairs[2 * j + 1];
@@ -222,12 +230,18 @@ namespace nbg
             }
             else
             {
-#pragma unroll 2
+                if (GATHER)
+                {
+                    for (int j = tid; j < TILE; j += BLOCK)
+                        pairs[j] = make_float4(tl[j * REC].x, tl[j * REC].y, tl[j * REC].z, tl[j * REC + 1].w);
+                    __syncthreads();
+                    tl = pairs;
+                }
+#pragma unroll U
                 for (int j = 0; j < TILE; ++j)
                 {
-                    const float4 s = tl[j * REC];
-                    const float m = AOS ? tl[j * REC + 1].w : s.w;
-                    const float2 sx = f2(s.x), sy = f2(s.y), sz = f2(s.z), sm = f2(m);
+                    const float4 s = tl[j];
+                    const float2 sx = f2(s.x), sy = f2(s.y), sz = f2(s.z), sm = f2(s.w);
 #pragma unroll
                     for (int p = 0; p < P; ++p)
                         interact2<LAW, PACKED>(sx, sy, sz, sm, nx[p], ny[p], nz[p], lim[p], ax[p], ay[p], az[p]);
@@ -360,9 +374,16 @@ namespace nbg
             cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         }
 
-        constexpr int kPlanned = 3;
+        // The shapes plan_direct chooses from (indices into variants()). Six targets a lane in
+        // CTAs of two warps is the fastest or within 2 % of it from 9,000 bodies up, and its CTAs
+        // are small enough to pack evenly. Body records under the cutoff law are 3 to 6 % faster
+        // with four a lane (100,003: 3.95 against 4.10 ms); the softened sum of 2^20 bodies is 0.5
+        // (records: 1.4) % faster with pre-paired tiles, 400,009 the same, 100,003 1.5 % slower.
+        constexpr int kPlan = 10, kWideAosPlan = 11, kPairedPlan = 0, kNarrowPlan = 2;
+        constexpr size_t kPairedMinN = 1 << 18;
+        constexpr size_t kMaxSplit = 64;                        // source chunks
 
-        template <int T, int B, bool PACKED = true, bool DUP = false>
+        template <int T, int B, bool PACKED = true, bool DUP = false, int U = 2>
         Variant make_variant()
         {
             Variant v;
@@ -370,22 +391,22 @@ namespace nbg
             v.block = B;
             v.packed = PACKED;
             v.dup = DUP;
-            v.fn[0][0] = direct_fp32_kernel<T, B, kTile, kStages, NBODY_LAW_CUTOFF, false, PACKED, DUP>;
-            v.fn[0][1] = direct_fp32_kernel<T, B, kTile, kStages, NBODY_LAW_CUTOFF, true, PACKED, DUP>;
-            v.fn[1][0] = direct_fp32_kernel<T, B, kTile, kStages, NBODY_LAW_SOFTENED, false, PACKED, DUP>;
-            v.fn[1][1] = direct_fp32_kernel<T, B, kTile, kStages, NBODY_LAW_SOFTENED, true, PACKED, DUP>;
+            v.fn[0][0] = direct_fp32_kernel<T, B, kTile, kStages, NBODY_LAW_CUTOFF, false, PACKED, DUP, U>;
+            v.fn[0][1] = direct_fp32_kernel<T, B, kTile, kStages, NBODY_LAW_CUTOFF, true, PACKED, DUP, U>;
+            v.fn[1][0] = direct_fp32_kernel<T, B, kTile, kStages, NBODY_LAW_SOFTENED, false, PACKED, DUP, U>;
+            v.fn[1][1] = direct_fp32_kernel<T, B, kTile, kStages, NBODY_LAW_SOFTENED, true, PACKED, DUP, U>;
             v.fold_bytes = fold_bytes_of(T, B);
             return v;
         }
 
         const Variant* variants(int* count)
         {
-            // The first kPlanned entries are what plan_direct chooses between by size; the
-            // rest are further shapes the direct-sum autotuner can time and pin.
+            // plan_direct chooses among four of them; the rest are further shapes the direct-sum
+            // autotuner can time and pin.
             static const Variant v[] = {
-                make_variant<4, 256, true, true>(),     // the fastest at N >= 65536 (timed)
+                make_variant<4, 256, true, true>(),     // kPairedPlan
                 make_variant<4, 128>(),
-                make_variant<2, 64>(),                  // the fastest at N = 16384
+                make_variant<2, 64, true, false, 8>(),      // kNarrowPlan
                 make_variant<8, 256>(),
                 make_variant<4, 256>(),
                 make_variant<8, 256, false>(),
@@ -393,6 +414,8 @@ namespace nbg
                 make_variant<6, 128>(),
                 make_variant<12, 128>(),
                 make_variant<8, 256, true, true>(),
+                make_variant<6, 64, true, false, 4>(),     // kPlan
+                make_variant<4, 128, true, false, 8>(),    // kWideAosPlan
             };
             *count = static_cast<int>(sizeof(v) / sizeof(v[0]));
             return v;
@@ -408,21 +431,10 @@ namespace nbg
             }();
             return sms;
         }
-
-        int occupancy(KernelFn fn, const int block, const int dyn_bytes)
-        {
-            int blocks = 0;
-            allow_dynamic_smem(fn, dyn_bytes);
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, block, dyn_bytes) != cudaSuccess)
-            {
-                cudaGetLastError();
-                return 1;
-            }
-            return blocks > 0 ? blocks : 1;
-        }
     }
 
-    DirectPlan plan_direct(const size_t n, const int law, const bool aos, const int force_variant)
+    DirectPlan plan_direct(const size_t n, const int law, const bool aos, const int force_variant,
+                           const size_t split_bytes)
     {
         DirectPlan plan{};
         if (force_variant < 0 && n <= kSmallDirect)
@@ -442,61 +454,50 @@ namespace nbg
         }
         int nv = 0;
         const Variant* vs = variants(&nv);
-        const int li = law == NBODY_LAW_SOFTENED ? 1 : 0;
-        const int ai = aos ? 1 : 0;
-        const int sms = sm_count();
-
-        int chosen = -1;
-        if (force_variant >= 0 && force_variant < nv)
-            chosen = force_variant;
-        else
+        // Chunks hold whole fold units, so the last chunk is the only ragged one.
+        const size_t unit = n >= kFoldMinN ? kTile * kFoldTiles : kTile;
+        const size_t units = std::max<size_t>(1, (n + unit - 1) / unit);
+        const size_t max_js = std::max<size_t>(1, std::min({ kMaxSplit, units, split_bytes / (32 * std::max<size_t>(1, n)) }));
+        const double sms = sm_count();
+        auto units_per_chunk = [&](const size_t js) { return (units + js - 1) / js; };
+        auto target_blocks = [&](const int k) {
+            const size_t per = static_cast<size_t>(vs[k].T) * vs[k].block;
+            return std::max<size_t>(1, (n + per - 1) / per);
+        };
+        // The split of the sources: the pairs the fullest SM computes one after another. CTAs end
+        // together and are not dealt evenly, which leaves an SM the last of ceil(CTAs / SMs) and on
+        // average one and a half more; a CTA's start costs about as much as 8,000 pairs, and the
+        // partials n / 16 pairs a chunk. Fitted to 1,500 timings (8,193 to 200,000 bodies, both laws
+        // and layouts, every split): its choice takes 0.7 % longer than the best split, 3 % at worst.
+        // The fewest chunks within 2 % of the least are taken, for the sake of the scratch.
+        auto cost = [&](const int k, const size_t js) {
+            const size_t c = units_per_chunk(js), per = static_cast<size_t>(vs[k].T) * vs[k].block;
+            const double ctas = static_cast<double>(target_blocks(k) * ((units + c - 1) / c)) / sms;
+            return (std::ceil(ctas) + 1.5) * static_cast<double>(c * unit * per) + 8000.0 * ctas
+                   + 0.06 * static_cast<double>(n * js);
+        };
+        auto least = [&](const int k) {
+            double v = cost(k, 1);
+            for (size_t js = 2; js <= max_js; ++js)
+                v = std::min(v, cost(k, js));
+            return v;
+        };
+        int chosen = force_variant;
+        if (chosen < 0 || chosen >= nv)
         {
-            // Largest register block whose (target blocks x max chunks) fills the GPU.
-            for (int k = 0; k < kPlanned; ++k)
-            {
-                const size_t per = static_cast<size_t>(vs[k].T) * vs[k].block;
-                const size_t tb = (n + per - 1) / per;
-                const size_t max_js = std::max<size_t>(1, n / (kTile * 4));
-                const size_t slots =
-                    static_cast<size_t>(occupancy(vs[k].fn[li][ai], vs[k].block, vs[k].fold_bytes)) * sms;
-                if (tb * max_js >= slots)
-                {
-                    chosen = k;
-                    break;
-                }
-            }
-            if (chosen < 0)
-                chosen = kPlanned - 1;
+            chosen = law == NBODY_LAW_CUTOFF && aos ? kWideAosPlan
+                                                    : (law == NBODY_LAW_SOFTENED && n >= kPairedMinN ? kPairedPlan : kPlan);
+            // a small scratch allows few chunks: then CTAs of 128 targets pack better, at 5 %
+            // longer a pair
+            if (split_bytes < kSplitBytes && 1.05 * least(kNarrowPlan) < least(chosen))
+                chosen = kNarrowPlan;
         }
         const Variant& v = vs[chosen];
-        const size_t per = static_cast<size_t>(v.T) * v.block;
-        const size_t tb = std::max<size_t>(1, (n + per - 1) / per);
-        const size_t slots = static_cast<size_t>(occupancy(v.fn[li][ai], v.block, v.fold_bytes)) * sms;
-        // Split the sources so tb*js CTAs pack into whole waves: minimise the padded
-        // work ceil(tb*js/slots)*slots/(tb*js) per unit, preferring fewer chunks. Chunks may
-        // be a single tile: at small n the target blocks alone would leave most SMs idle
-        // (N = 4096 has 32 target blocks of 128).
-        const size_t max_js = std::max<size_t>(1, std::min<size_t>(64, n / kTile));
-        size_t best_js = 1;
-        double best_cost = 1e300;
-        for (size_t js = 1; js <= max_js; ++js)
-        {
-            const size_t ctas = tb * js;
-            const size_t waves = (ctas + slots - 1) / slots;
-            // time ~ waves * (work per CTA) = waves / js (work per CTA shrinks with js)
-            const double cost = static_cast<double>(waves) / static_cast<double>(js)
-                                * (1.0 + 0.002 * static_cast<double>(js));
-            if (cost < best_cost - 1e-12)
-            {
-                best_cost = cost;
-                best_js = js;
-            }
-        }
-        // Chunks hold whole fold units, so the last chunk is the only ragged one.
-        const int fold = n >= kFoldMinN ? kFoldTiles : 1;
-        const size_t unit = static_cast<size_t>(kTile) * fold;
-        size_t chunk = (n + best_js - 1) / best_js;
-        chunk = (chunk + unit - 1) / unit * unit;
+        const double bar = 1.02 * least(chosen);
+        size_t split = 1;
+        while (cost(chosen, split) > bar)
+            ++split;
+        const size_t chunk = units_per_chunk(split) * unit;
         const size_t js = std::max<size_t>(1, (n + chunk - 1) / chunk);
 
         plan.variant = chosen;
@@ -504,10 +505,10 @@ namespace nbg
         plan.T = v.T;
         plan.block = v.block;
         plan.tile = kTile;
-        plan.fold = fold;
+        plan.fold = static_cast<int>(unit / kTile);
         plan.jsplit = static_cast<int>(js);
         plan.chunk = static_cast<int>(chunk);
-        plan.grid_x = static_cast<int>(tb);
+        plan.grid_x = static_cast<int>(target_blocks(chosen));
         plan.law = law;
         plan.aos = aos;
         return plan;

@@ -129,8 +129,10 @@ namespace nbg
     // so the sums do not depend on which kernel combines them.
     inline int combine_width(const int n, const int js) { return (js >= 8 && n <= (1 << 16)) ? 8 : 1; }
 
-    // Pick a launch shape for n bodies. force_variant >= 0 pins the (T, block) entry.
-    DirectPlan plan_direct(size_t n, int law, bool aos, int force_variant = -1);
+    // Pick a launch shape for n bodies. force_variant >= 0 pins the (T, block) entry; the
+    // chunk partials stay within split_bytes.
+    constexpr size_t kSplitBytes = size_t(256) << 20;
+    DirectPlan plan_direct(size_t n, int law, bool aos, int force_variant = -1, size_t split_bytes = kSplitBytes);
 
     // The instantiated kernel shapes: targets per thread, threads per CTA, packed FP32x2 or not.
     int direct_variant_count();

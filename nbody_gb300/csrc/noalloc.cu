@@ -16,7 +16,6 @@
 // The module is loaded anew in every context (a second context on the same device, or
 // the primary context re-created after cudaDeviceReset), so an address is never reused
 // outside the context it came from.
-#include <algorithm>
 #include <mutex>
 
 #include <cuda.h>       // CUcontext and CUresult only: the two driver calls are resolved at run time
@@ -152,16 +151,7 @@ extern "C" int nbody_cuda_dev_accel_soa_noalloc(const void* pos_mass, const void
 
     // The usual launch shape, with the source split capped so its partials fit: a chunk
     // leaves two float4 per body (its sum and the sum's compensation).
-    DirectPlan plan = plan_direct(n, p->law, false);
-    if (direct_scratch_bytes(plan, n) > kNoAllocPartials * sizeof(float4))
-    {
-        const size_t js = std::max<size_t>(1, kNoAllocPartials / (2 * n));
-        size_t chunk = (n + js - 1) / js;
-        const size_t unit = static_cast<size_t>(plan.tile) * plan.fold;
-        chunk = (chunk + unit - 1) / unit * unit;
-        plan.chunk = static_cast<int>(chunk);
-        plan.jsplit = static_cast<int>((n + chunk - 1) / chunk);
-    }
+    const DirectPlan plan = plan_direct(n, p->law, false, -1, kNoAllocPartials * sizeof(float4));
 
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     // The error word keeps the previous call's value: clear it first.

@@ -389,3 +389,27 @@ def test_small_systems(gpu, n, layout, law):
     assert np.array_equal(out[:, :8], b[:, :8])
     err = scaled_err(out[:, 8:11] / np.float32(1.5), b, law, eps2=eps2)
     assert err.max() <= TOL_MAX and np.median(err) <= TOL_MEDIAN
+
+
+@pytest.mark.parametrize("law", [0, 1], ids=["cutoff", "softened"])
+@pytest.mark.parametrize("layout", [0, 1], ids=["soa", "aos"])
+@pytest.mark.parametrize("n", [8193, 8449, 16385, 65535, 65536, 65537, (1 << 18) - 1, 1 << 18])
+def test_planned_shapes(gpu, n, layout, law):
+    """The planned launch at the edges of its sizes (a chunk of one ragged tile, the longer
+    sums from 65,536 bodies, the other shape from 2^18): sampled targets, the first and last
+    of the bodies among them, against FP64 with the file's bar, and repeats are identical."""
+    from nbody_gb300 import scenes
+    b = scenes.uniform_cube(n, seed=n)
+    b[:, 3] = np.float32(1e-3)
+    b[n // 2, 7] = 0.0
+    eps2 = 1e-6 if law == gpu.LAW_SOFTENED else 0.0
+    p = gpu.params(law=law, eps2=eps2)
+    with gpu.Context(layout) as ctx:
+        ctx.upload_bodies(b)
+        ctx.accelerate(p)
+        out = ctx.download_bodies()[:, 8:11].copy()
+        ctx.accelerate(p)
+        assert np.array_equal(out, ctx.download_bodies()[:, 8:11])
+    tg = np.unique(np.r_[0, n - 1, np.random.default_rng(n).integers(0, n, 60)])
+    err = scaled_err(out[tg], b, law, eps2=eps2, targets=tg)
+    assert err.max() <= TOL_MAX and np.median(err) <= TOL_MEDIAN
