@@ -78,7 +78,7 @@ namespace nbg
     // One work item, start to finish. Kept out of line: compiled on its own, the source loop
     // gets the same code as in a one-item-per-CTA launch; inlined into the persistent loop
     // it came out with a fifth of its instructions in extra integer work.
-    template <int BLOCK, int T, int LAW, bool DUP>
+    template <int BLOCK, int T, int LAW, bool DUP, int U>
     __device__ __noinline__ bool run_item(BatchShared& sh, const Item& w, unsigned& seq, const float4* __restrict__ pm,
                                           const float4* __restrict__ vr, const int csize, float4* __restrict__ acc,
                                           float4* __restrict__ partial, unsigned* __restrict__ block_done,
@@ -155,7 +155,7 @@ namespace nbg
                     sh.dup[2 * j + 1] = make_float4(v.z, v.z, v.w, v.w);
                 }
                 __syncthreads();
-#pragma unroll 2
+#pragma unroll U
                 for (int j = 0; j < padded; ++j)
                 {
                     const float4 a = sh.dup[2 * j], b = sh.dup[2 * j + 1];
@@ -175,7 +175,7 @@ namespace nbg
                     __syncthreads();
                 }
                 const float4* tl = sh.tile[stage];
-#pragma unroll 2
+#pragma unroll U
                 for (int j = 0; j < padded; ++j)
                 {
                     const float4 v = tl[j];
@@ -247,7 +247,7 @@ namespace nbg
     }
 
     // Persistent CTAs pull items from the counter until the list is exhausted.
-    template <int BLOCK, int T, int LAW, bool DUP>
+    template <int BLOCK, int T, int LAW, bool DUP, int U>
     __global__ void __launch_bounds__(BLOCK)
     batch_kernel(const float4* __restrict__ pm, const float4* __restrict__ vr, const Item* __restrict__ items,
                  const int nitems, const int csize, unsigned* __restrict__ counter, float4* __restrict__ acc,
@@ -274,7 +274,7 @@ namespace nbg
             if (it >= nitems)
                 return;
             const Item w = items[it];
-            if (!run_item<BLOCK, T, LAW, DUP>(sh, w, seq, pm, vr, csize, acc, partial, block_done, G, eps2, err))
+            if (!run_item<BLOCK, T, LAW, DUP, U>(sh, w, seq, pm, vr, csize, acc, partial, block_done, G, eps2, err))
                 return;
         }
     }
@@ -343,11 +343,11 @@ namespace nbg
             BatchFn soft, cutoff;
         };
 
-        template <int BLOCK, int T, bool DUP = false>
+        template <int BLOCK, int T, bool DUP = false, int U = 2>
         Config cfg(const int chunk)
         {
-            return { BLOCK, T, chunk, batch_kernel<BLOCK, T, NBODY_LAW_SOFTENED, DUP>,
-                     batch_kernel<BLOCK, T, NBODY_LAW_CUTOFF, DUP> };
+            return { BLOCK, T, chunk, batch_kernel<BLOCK, T, NBODY_LAW_SOFTENED, DUP, U>,
+                     batch_kernel<BLOCK, T, NBODY_LAW_CUTOFF, DUP, U> };
         }
 
         // Shapes the autotuner times: threads per CTA, targets per thread, sources per chunk.
@@ -356,9 +356,23 @@ namespace nbg
             static const std::vector<Config> c = {
                 cfg<64, 4>(1024), cfg<64, 4>(512),  cfg<64, 4>(2048), cfg<128, 4>(1024), cfg<64, 2>(1024),
                 cfg<128, 2>(1024), cfg<64, 8>(1024), cfg<64, 2, true>(1024), cfg<64, 4, true>(1024),
-                cfg<128, 4, true>(1024),
+                cfg<128, 4, true>(1024), cfg<64, 2, false, 8>(512), cfg<64, 4, true>(512),
             };
             return c;
+        }
+
+        // The configuration of a new system table, until one is pinned or tuned. Bound by the FP32
+        // pipe once there are items enough for every SM. Small items fill the chip and leave
+        // few targets unused: 64 systems of 64 to 1,024 bodies take 19 us against 44 with
+        // cfg<64, 4>(1024), 32 of 64 to 8,192 135 against 165, 300 of 64 to 4,096 (6e8 pairs) 240
+        // against 254. From about 1e9 pairs four targets a lane and pre-paired sources win: 512
+        // systems of 64 to 8,192 (3.5e9 pairs) 1,516 us against 1,572 with small items.
+        int default_config(const std::vector<int>& off)
+        {
+            double pairs = 0;
+            for (size_t s = 0; s + 1 < off.size(); ++s)
+                pairs += static_cast<double>(off[s + 1] - off[s]) * (off[s + 1] - off[s]);
+            return pairs < 1e9 ? 10 : 11;
         }
 
         int targets_per_item(const Config& c) { return c.block * c.t; }
@@ -380,7 +394,7 @@ namespace nbg
         float4* partial = nullptr;      // chunk partial sums, TB per item of a multi-chunk block
         size_t partial_cap = 0;
         int config = 0;                 // index into configs()
-        bool tuned = false;
+        bool pinned = false;            // by the user or the autotuner
     };
 
     int batch_config_count() { return static_cast<int>(configs().size()); }
@@ -505,6 +519,8 @@ namespace nbg
         b.off.assign(nsys + 1, 0);
         for (size_t s = 0; s <= nsys; ++s)
             b.off[s] = static_cast<int>(offsets[s]);
+        if (!b.pinned)
+            b.config = default_config(b.off);
         if (b.off.size() > b.off_cap)
         {
             cudaFreeAsync(b.d_off, ctx->stream);
@@ -597,8 +613,8 @@ namespace nbg
             }
         }
         b.config = best_i;
+        b.pinned = true;
         b.items_config = -1;
-        b.tuned = true;
         if (best)
             *best = best_i;
         return check_device_error(ctx);
@@ -611,6 +627,7 @@ namespace nbg
         if (index < 0 || index >= batch_config_count())
             return ctx_fail(ctx, NBODY_ERR_INVALID, "no such batched configuration");
         ctx->batch->config = index;
+        ctx->batch->pinned = true;
         ctx->batch->items_config = -1;
         return NBODY_OK;
     }

@@ -189,3 +189,25 @@ def test_config4_batch(gpu):
     E1 = e1[:, 0] + e1[:, 1]
     drift = np.abs((E1 - E0) / E0)
     assert np.all(np.isfinite(drift)) and np.median(drift) < 1e-3, np.median(drift)
+
+
+@pytest.mark.parametrize("sizes,index", [([31618, 500, 1], 10), ([32768, 129, 513, 1], 11)], ids=["small", "large"])
+def test_default_configuration(gpu, sizes, index):
+    """The configuration a system table gets on either side of 1e9 pairs: sampled targets against
+    FP64 with this file's bar, and a pinned configuration outlives a new table."""
+    b, off = make_batch(sizes)
+    p = gpu.params(mode=gpu.MODE_BATCHED, law=gpu.LAW_SOFTENED, eps2=EPS2)
+    with gpu.Context() as ctx:
+        ctx.upload_bodies(b)
+        ctx.set_systems(off)
+        assert ctx.batch_config(-1) == ctx.batch_config(index)
+        ctx.accelerate(p)
+        acc = ctx.download_bodies()[:, 8:11]
+        ctx.batch_set_config(3)
+        ctx.set_systems(off)
+        assert ctx.batch_config(-1) == ctx.batch_config(3)
+    for s in range(len(sizes)):
+        sb = b[off[s]:off[s + 1]]
+        tg = np.unique(np.r_[0, len(sb) - 1, np.random.default_rng(s).integers(0, len(sb), 60)])
+        ref, scale = O.direct_f64(sb[:, [0, 1, 2, 7]], 1.0, float(np.float32(EPS2)), O.LAW_SOFTENED, targets=tg, with_scale=True)
+        assert (np.linalg.norm(acc[off[s]:off[s + 1]][tg] - ref, axis=1) / np.maximum(scale, 1e-30)).max() <= 5e-5
