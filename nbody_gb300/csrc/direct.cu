@@ -29,7 +29,6 @@
 //     launch shape (up to a rounding tie of the last fold), and it is more accurate than
 //     one FP32 running sum over all N sources.
 #include <algorithm>
-#include <cmath>
 #include <cstdio>
 
 #include "common.cuh"
@@ -458,29 +457,10 @@ namespace nbg
         const size_t unit = n >= kFoldMinN ? kTile * kFoldTiles : kTile;
         const size_t units = std::max<size_t>(1, (n + unit - 1) / unit);
         const size_t max_js = std::max<size_t>(1, std::min({ kMaxSplit, units, split_bytes / (32 * std::max<size_t>(1, n)) }));
-        const double sms = sm_count();
-        auto units_per_chunk = [&](const size_t js) { return (units + js - 1) / js; };
-        auto target_blocks = [&](const int k) {
+        auto split_of = [&](const int k) {
             const size_t per = static_cast<size_t>(vs[k].T) * vs[k].block;
-            return std::max<size_t>(1, (n + per - 1) / per);
-        };
-        // The split of the sources: the pairs the fullest SM computes one after another. CTAs end
-        // together and are not dealt evenly, which leaves an SM the last of ceil(CTAs / SMs) and on
-        // average one and a half more; a CTA's start costs about as much as 8,000 pairs, and the
-        // partials n / 16 pairs a chunk. Fitted to 1,500 timings (8,193 to 200,000 bodies, both laws
-        // and layouts, every split): its choice takes 0.7 % longer than the best split, 3 % at worst.
-        // The fewest chunks within 2 % of the least are taken, for the sake of the scratch.
-        auto cost = [&](const int k, const size_t js) {
-            const size_t c = units_per_chunk(js), per = static_cast<size_t>(vs[k].T) * vs[k].block;
-            const double ctas = static_cast<double>(target_blocks(k) * ((units + c - 1) / c)) / sms;
-            return (std::ceil(ctas) + 1.5) * static_cast<double>(c * unit * per) + 8000.0 * ctas
-                   + 0.06 * static_cast<double>(n * js);
-        };
-        auto least = [&](const int k) {
-            double v = cost(k, 1);
-            for (size_t js = 2; js <= max_js; ++js)
-                v = std::min(v, cost(k, js));
-            return v;
+            return SourceSplit{ std::max<size_t>(1, (n + per - 1) / per), per, units, unit, n,
+                                static_cast<double>(sm_count()) };
         };
         int chosen = force_variant;
         if (chosen < 0 || chosen >= nv)
@@ -489,15 +469,12 @@ namespace nbg
                                                     : (law == NBODY_LAW_SOFTENED && n >= kPairedMinN ? kPairedPlan : kPlan);
             // a small scratch allows few chunks: then CTAs of 128 targets pack better, at 5 %
             // longer a pair
-            if (split_bytes < kSplitBytes && 1.05 * least(kNarrowPlan) < least(chosen))
+            if (split_bytes < kSplitBytes && 1.05 * split_of(kNarrowPlan).least(max_js) < split_of(chosen).least(max_js))
                 chosen = kNarrowPlan;
         }
         const Variant& v = vs[chosen];
-        const double bar = 1.02 * least(chosen);
-        size_t split = 1;
-        while (cost(chosen, split) > bar)
-            ++split;
-        const size_t chunk = units_per_chunk(split) * unit;
+        const SourceSplit sp = split_of(chosen);
+        const size_t chunk = sp.chunk(max_js, 1.02);
         const size_t js = std::max<size_t>(1, (n + chunk - 1) / chunk);
 
         plan.variant = chosen;
@@ -508,7 +485,7 @@ namespace nbg
         plan.fold = static_cast<int>(unit / kTile);
         plan.jsplit = static_cast<int>(js);
         plan.chunk = static_cast<int>(chunk);
-        plan.grid_x = static_cast<int>(target_blocks(chosen));
+        plan.grid_x = static_cast<int>(sp.tb);
         plan.law = law;
         plan.aos = aos;
         return plan;

@@ -212,16 +212,18 @@ namespace nbg
 
     // Targets: all n (tlist == nullptr) or tlist[0 .. nt). Output: FP64 partials
     // part[blockIdx.y * nt + t] = G * (sum - compensation).
+    // Bound by the FP32 pipe (12 packed instructions a source and pair of targets, and the Kahan
+    // steps of every 64 sources). Eight sources an iteration overlap their chains, and CTAs of two
+    // warps pack evenly: 1,000 bodies took 73 us with 1,024 targets a CTA and whole-wave splits,
+    // now 14; 8,192 79, now 47; 20,011 195, now 178; 50,021 970, now 939; 100,003 3.78 ms, now 3.61.
     template <int T, int BLOCK, int LAW>
-    __global__ void __launch_bounds__(BLOCK, 2)
+    __global__ void __launch_bounds__(BLOCK, 2 * 256 / BLOCK * 4 / T)
     direct_comp_kernel(const float4* __restrict__ src, const float* __restrict__ radius2, const int* __restrict__ tlist,
                        const int nt, const int n, const int chunk, const float G, const float eps2,
                        double4* __restrict__ part, unsigned* __restrict__ err)
     {
         constexpr int P = T / 2;
         __shared__ __align__(128) float4 tile[kStages][kTileC];
-        // each landed tile rewritten as operand pairs {x,x,y,y}, {z,z,m,m} (see direct.cu)
-        __shared__ __align__(16) float4 pairs[2 * kTileC];
         __shared__ __align__(8) uint64_t bar[kStages];
         const int tid = threadIdx.x;
         const int base = blockIdx.x * (BLOCK * T);
@@ -289,21 +291,13 @@ namespace nbg
                 __syncthreads();
             }
             const float4* tl = tile[stage];
-            for (int j = tid; j < kTileC; j += BLOCK)
-            {
-                const float4 s = tl[j];
-                pairs[2 * j] = make_float4(s.x, s.x, s.y, s.y);
-                pairs[2 * j + 1] = make_float4(s.z, s.z, s.w, s.w);
-            }
-            __syncthreads();
             for (int sb = 0; sb < kTileC; sb += kSub)
             {
-#pragma unroll 2
+#pragma unroll 8
                 for (int j = sb; j < sb + kSub; ++j)
                 {
-                    const float4 a = pairs[2 * j], b = pairs[2 * j + 1];
-                    const float2 sx = make_float2(a.x, a.y), sy = make_float2(a.z, a.w);
-                    const float2 sz = make_float2(b.x, b.y), sm = make_float2(b.z, b.w);
+                    const float4 v = tl[j];
+                    const float2 sx = f2(v.x), sy = f2(v.y), sz = f2(v.z), sm = f2(v.w);
 #pragma unroll
                     for (int p = 0; p < P; ++p)
                         interact2c<LAW>(sx, sy, sz, sm, nx[p], ny[p], nz[p], lim[p], ax[p], ay[p], az[p]);
@@ -665,27 +659,16 @@ namespace nbg
             int tb, js, chunk;
         };
 
-        Split plan_split(const size_t nt, const size_t n, const int per_cta, const int tile, const int slots)
+        Split plan_split(const size_t nt, const size_t n, const int per_cta, const int tile, const int sms)
         {
+            const SourceSplit sp{ std::max<size_t>(1, (nt + per_cta - 1) / per_cta), static_cast<size_t>(per_cta),
+                                  std::max<size_t>(1, (n + tile - 1) / tile), static_cast<size_t>(tile), nt,
+                                  static_cast<double>(sms) };
+            const size_t max_js = std::max<size_t>(1, std::min({ size_t(64), sp.units, kSplitBytes / (32 * std::max<size_t>(1, nt)) }));
             Split p;
-            p.tb = static_cast<int>(std::max<size_t>(1, (nt + per_cta - 1) / per_cta));
-            const size_t max_js = std::max<size_t>(1, std::min<size_t>(64, n / (static_cast<size_t>(tile) * 4)));
-            size_t best = 1;
-            double best_cost = 1e300;
-            for (size_t js = 1; js <= max_js; ++js)
-            {
-                const size_t waves = (p.tb * js + slots - 1) / slots;
-                const double cost = static_cast<double>(waves) / static_cast<double>(js) * (1.0 + 0.002 * js);
-                if (cost < best_cost - 1e-12)
-                {
-                    best_cost = cost;
-                    best = js;
-                }
-            }
-            size_t chunk = (n + best - 1) / best;
-            chunk = (chunk + tile - 1) / tile * tile;
-            p.chunk = static_cast<int>(chunk);
-            p.js = static_cast<int>((n + chunk - 1) / chunk);
+            p.tb = static_cast<int>(sp.tb);
+            p.chunk = static_cast<int>(sp.chunk(max_js, 1.0));
+            p.js = static_cast<int>((n + p.chunk - 1) / p.chunk);
             return p;
         }
 
@@ -724,9 +707,12 @@ namespace nbg
             const int ni = static_cast<int>(n), nti = static_cast<int>(nt);
             const bool fp64 = p->precision == NBODY_PREC_FP64;
             const int sms = sms_of(ctx);
-            constexpr int kT = 4, kB = 256, kB64 = 128;
+            constexpr int kB = 64, kB64 = 128;
+            // compensated: four targets a lane from 5e8 pairs (20,011 bodies 178 us with two and 184
+            // with four, 32,768: 434 and 422, 50,021: 970 and 939), two below
+            const int targets = static_cast<double>(nt) * n < 5e8 ? 2 : 4;
             const Split sp = fp64 ? plan_split64(nt, n, kB64 * 2, kTile64, sms)
-                                  : plan_split(nt, n, kB * kT, kTileC, sms * 2);
+                                  : plan_split(nt, n, kB * targets, kTileC, sms);
             // scratch: partials (js * nt double4) + radius^2 (n floats)
             const size_t part_bytes = static_cast<size_t>(sp.js) * nt * sizeof(double4);
             const size_t rad_bytes = (p->law == NBODY_LAW_CUTOFF) ? n * sizeof(float) : 0;
@@ -755,12 +741,12 @@ namespace nbg
             }
             else
             {
-                if (p->law == NBODY_LAW_SOFTENED)
-                    direct_comp_kernel<kT, kB, NBODY_LAW_SOFTENED><<<grid, kB, 0, st>>>(
-                        s.off, rad2, tlist, nti, ni, sp.chunk, p->G, p->eps2, part, ctx->dev_error);
-                else
-                    direct_comp_kernel<kT, kB, NBODY_LAW_CUTOFF><<<grid, kB, 0, st>>>(
-                        s.off, rad2, tlist, nti, ni, sp.chunk, p->G, p->eps2, part, ctx->dev_error);
+                const bool soft = p->law == NBODY_LAW_SOFTENED;
+                const auto fn = targets == 2 ? (soft ? direct_comp_kernel<2, kB, NBODY_LAW_SOFTENED>
+                                                : direct_comp_kernel<2, kB, NBODY_LAW_CUTOFF>)
+                                        : (soft ? direct_comp_kernel<4, kB, NBODY_LAW_SOFTENED>
+                                                : direct_comp_kernel<4, kB, NBODY_LAW_CUTOFF>);
+                fn<<<grid, kB, 0, st>>>(s.off, rad2, tlist, nti, ni, sp.chunk, p->G, p->eps2, part, ctx->dev_error);
                 ++ctx->launches;
             }
             float4* acc = (write_acc && ctx->layout == NBODY_LAYOUT_SOA) ? ctx->acc : nullptr;
@@ -769,7 +755,7 @@ namespace nbg
             ++ctx->launches;
             DirectPlan& lp = ctx->last_plan;
             lp = DirectPlan{};
-            lp.T = fp64 ? 2 : kT;
+            lp.T = fp64 ? 2 : targets;
             lp.block = fp64 ? kB64 : kB;
             lp.tile = fp64 ? kTile64 : kTileC;
             lp.jsplit = sp.js;

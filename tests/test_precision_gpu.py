@@ -217,3 +217,28 @@ def test_fp64_sizes_and_ranges(gpu, law, n, scale_pos):
     assert np.all(np.isfinite(got))
     assert np.all(np.linalg.norm(got - ref, axis=1) <= 1e-12 * scale)
     assert np.all(np.linalg.norm(few - ref[::50], axis=1) <= 1e-12 * scale[::50])
+
+
+@pytest.mark.parametrize("law", [0, 1], ids=["cutoff", "softened"])
+@pytest.mark.parametrize("n", [1, 2, 63, 129, 257, 1000, 8191, 22360, 22361])
+def test_compensated_sums_of_other_splits_agree(gpu, n, law):
+    """The compensated sum at the edges of its target blocks and source tiles, and on either side
+    of 5e8 pairs: a sample of the targets (other blocks, another split, another shape) against
+    the accelerations of all of them. A Kahan step rounds the 64-source sum it adds once, which
+    is 2^-24 of the terms' magnitudes in all for either, and the stored accelerations are
+    rounded to FP32 once more. Repeats are identical."""
+    from nbody_gb300 import scenes
+    b = scenes.uniform_cube(n, seed=n)
+    b[:, 3] = np.float32(0.01)
+    p = gpu.params(law=law, eps2=1e-6 if law == gpu.LAW_SOFTENED else 0.0, precision=gpu.PREC_COMPENSATED)
+    tg = np.unique(np.r_[0, n - 1, np.random.default_rng(n).integers(0, n, 200)])
+    with gpu.Context() as ctx:
+        ctx.upload_bodies(b)
+        ctx.accelerate(p)
+        acc = ctx.download_bodies()[:, 8:11].copy()
+        sampled = ctx.accel_sampled(p, tg)
+        ctx.accelerate(p)
+        assert np.array_equal(acc, ctx.download_bodies()[:, 8:11])
+    assert np.all(np.isfinite(acc)) and (n == 1 or np.all(np.any(acc != 0, axis=1)))
+    _, scale = f64_ref(b, p.eps2, law, targets=tg)
+    assert np.all(np.linalg.norm(sampled - acc[tg], axis=1) <= 3 * 2.0**-24 * np.sqrt(3) * scale)
