@@ -24,7 +24,7 @@ namespace nbg
         long long lo_cells[3];      // lo / cell
         // Fixed-point cell sums: a body's mass is summed as the integer m 2^mass_shift and
         // its moment as m x 2^mom_shift, both rounded; the shifts keep every sum of all n
-        // bodies below 2^61 (from the largest finite |m| and |x|, see box_final_kernel).
+        // bodies below 2^61 (from the largest finite |m| and |x|, see finish_box).
         int mass_shift;
         int mom_shift;
         float edge_f;       // the edge in float (exact: a float size or a power of two)
