@@ -215,8 +215,10 @@ namespace nbg
     // Bound by the FP32 pipe (12 packed instructions a source and pair of targets, and the Kahan
     // steps of every 64 sources). Eight sources an iteration overlap their chains, and CTAs of two
     // warps pack evenly: 1,000 bodies took 73 us with 1,024 targets a CTA and whole-wave splits,
-    // now 14; 8,192 79, now 47; 20,011 195, now 178; 50,021 970, now 939; 100,003 3.78 ms, now 3.61.
-    template <int T, int BLOCK, int LAW>
+    // now 14; 8,192 79, now 47; 20,011 195, now 178; 50,021 970, now 939. DUP: each landed tile is
+    // first rewritten as operand pairs {x,x,y,y}, {z,z,m,m} (see direct.cu), for large systems
+    // with two sources an iteration (100,003: 3.58 ms against 3.61; 2^20: 380 against 385).
+    template <int T, int BLOCK, int LAW, bool DUP>
     __global__ void __launch_bounds__(BLOCK, 2 * 256 / BLOCK * 4 / T)
     direct_comp_kernel(const float4* __restrict__ src, const float* __restrict__ radius2, const int* __restrict__ tlist,
                        const int nt, const int n, const int chunk, const float G, const float eps2,
@@ -224,6 +226,7 @@ namespace nbg
     {
         constexpr int P = T / 2;
         __shared__ __align__(128) float4 tile[kStages][kTileC];
+        __shared__ __align__(16) float4 pairs[DUP ? 2 * kTileC : 1];
         __shared__ __align__(8) uint64_t bar[kStages];
         const int tid = threadIdx.x;
         const int base = blockIdx.x * (BLOCK * T);
@@ -291,13 +294,33 @@ namespace nbg
                 __syncthreads();
             }
             const float4* tl = tile[stage];
+            if (DUP)
+            {
+                for (int j = tid; j < kTileC; j += BLOCK)
+                {
+                    const float4 s = tl[j];
+                    pairs[2 * j] = make_float4(s.x, s.x, s.y, s.y);
+                    pairs[2 * j + 1] = make_float4(s.z, s.z, s.w, s.w);
+                }
+                __syncthreads();
+            }
             for (int sb = 0; sb < kTileC; sb += kSub)
             {
-#pragma unroll 8
+#pragma unroll (DUP ? 2 : 8)
                 for (int j = sb; j < sb + kSub; ++j)
                 {
-                    const float4 v = tl[j];
-                    const float2 sx = f2(v.x), sy = f2(v.y), sz = f2(v.z), sm = f2(v.w);
+                    float2 sx, sy, sz, sm;
+                    if (DUP)
+                    {
+                        const float4 a = pairs[2 * j], b = pairs[2 * j + 1];
+                        sx = make_float2(a.x, a.y), sy = make_float2(a.z, a.w);
+                        sz = make_float2(b.x, b.y), sm = make_float2(b.z, b.w);
+                    }
+                    else
+                    {
+                        const float4 v = tl[j];
+                        sx = f2(v.x), sy = f2(v.y), sz = f2(v.z), sm = f2(v.w);
+                    }
 #pragma unroll
                     for (int p = 0; p < P; ++p)
                         interact2c<LAW>(sx, sy, sz, sm, nx[p], ny[p], nz[p], lim[p], ax[p], ay[p], az[p]);
@@ -707,12 +730,16 @@ namespace nbg
             const int ni = static_cast<int>(n), nti = static_cast<int>(nt);
             const bool fp64 = p->precision == NBODY_PREC_FP64;
             const int sms = sms_of(ctx);
-            constexpr int kB = 64, kB64 = 128;
+            constexpr int kB64 = 128;
             // compensated: four targets a lane from 5e8 pairs (20,011 bodies 178 us with two and 184
-            // with four, 32,768: 434 and 422, 50,021: 970 and 939), two below
-            const int targets = static_cast<double>(nt) * n < 5e8 ? 2 : 4;
+            // with four, 32,768: 434 and 422, 50,021: 970 and 939), two below; pre-paired and in
+            // larger CTAs from 8e9 (63,246: 1,487 and 1,506, 100,003: 3,614 and 3,583 without and with)
+            const double pairs = static_cast<double>(nt) * static_cast<double>(n);
+            const int targets = pairs < 5e8 ? 2 : 4;
+            const bool dup = pairs >= 8e9;
+            const int block = fp64 ? kB64 : (dup ? 256 : 64);
             const Split sp = fp64 ? plan_split64(nt, n, kB64 * 2, kTile64, sms)
-                                  : plan_split(nt, n, kB * targets, kTileC, sms);
+                                  : plan_split(nt, n, block * targets, kTileC, sms);
             // scratch: partials (js * nt double4) + radius^2 (n floats)
             const size_t part_bytes = static_cast<size_t>(sp.js) * nt * sizeof(double4);
             const size_t rad_bytes = (p->law == NBODY_LAW_CUTOFF) ? n * sizeof(float) : 0;
@@ -742,11 +769,13 @@ namespace nbg
             else
             {
                 const bool soft = p->law == NBODY_LAW_SOFTENED;
-                const auto fn = targets == 2 ? (soft ? direct_comp_kernel<2, kB, NBODY_LAW_SOFTENED>
-                                                : direct_comp_kernel<2, kB, NBODY_LAW_CUTOFF>)
-                                        : (soft ? direct_comp_kernel<4, kB, NBODY_LAW_SOFTENED>
-                                                : direct_comp_kernel<4, kB, NBODY_LAW_CUTOFF>);
-                fn<<<grid, kB, 0, st>>>(s.off, rad2, tlist, nti, ni, sp.chunk, p->G, p->eps2, part, ctx->dev_error);
+                const auto fn = targets == 2 ? (soft ? direct_comp_kernel<2, 64, NBODY_LAW_SOFTENED, false>
+                                                     : direct_comp_kernel<2, 64, NBODY_LAW_CUTOFF, false>)
+                                : dup ? (soft ? direct_comp_kernel<4, 256, NBODY_LAW_SOFTENED, true>
+                                              : direct_comp_kernel<4, 256, NBODY_LAW_CUTOFF, true>)
+                                      : (soft ? direct_comp_kernel<4, 64, NBODY_LAW_SOFTENED, false>
+                                              : direct_comp_kernel<4, 64, NBODY_LAW_CUTOFF, false>);
+                fn<<<grid, block, 0, st>>>(s.off, rad2, tlist, nti, ni, sp.chunk, p->G, p->eps2, part, ctx->dev_error);
                 ++ctx->launches;
             }
             float4* acc = (write_acc && ctx->layout == NBODY_LAYOUT_SOA) ? ctx->acc : nullptr;
@@ -756,7 +785,7 @@ namespace nbg
             DirectPlan& lp = ctx->last_plan;
             lp = DirectPlan{};
             lp.T = fp64 ? 2 : targets;
-            lp.block = fp64 ? kB64 : kB;
+            lp.block = block;
             lp.tile = fp64 ? kTile64 : kTileC;
             lp.jsplit = sp.js;
             lp.chunk = sp.chunk;

@@ -220,10 +220,10 @@ def test_fp64_sizes_and_ranges(gpu, law, n, scale_pos):
 
 
 @pytest.mark.parametrize("law", [0, 1], ids=["cutoff", "softened"])
-@pytest.mark.parametrize("n", [1, 2, 63, 129, 257, 1000, 8191, 22360, 22361])
+@pytest.mark.parametrize("n", [1, 2, 63, 129, 257, 1000, 8191, 22360, 22361, 89442, 89443])
 def test_compensated_sums_of_other_splits_agree(gpu, n, law):
     """The compensated sum at the edges of its target blocks and source tiles, and on either side
-    of 5e8 pairs: a sample of the targets (other blocks, another split, another shape) against
+    of 5e8 and 8e9 pairs: a sample of the targets (other blocks, another split, another shape) against
     the accelerations of all of them. A Kahan step rounds the 64-source sum it adds once, which
     is 2^-24 of the terms' magnitudes in all for either, and the stored accelerations are
     rounded to FP32 once more. Repeats are identical."""
