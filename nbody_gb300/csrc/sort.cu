@@ -40,6 +40,11 @@ namespace nbg
         constexpr int kPer = kDigits / kThreads;      // digits per thread in the per-digit steps
         constexpr int kMaxPasses = 16;      // of the two sorts that share one set of temporaries
         constexpr int kHistThreads = 1024;
+        // Tiles an SM up to which a pass is bound by latency (1.2M keys): two CTAs of 64 registers
+        // fit an SM, and a pass of one wave gains by AHEAD (see digit_pass): a Barnes-Hut step of
+        // 65,536 bodies 141.9 -> 133.4 us, of 262,144 201.4 -> 197.2, of 1,000,003 419.5 -> 410.5.
+        // Beyond, three CTAs of 40 registers hide the latency, and votes and matches cost the same.
+        constexpr int kAheadTiles = 2;
 
         // A tile's published count for one digit: flag in bits 62-63, the pass's epoch
         // (pass + 1) in bits 32-61, the count in bits 0-31. A word from an earlier pass (or
@@ -158,9 +163,30 @@ namespace nbg
         return L2 ? __ldcg(p) : *p;
     }
 
+    // The lanes of the warp whose d (9 bits, kDigits for none) is this lane's. With VOTES by a
+    // vote a bit: a fixed number of instructions, and those of independent calls overlap, where
+    // a match takes a turn for every distinct d.
+    template <bool VOTES>
+    __device__ __forceinline__ unsigned same_digit(const unsigned d)
+    {
+        if (!VOTES)
+            return __match_any_sync(0xffffffffu, d);
+        unsigned peers = 0xffffffffu;
+#pragma unroll
+        for (int b = 0; b <= kBits; ++b)
+        {
+            const bool set = (d >> b) & 1u;
+            const unsigned m = __ballot_sync(0xffffffffu, set);
+            peers &= set ? m : ~m;
+        }
+        return peers;
+    }
+
     // One pass over the tiles that this CTA takes: until none is left when PERSIST, else one.
-    // smem: kPassSmem bytes.
-    template <bool PERSIST>
+    // smem: kPassSmem bytes. AHEAD, for a grid that leaves each SM a CTA or two, spends
+    // registers and instructions on latency: digits matched by votes, the values and the
+    // global counts loaded with the keys.
+    template <bool PERSIST, bool AHEAD = false>
     __device__ __forceinline__ void digit_pass(unsigned char* smem, const uint64_t* __restrict__ keys,
                                                const uint32_t* __restrict__ vals, uint64_t* __restrict__ keys_out,
                                                uint32_t* __restrict__ vals_out, const int n, const int shift,
@@ -197,19 +223,31 @@ namespace nbg
             // load and rank (out-of-range lanes take digit kDigits, which no key has: they are
             // matched among themselves, counted nowhere and never written)
             uint64_t key[kRounds];
-            uint32_t rank[kRounds];
+            uint32_t rank[kRounds], val[AHEAD ? kRounds : 1], ahead[AHEAD ? kPer : 1];
 #pragma unroll
             for (int r = 0; r < kRounds; ++r)
             {
                 const int i = base + r * 32 + lane;
                 key[r] = i < n ? fetch<PERSIST>(&keys[i]) : 0ull;
             }
+            if (AHEAD)
+            {
+#pragma unroll
+                for (int r = 0; r < kRounds; ++r)
+                {
+                    const int i = base + r * 32 + lane;
+                    val[r] = i < n ? fetch<PERSIST>(&vals[i]) : 0u;
+                }
+#pragma unroll
+                for (int q = 0; q < kPer; ++q)
+                    ahead[q] = fetch<PERSIST>(&ghist[threadIdx.x * kPer + q]);
+            }
 #pragma unroll
             for (int r = 0; r < kRounds; ++r)
             {
                 const bool ok = base + r * 32 + lane < n;
                 const unsigned d = ok ? static_cast<unsigned>((key[r] >> shift) & kMask) : static_cast<unsigned>(kDigits);
-                const unsigned peers = __match_any_sync(0xffffffffu, d);
+                const unsigned peers = same_digit<AHEAD>(d);
                 const int leader = __ffs(peers) - 1;
                 uint32_t before = 0;
                 if (lane == leader && ok)
@@ -256,7 +294,7 @@ namespace nbg
                 block_exclusive(total, start, warp_sum[0]);
 #pragma unroll
                 for (int q = 0; q < kPer; ++q)
-                    gcount[q] = fetch<PERSIST>(&ghist[threadIdx.x * kPer + q]);
+                    gcount[q] = AHEAD ? ahead[AHEAD ? q : 0] : fetch<PERSIST>(&ghist[threadIdx.x * kPer + q]);
                 block_exclusive(gcount, gstart, warp_sum[1]);
 #pragma unroll
                 for (int q = 0; q < kPer; ++q)
@@ -277,7 +315,7 @@ namespace nbg
                 const unsigned d = static_cast<unsigned>((key[r] >> shift) & kMask);
                 const uint32_t pos = digit_start[d] + warp_cnt[warp * kDigits + d] + rank[r];
                 stage_k[pos] = key[r];
-                stage_v[pos] = fetch<PERSIST>(&vals[i]);
+                stage_v[pos] = AHEAD ? val[AHEAD ? r : 0] : fetch<PERSIST>(&vals[i]);
             }
             // decoupled look-back: sum the earlier tiles' counts of each digit, four tiles per
             // step, back to the nearest tile that has published an inclusive count
@@ -364,6 +402,17 @@ namespace nbg
         after_previous();
         extern __shared__ __align__(16) unsigned char smem[];
         digit_pass<false>(smem, keys, vals, keys_out, vals_out, n, shift, pass, ghist, status, ticket, err);
+    }
+
+    __global__ void __launch_bounds__(kThreads, 2) digit_pass_ahead_kernel(
+        const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t* __restrict__ keys_out,
+        uint32_t* __restrict__ vals_out, const int n, const int shift, const int pass,
+        const uint32_t* __restrict__ ghist, uint64_t* __restrict__ status, uint32_t* __restrict__ ticket,
+        unsigned* __restrict__ err)
+    {
+        after_previous();
+        extern __shared__ __align__(16) unsigned char smem[];
+        digit_pass<false, true>(smem, keys, vals, keys_out, vals_out, n, shift, pass, ghist, status, ticket, err);
     }
 
     // Every CTA of the grid arrives, then goes on; *count counts arrivals over all barriers and
@@ -466,10 +515,14 @@ namespace nbg
         const int passes = (end_bit - begin_bit + kBits - 1) / kBits;
         if (passes < 1 || passes > kMaxPasses)
             return cudaErrorInvalidValue;
-        static const cudaError_t attr = allow_smem(reinterpret_cast<const void*>(digit_pass_kernel));
+        static const cudaError_t attr = [] {
+            const cudaError_t a = allow_smem(reinterpret_cast<const void*>(digit_pass_kernel));
+            return a != cudaSuccess ? a : allow_smem(reinterpret_cast<const void*>(digit_pass_ahead_kernel));
+        }();
         if (attr != cudaSuccess)
             return attr;
         const int tiles = static_cast<int>((n + kTile - 1) / kTile);
+        const auto pass_kernel = tiles <= kAheadTiles * sm_count() ? digit_pass_ahead_kernel : digit_pass_kernel;
         const TempLayout t = layout(temp, static_cast<size_t>(tiles));
         const int hist_grid = std::max(1, std::min((static_cast<int>(n) + kHistThreads - 1) / kHistThreads, 2 * sm_count()));
         launch_after(early, digit_hist_kernel, hist_grid, kHistThreads, 0, stream, keys, static_cast<int>(n), begin_bit, passes, t.ghist);
@@ -481,7 +534,7 @@ namespace nbg
         uint32_t* vout = vals_alt;
         for (int p = 0; p < passes && e == cudaSuccess; ++p)
         {
-            launch_after(early, digit_pass_kernel, tiles, kThreads, kPassSmem, stream, kin, vin, kout, vout, static_cast<int>(n),
+            launch_after(early, pass_kernel, tiles, kThreads, kPassSmem, stream, kin, vin, kout, vout, static_cast<int>(n),
                                                                       begin_bit + p * kBits, p, t.ghist + p * kDigits,
                                                                       t.status, t.tickets + p, err);
             ++*launches;

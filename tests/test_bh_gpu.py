@@ -737,3 +737,10 @@ def test_tree_of_nodes_with_far_ends(gpu, n):
     assert len(nodes) == len(ref)
     assert np.array_equal(nodes["next"], [r[4] for r in ref])
     assert np.array_equal(nodes["children"], [r[5] for r in ref])
+
+
+@pytest.mark.parametrize("past", [0, 1])
+def test_sort_order_around_two_tiles_an_sm(gpu, past):
+    """The last size of the passes that spend registers on latency, and the first one beyond."""
+    import torch
+    test_sort_order_at_tile_edges(gpu, 2 * torch.cuda.get_device_properties(0).multi_processor_count * 4096 + past)
