@@ -143,14 +143,14 @@ namespace nbg
                 return false;
             }
             const int cnt = min(kTile, jn - k * kTile);
-            // pad to whole pairs with massless sources at the origin, which add exactly
-            // zero under both laws (the copy wrote [0, cnt))
+            // pad to whole pairs with sources that add exactly zero under both laws (the copy
+            // wrote [0, cnt))
             const int padded = (cnt + 1) & ~1;
             if (DUP)
             {
                 for (int j = tid; j < padded; j += BLOCK)
                 {
-                    const float4 v = j < cnt ? sh.tile[stage][j] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 v = j < cnt ? sh.tile[stage][j] : no_source<LAW>();
                     sh.dup[2 * j] = make_float4(v.x, v.x, v.y, v.y);
                     sh.dup[2 * j + 1] = make_float4(v.z, v.z, v.w, v.w);
                 }
@@ -171,7 +171,7 @@ namespace nbg
                 if (padded > cnt)
                 {
                     if (tid == 0)
-                        sh.tile[stage][cnt] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        sh.tile[stage][cnt] = no_source<LAW>();
                     __syncthreads();
                 }
                 const float4* tl = sh.tile[stage];

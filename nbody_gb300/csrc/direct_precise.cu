@@ -290,7 +290,7 @@ namespace nbg
             if (cnt < kTileC)
             {
                 for (int k = cnt + tid; k < kTileC; k += BLOCK)
-                    tile[stage][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    tile[stage][k] = no_source<LAW>();
                 __syncthreads();
             }
             const float4* tl = tile[stage];

@@ -51,9 +51,9 @@ namespace nbg
         const int len = (n + kSlices - 1) / kSlices;
         const int j0 = min(n, (static_cast<int>(blockIdx.y) * kWarps + warp) * len), j1 = min(n, j0 + len);
 
-        // a massless source at the origin past the slice's end: it adds exactly zero
+        // past the slice's end a source that adds exactly zero
         auto fetch = [&](const int j) {
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 s = no_source<LAW>();
             if (j < j1)
             {
                 s = src[static_cast<size_t>(j) * REC];

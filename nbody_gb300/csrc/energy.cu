@@ -108,7 +108,7 @@ namespace nbg
         for (int j0 = static_cast<int>(first); j0 < last; j0 += kEBlock)
         {
             const int j = j0 + tid;
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);     // padding: massless, adds 0
+            float4 s = no_source<NBODY_LAW_CUTOFF>();     // padding: adds 0
             if (j < n)
             {
                 s = src[static_cast<size_t>(j) * stride];

@@ -413,3 +413,40 @@ def test_planned_shapes(gpu, n, layout, law):
     tg = np.unique(np.r_[0, n - 1, np.random.default_rng(n).integers(0, n, 60)])
     err = scaled_err(out[tg], b, law, eps2=eps2, targets=tg)
     assert err.max() <= TOL_MAX and np.median(err) <= TOL_MEDIAN
+
+
+@pytest.mark.parametrize("layout", [0, 1], ids=["soa", "aos"])
+@pytest.mark.parametrize("how", ["fp32", "comp", "batch", "energy"])
+@pytest.mark.parametrize("n", [2, 9, 768, 1000, 8193, 9001])
+def test_body_next_to_the_origin(gpu, n, how, layout):
+    """A body of radius 0 closer to the origin than 1e-19 under the cutoff law, at sizes whose last
+    slice or tile is filled up with massless sources: what fills it up adds nothing, so that
+    every sum is finite and meets the file's bar. (The energy's terms have one sign, and each is
+    within 4 units of 2^-23: its argument's rounding, the reciprocal root's 2 and the product's.)"""
+    from nbody_gb300 import scenes
+    if how == "batch" and layout == gpu.LAYOUT_AOS:
+        pytest.skip("batched systems run on the split layout")
+    b = scenes.uniform_cube(n, seed=n)
+    b[:, 3] = 0.0
+    b[n // 2, :3] = (1e-20, 0, 0)
+    p = gpu.params(law=gpu.LAW_CUTOFF, precision=gpu.PREC_COMPENSATED if how == "comp" else gpu.PREC_FP32,
+                   mode=gpu.MODE_BATCHED if how == "batch" else gpu.MODE_N2)
+    tg = np.unique(np.r_[0, n // 2, n - 1, np.random.default_rng(n).integers(0, n, 60)])
+    with gpu.Context(layout) as ctx:
+        ctx.upload_bodies(b)
+        if how == "energy":
+            e = ctx.energy(p)["potential"]
+            x, v, m = (b[:, c].astype(np.float64) for c in (slice(0, 3), slice(4, 7), 7))
+            ref = O.energy_f64(x, v, m, 1.0, 0.0)[1]
+            assert abs(e - ref) <= 4 * 2.0 ** -23 * abs(ref), (e, ref)
+            return
+        if how == "batch":
+            ctx.set_systems([0, n])
+        shapes = range(-1, gpu.Context.direct_variant_count()) if how == "fp32" else [-1]
+        for shape in shapes:
+            ctx.set_direct_variant(shape)
+            ctx.accelerate(p)
+            out = ctx.download_bodies()[:, 8:11]
+            assert np.isfinite(out).all(), shape
+            err = scaled_err(out[tg], b, O.LAW_CUTOFF, targets=tg)
+            assert err.max() <= TOL_MAX and np.median(err) <= TOL_MEDIAN, (shape, err.max())
