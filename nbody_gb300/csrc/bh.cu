@@ -114,12 +114,13 @@ namespace nbg
         BoxParams* box = nullptr;
         float* bbox_part = nullptr;
         unsigned* box_ticket = nullptr; // blocks that have left their bounds; 0 between builds
+        bool small_ready = false;       // box, bbox_part and box_ticket are there
         unsigned long long* stats = nullptr;   // [0] interactions, [1] node visits, [2] octree nodes,
                                                // [3] the traversal's tile counter, [4] the Morton
                                                // sort's full-sort flag (as unsigned)
         const uint32_t* order = nullptr;       // sorted indices of the last build (keys/vals ping-pong)
         const uint64_t* codes = nullptr;
-        bool built = false;                    // a tree for built_n bodies is on the device
+        bool built = false;                    // a whole tree, for built_n bodies, is on the device
         cudaEvent_t ev[3] = { nullptr, nullptr, nullptr };  // build start, traversal start, end
         bool timed = false;                    // ev[] bracket the last accelerate
         size_t built_n = 0;
@@ -2217,18 +2218,18 @@ namespace nbg
             if (!ctx->bh)
                 ctx->bh = new BhState();
             BhState& b = *ctx->bh;
-            if (!b.box)
+            if (!b.small_ready)
             {
-                cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&b.box), sizeof(BoxParams), ctx->stream);
+                cudaError_t e = grow(&b.box, 1, ctx->stream);
                 if (e == cudaSuccess)
-                    e = cudaMallocAsync(reinterpret_cast<void**>(&b.bbox_part), kBboxBlocks * kBboxVals * sizeof(float),
-                                        ctx->stream);
+                    e = grow(&b.bbox_part, kBboxBlocks * kBboxVals, ctx->stream);
                 if (e == cudaSuccess)
-                    e = cudaMallocAsync(reinterpret_cast<void**>(&b.box_ticket), sizeof(unsigned), ctx->stream);
+                    e = grow(&b.box_ticket, 1, ctx->stream);
                 if (e == cudaSuccess)
                     e = cudaMemsetAsync(b.box_ticket, 0, sizeof(unsigned), ctx->stream);
                 if (e != cudaSuccess)
                     return ctx_cuda_fail(ctx, e, "tree allocation");
+                b.small_ready = true;
             }
             if (n <= b.cap)
                 return NBODY_OK;
@@ -2242,12 +2243,16 @@ namespace nbg
                                          scan_temp_elems(cap) * sizeof(uint32_t) });
             cudaError_t e = cudaSuccess;
             cudaStream_t s = ctx->stream;
+            // the last tree goes with its buffers, also when not all of the new ones can be had
+            b.built = false;
             for (int k = 0; k < 2 && e == cudaSuccess; ++k)
             {
                 e = grow(&b.keys[k], cap, s);
                 if (e == cudaSuccess)
                     e = grow(&b.vals[k], cap, s);
             }
+            if (e == cudaSuccess && fault_injected("tree"))
+                e = cudaErrorMemoryAllocation;
             if (e == cudaSuccess) e = grow(&b.spm, cap, s);
             if (e == cudaSuccess) e = grow(&b.srad, cap, s);
             if (e == cudaSuccess) e = grow(&b.child, cap, s);
@@ -2307,6 +2312,7 @@ namespace nbg
         if (const int st = reserve_bh(ctx, n))
             return st;
         BhState& b = *ctx->bh;
+        b.built = false;    // until all that makes a tree is launched
         cudaStream_t s = ctx->stream;
         int stride = 1;
         const float4* src = body_src(ctx, &stride);
@@ -2364,6 +2370,9 @@ namespace nbg
         ++L;
         if (n < 2)
         {
+            e = cudaGetLastError();
+            if (e != cudaSuccess)
+                return ctx_cuda_fail(ctx, e, "tree build");
             b.built = true;
             b.built_n = n;
             ++b.build_id;
@@ -2574,7 +2583,7 @@ namespace nbg
 
     uint64_t bh_build_id(const nbody_cuda* ctx)
     {
-        return (ctx->bh && ctx->bh->built) ? ctx->bh->build_id : 0;
+        return ctx->bh ? ctx->bh->build_id : 0;
     }
 
     int bh_view(nbody_cuda* ctx, TreeView* out)

@@ -58,7 +58,7 @@ namespace nbg
 
     int bh_build(nbody_cuda* ctx, const nbody_step_params* p);
     int bh_view(nbody_cuda* ctx, TreeView* out);
-    uint64_t bh_build_id(const nbody_cuda* ctx);    // 0 before the first build
+    uint64_t bh_build_id(const nbody_cuda* ctx);    // of the last whole build; 0 before the first
     int bh_stats(nbody_cuda* ctx, unsigned long long out[3]);
     int bh_stage_ms(nbody_cuda* ctx, float ms[2]);
     int bh_morton(nbody_cuda* ctx, const nbody_step_params* p, uint64_t* codes, uint32_t* order, double box[4]);

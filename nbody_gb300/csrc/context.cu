@@ -62,12 +62,6 @@ namespace
             return cuda_fail((ctx), e_, (what));        \
     } while (0)
 
-    bool fault_injected(const char* what)
-    {
-        const char* f = std::getenv("NBODY_CUDA_FAULT");
-        return f && std::strcmp(f, what) == 0;
-    }
-
     int check_params(nbody_cuda* ctx, const nbody_step_params* p)
     {
         if (!p)
@@ -110,6 +104,12 @@ namespace nbg
     int ctx_cuda_fail(nbody_cuda* ctx, const cudaError_t e, const char* what)
     {
         return cuda_fail(ctx, e, what);
+    }
+
+    bool fault_injected(const char* what)
+    {
+        const char* f = std::getenv("NBODY_CUDA_FAULT");
+        return f && std::strcmp(f, what) == 0;
     }
 
     int before_allocation(nbody_cuda* ctx)

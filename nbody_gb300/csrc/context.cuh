@@ -145,6 +145,8 @@ namespace nbg
     // pointers a graph holds must stay valid), and it retires any captured graph.
     int before_allocation(nbody_cuda* ctx);
     int check_device_error(nbody_cuda* ctx);
+    // Whether NBODY_CUDA_FAULT names this failure (host-side fault injection for tests).
+    bool fault_injected(const char* what);
 
     // context.cu: copies through the pinned staging buffer, and the device-side Body staging
     int staging(nbody_cuda* ctx, size_t bytes, void** out);

@@ -238,14 +238,14 @@ namespace nbg
 
     int tree_on_device(nbody_cuda* ctx, size_t* count)
     {
-        TreeView t;
-        if (const int st = bh_view(ctx, &t))
-            return st;
-        if (ctx->query_nodes_id == t.build_id)
+        if (const uint64_t id = bh_build_id(ctx); id && ctx->query_nodes_id == id)
         {
             *count = ctx->query_nodes_count;
             return NBODY_OK;
         }
+        TreeView t;
+        if (const int st = bh_view(ctx, &t))
+            return st;
         cudaStream_t s = ctx->stream;
         const int n = t.n;
         uint32_t* counts = t.words[0];

@@ -42,3 +42,35 @@ def test_injected_allocation_failure_is_reported(gpu, monkeypatch):
     with pytest.raises(gpu.NbodyError) as e:
         gpu.Context()
     assert e.value.status == gpu.ERR_ALLOC
+
+
+@pytest.mark.parametrize("exported", [False, True])
+def test_tree_that_lost_its_buffers(gpu, monkeypatch, exported):
+    """A build whose larger buffers cannot be had gives up the last tree's: an export or a query
+    of it is then refused, or served from the copy an earlier export left, and never reads the
+    buffers that are gone. The next build works again."""
+    from nbody_gb300 import scenes
+    small, large = scenes.plummer(100, seed=3), scenes.plummer(5000, seed=4)
+    p = gpu.params(mode=gpu.MODE_NLOGN, law=gpu.LAW_CUTOFF, theta=0.5, size=0.0, tree_box=1)
+    ray = np.array([[0, 0, 0, 1, 2, 3]], np.float32)
+    with gpu.Context() as ctx:
+        ctx.upload_bodies(small)
+        ctx.accelerate(p)
+        before = ctx.tree_export() if exported else None
+        ctx.upload_bodies(large)
+        monkeypatch.setenv("NBODY_CUDA_FAULT", "tree")
+        with pytest.raises(gpu.NbodyError) as e:
+            ctx.accelerate(p)
+        assert e.value.status == gpu.ERR_ALLOC
+        monkeypatch.delenv("NBODY_CUDA_FAULT")
+        if exported:
+            assert np.array_equal(ctx.tree_export(), before)
+            assert ctx.tree_query(ray)[1][0] > 0
+        else:
+            for call in (ctx.tree_export, lambda: ctx.tree_query(ray)):
+                with pytest.raises(gpu.NbodyError) as e:
+                    call()
+                assert e.value.status == gpu.ERR_INVALID
+        ctx.accelerate(p)
+        nodes = ctx.tree_export()
+        assert len(nodes) > 5000 and nodes["mass"][0] == pytest.approx(large[:, 7].sum(dtype=np.float64), rel=1e-6)
