@@ -114,6 +114,7 @@ namespace nbg
         BoxParams* box = nullptr;
         float* bbox_part = nullptr;
         unsigned* box_ticket = nullptr; // blocks that have left their bounds; 0 between builds
+        SortSetup sort;
         bool small_ready = false;       // box, bbox_part and box_ticket are there
         unsigned long long* stats = nullptr;   // [0] interactions, [1] node visits, [2] octree nodes,
                                                // [3] the traversal's tile counter, [4] the Morton
@@ -2231,6 +2232,9 @@ namespace nbg
                     return ctx_cuda_fail(ctx, e, "tree allocation");
                 b.small_ready = true;
             }
+            if (!b.sort.sms)
+                if (const cudaError_t e = setup_sort(&b.sort))
+                    return ctx_cuda_fail(ctx, e, "radix sort set-up");
             if (n <= b.cap)
                 return NBODY_OK;
             if (const int st = before_allocation(ctx))
@@ -2331,7 +2335,7 @@ namespace nbg
         ++L;
         bool in_alt = false;
         cudaError_t e = radix_sort_pairs(b.keys[0], b.vals[0], b.keys[1], b.vals[1], n, kRunShift, 63, b.temp, s, &L,
-                                         &in_alt, ctx->dev_error, early);
+                                         &in_alt, ctx->dev_error, early, b.sort);
         if (e != cudaSuccess)
             return ctx_cuda_fail(ctx, e, "radix sort");
         if (n > 1)
@@ -2343,7 +2347,7 @@ namespace nbg
             launch_after(early, run_sort_kernel, ceil_div(n, 256), 256, 0, s, b.keys[cur], b.vals[cur], ni, full);
             ++L;
             e = radix_sort_if(b.keys[cur], b.vals[cur], b.keys[1 - cur], b.vals[1 - cur], n, 0, 63, b.temp,
-                              (63 - kRunShift + 8) / 9, s, &L, ctx->dev_error, full);
+                              (63 - kRunShift + 8) / 9, s, &L, ctx->dev_error, full, b.sort);
             if (e != cudaSuccess)
                 return ctx_cuda_fail(ctx, e, "radix sort");
         }

@@ -429,13 +429,10 @@ namespace nbg
 
         int sm_count()
         {
-            static int sms = [] {
-                int dev = 0, s = 0;
-                cudaGetDevice(&dev);
-                cudaDeviceGetAttribute(&s, cudaDevAttrMultiProcessorCount, dev);
-                return s > 0 ? s : 1;
-            }();
-            return sms;
+            int dev = 0, sms = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            return std::max(1, sms);
         }
     }
 

@@ -486,26 +486,31 @@ namespace nbg
 
     size_t sort_temp_bytes(const size_t n) { return sort_zero_bytes(n) + 256; }
 
-    namespace
+    cudaError_t setup_sort(SortSetup* setup)
     {
-        int sm_count()
-        {
-            int dev = 0, sms = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            return std::max(1, sms);
-        }
-
-        cudaError_t allow_smem(const void* fn)
-        {
-            return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPassSmem));
-        }
+        for (const void* fn : { reinterpret_cast<const void*>(digit_pass_kernel),
+                                reinterpret_cast<const void*>(digit_pass_ahead_kernel),
+                                reinterpret_cast<const void*>(whole_sort_kernel) })
+            if (const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                           static_cast<int>(kPassSmem)))
+                return e;
+        int dev = 0, sms = 0, per_sm = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess)
+            e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, whole_sort_kernel, kThreads, kPassSmem);
+        if (e != cudaSuccess)
+            return e;
+        setup->sms = std::max(1, sms);
+        setup->whole_per_sm = std::max(1, per_sm);
+        return cudaSuccess;
     }
 
     cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt,
                                  const size_t n, const int begin_bit, const int end_bit, void* temp,
                                  cudaStream_t stream, uint64_t* launches, bool* in_alt, unsigned* err,
-                                 const bool early)
+                                 const bool early, const SortSetup& setup)
     {
         *in_alt = false;
         if (n <= 1)
@@ -515,16 +520,10 @@ namespace nbg
         const int passes = (end_bit - begin_bit + kBits - 1) / kBits;
         if (passes < 1 || passes > kMaxPasses)
             return cudaErrorInvalidValue;
-        static const cudaError_t attr = [] {
-            const cudaError_t a = allow_smem(reinterpret_cast<const void*>(digit_pass_kernel));
-            return a != cudaSuccess ? a : allow_smem(reinterpret_cast<const void*>(digit_pass_ahead_kernel));
-        }();
-        if (attr != cudaSuccess)
-            return attr;
         const int tiles = static_cast<int>((n + kTile - 1) / kTile);
-        const auto pass_kernel = tiles <= kAheadTiles * sm_count() ? digit_pass_ahead_kernel : digit_pass_kernel;
+        const auto pass_kernel = tiles <= kAheadTiles * setup.sms ? digit_pass_ahead_kernel : digit_pass_kernel;
         const TempLayout t = layout(temp, static_cast<size_t>(tiles));
-        const int hist_grid = std::max(1, std::min((static_cast<int>(n) + kHistThreads - 1) / kHistThreads, 2 * sm_count()));
+        const int hist_grid = std::max(1, std::min((static_cast<int>(n) + kHistThreads - 1) / kHistThreads, 2 * setup.sms));
         launch_after(early, digit_hist_kernel, hist_grid, kHistThreads, 0, stream, keys, static_cast<int>(n), begin_bit, passes, t.ghist);
         ++*launches;
         cudaError_t e = cudaGetLastError();
@@ -548,7 +547,8 @@ namespace nbg
 
     cudaError_t radix_sort_if(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, const size_t n,
                               const int begin_bit, const int end_bit, void* temp, const int pass_base,
-                              cudaStream_t stream, uint64_t* launches, unsigned* err, const unsigned* run_if)
+                              cudaStream_t stream, uint64_t* launches, unsigned* err, const unsigned* run_if,
+                              const SortSetup& setup)
     {
         if (n <= 1)
             return cudaSuccess;
@@ -557,18 +557,10 @@ namespace nbg
         const int passes = (end_bit - begin_bit + kBits - 1) / kBits;
         if (passes < 1 || pass_base < 0 || pass_base + passes > kMaxPasses)
             return cudaErrorInvalidValue;
-        static const cudaError_t attr = allow_smem(reinterpret_cast<const void*>(whole_sort_kernel));
-        if (attr != cudaSuccess)
-            return attr;
-        static const int per_sm = [] {
-            int b = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, whole_sort_kernel, kThreads, kPassSmem);
-            return std::max(1, b);
-        }();
         const int tiles = static_cast<int>((n + kTile - 1) / kTile);
         const TempLayout t = layout(temp, static_cast<size_t>(tiles));
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(static_cast<unsigned>(std::min(tiles, per_sm * sm_count())));
+        cfg.gridDim = dim3(static_cast<unsigned>(std::min(tiles, setup.whole_per_sm * setup.sms)));
         cfg.blockDim = dim3(kThreads);
         cfg.dynamicSmemBytes = kPassSmem;
         cfg.stream = stream;
