@@ -1074,15 +1074,11 @@ namespace nbg
     constexpr uint32_t kIsOct = 0x80000000u;
     constexpr int kNumTile = 4096;      // binary nodes per CTA of the numbering
 
-    // A tile's published count of octree nodes: its own, or with all earlier tiles'.
-    constexpr uint64_t kCountOwn = 1ull << 62, kCountAll = 2ull << 62;
-
     // octidx[i] = the octree nodes among binary nodes 0 .. i - 1, with kIsOct set when node i is one
     // itself (its index in the record array is then octidx[i] without it). One launch: tiles of
-    // 4096 nodes taken in ticket order, the earlier tiles' count found by decoupled look-back,
-    // 32 tiles at a time (the waits are bounded and on CTAs that are running, as in the radix
-    // sort). status[0] is the ticket, status[1 + t] tile t's count, all zero before. A wait that
-    // gives up counts nothing before its tile: indices stay in range.
+    // 4096 nodes taken in ticket order, the earlier tiles' count found by decoupled look-back
+    // (count_before). status[0] is the ticket, status[1 + t] tile t's count, all zero before. A
+    // wait that gives up counts nothing before its tile: indices stay in range.
     __global__ void __launch_bounds__(1024) number_kernel(const uint8_t* __restrict__ flag, const int m,
                                                           uint32_t* __restrict__ octidx, uint64_t* __restrict__ status,
                                                           unsigned* __restrict__ err)
@@ -1130,35 +1126,7 @@ namespace nbg
             const uint32_t total = __shfl_sync(0xffffffffu, wi, 31);
             if (lane == 0)
                 store_relaxed(&status[1 + tile], (tile ? kCountOwn : kCountAll) | total);
-            uint32_t before = 0;
-            uint64_t t0 = 0;
-            for (int j = tile - 1; j >= 0;)
-            {
-                const uint64_t v = j - lane >= 0 ? load_relaxed(&status[1 + j - lane]) : kCountAll;
-                const unsigned missing = __ballot_sync(0xffffffffu, !(v >> 62));
-                const unsigned all = __ballot_sync(0xffffffffu, (v >> 62) == 2);
-                // the lanes before the first missing word, up to and with the first that counts all
-                const unsigned stop = all & (0u - all);
-                const unsigned use = all ? (stop << 1) - 1u : 0xffffffffu;
-                if (missing & use)
-                {
-                    if (!t0)
-                        t0 = globaltimer();
-                    else if (globaltimer() - t0 > kWaitLimitNs)
-                    {
-                        if (lane == 0)
-                            atomicOr(err, DEV_ERR_TIMEOUT);
-                        before = 0;
-                        break;
-                    }
-                    __nanosleep(100);
-                    continue;
-                }
-                before += __reduce_add_sync(0xffffffffu, (use >> lane) & 1u ? static_cast<uint32_t>(v) : 0u);
-                if (all)
-                    break;
-                j -= 32;
-            }
+            const uint32_t before = count_before(status + 1, tile, err);
             if (lane == 0)
             {
                 if (tile)

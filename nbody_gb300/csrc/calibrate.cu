@@ -140,18 +140,29 @@ extern "C" int nbody_cuda_calibrate_fp64(nbody_cuda* ctx, double* tflops)
 namespace nbg
 {
     // Waits on an mbarrier phase that nothing completes (one arrival expected, none made,
-    // no copy issued), with the bounded wait every pipeline uses, so the give-up path runs:
-    // the wait returns after limit_ns, sets DEV_ERR_TIMEOUT and the kernel exits normally.
-    __global__ void selftest_wait_kernel(unsigned* err, const unsigned long long limit_ns)
+    // no copy issued), with the bounded wait every pipeline uses, then for counts that no tile
+    // publishes, with the numbering's look-back, so that both give-up paths run: each wait
+    // returns after limit_ns. Sets DEV_ERR_TIMEOUT when both gave up (and the whole warp
+    // left the second with 0), and exits normally. status: kSelftestTiles zeros.
+    constexpr int kSelftestTiles = 40;
+
+    __global__ void selftest_wait_kernel(const uint64_t* status, unsigned* err, const unsigned long long limit_ns)
     {
         __shared__ __align__(8) uint64_t bar;
+        __shared__ unsigned errs[2];
         if (threadIdx.x == 0)
         {
+            errs[0] = errs[1] = 0;
             mbar_init(&bar, 1);
             fence_mbar_init();
         }
         __syncthreads();
-        mbar_wait_bounded(&bar, 0, err, limit_ns);
+        mbar_wait_bounded(&bar, 0, &errs[0], limit_ns);
+        __syncthreads();
+        const bool none = __all_sync(0xffffffffu, count_before(status, kSelftestTiles, &errs[1], limit_ns) == 0u);
+        __syncthreads();
+        if (threadIdx.x == 0 && none && (errs[0] & errs[1] & DEV_ERR_TIMEOUT))
+            atomicOr(err, DEV_ERR_TIMEOUT);
     }
 }
 
@@ -162,9 +173,16 @@ extern "C" int nbody_cuda_selftest_wait(nbody_cuda* ctx, const uint64_t limit_ns
         return NBODY_ERR_INVALID;
     if (limit_ns == 0 || limit_ns > 100000000ull)
         return ctx_fail(ctx, NBODY_ERR_INVALID, "self-test wait limit must be in (0, 0.1 s]");
-    selftest_wait_kernel<<<1, 32, 0, ctx->stream>>>(ctx->dev_error, limit_ns);
+    const size_t bytes = kSelftestTiles * sizeof(uint64_t);
+    if (const int st = ensure_scratch(ctx, bytes))
+        return st;
+    ctx->pending_partials = 0;      // the scratch is reused here
+    cudaError_t e = cudaMemsetAsync(ctx->scratch, 0, bytes, ctx->stream);
+    if (e != cudaSuccess)
+        return ctx_cuda_fail(ctx, e, "self-test set-up");
+    selftest_wait_kernel<<<1, 32, 0, ctx->stream>>>(static_cast<const uint64_t*>(ctx->scratch), ctx->dev_error, limit_ns);
     ++ctx->launches;
-    const cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess)
         return ctx_cuda_fail(ctx, e, "self-test launch");
     return check_device_error(ctx);

@@ -109,6 +109,49 @@ namespace nbg
         asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
     }
 
+    // A tile's published count: its own, or with all earlier tiles'; 0 while there is none yet.
+    constexpr uint64_t kCountOwn = 1ull << 62, kCountAll = 2ull << 62;
+
+    // The sum of the earlier tiles' counts, status[0 .. tile - 1], by a whole warp: 32 tiles at a
+    // time, back to the nearest one that counts all. The waits are on CTAs that are running. A
+    // wait that gives up after limit_ns records it in *err and returns 0; one lane's clock
+    // decides for the warp, whose lanes stay together for the votes.
+    __device__ __forceinline__ uint32_t count_before(const uint64_t* status, const int tile, unsigned* err,
+                                                     const uint64_t limit_ns = kWaitLimitNs)
+    {
+        const int lane = threadIdx.x & 31;
+        uint32_t before = 0;
+        uint64_t t0 = 0;
+        for (int j = tile - 1; j >= 0;)
+        {
+            const uint64_t v = j - lane >= 0 ? load_relaxed(&status[j - lane]) : kCountAll;
+            const unsigned missing = __ballot_sync(0xffffffffu, !(v >> 62));
+            const unsigned all = __ballot_sync(0xffffffffu, (v >> 62) == 2);
+            // the words up to and with the first that counts all
+            const unsigned stop = all & (0u - all);
+            const unsigned use = all ? (stop << 1) - 1u : 0xffffffffu;
+            if (missing & use)
+            {
+                const uint64_t now = __shfl_sync(0xffffffffu, globaltimer(), 0);
+                if (!t0)
+                    t0 = now;
+                else if (now - t0 > limit_ns)
+                {
+                    if (lane == 0)
+                        atomicOr(err, DEV_ERR_TIMEOUT);
+                    return 0;
+                }
+                __nanosleep(100);
+                continue;
+            }
+            before += __reduce_add_sync(0xffffffffu, (use >> lane) & 1u ? static_cast<uint32_t>(v) : 0u);
+            if (all)
+                break;
+            j -= 32;
+        }
+        return before;
+    }
+
     // Programmatic dependent launch: the first statement of every kernel that launch_after
     // starts. The next kernel of the stream may be made ready as soon as all of this one's CTAs
     // have begun, and this one goes on once every kernel before it has ended and its writes

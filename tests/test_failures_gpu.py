@@ -3,6 +3,7 @@ run out reports NBODY_ERR_TIMEOUT through the device error word and the context 
 working; host-side injected failures surface as statuses with reasons, as the reference's
 probe / constructor failures do (source/gpu.cpp:115-149, source/sim.cpp:226-239)."""
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -74,3 +75,19 @@ def test_tree_that_lost_its_buffers(gpu, monkeypatch, exported):
         ctx.accelerate(p)
         nodes = ctx.tree_export()
         assert len(nodes) > 5000 and nodes["mass"][0] == pytest.approx(large[:, 7].sum(dtype=np.float64), rel=1e-6)
+
+
+def test_look_back_gives_up_as_a_warp(gpu):
+    """The self-test makes both bounded waits run out, the second that of the tree build's
+    look-back, whose warp votes between its looks: its lanes leave together (the kernel checks
+    that), after the limit, and the context goes on to build a tree."""
+    from nbody_gb300 import scenes
+    with gpu.Context() as ctx:
+        ctx.upload_bodies(scenes.plummer(2000, seed=6))
+        ctx.synchronize()
+        start = time.perf_counter()
+        assert gpu.lib().nbody_cuda_selftest_wait(ctx.h, C.c_uint64(50_000_000)) == gpu.ERR_TIMEOUT
+        assert time.perf_counter() - start >= 0.1        # 50 ms each
+        ctx.accelerate(gpu.params(mode=gpu.MODE_NLOGN, law=gpu.LAW_CUTOFF, theta=0.5, size=0.0, tree_box=1))
+        ctx.synchronize()
+        assert ctx.bh_stats()["cells"] > 0
