@@ -27,8 +27,10 @@
 //     combine_partials). The runs are the same sources
 //     for every kernel shape and split, so the result does not depend on the
 //     launch shape (up to a rounding tie of the last fold), and it is more accurate than
-//     one FP32 running sum over all N sources.
+//     one FP32 running sum over all N sources. Systems of up to 3072 bodies are the exception
+//     while no shape is pinned: their own kernel (direct_small.cu) sums shorter runs.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 
 #include "common.cuh"
@@ -386,8 +388,16 @@ namespace nbg
         // with four a lane (100,003: 3.95 against 4.10 ms); the softened sum of 2^20 bodies is 0.5
         // (records: 1.4) % faster with pre-paired tiles, 400,009 the same, 100,003 1.5 % slower.
         constexpr int kPlan = 10, kWideAosPlan = 11, kPairedPlan = 0, kNarrowPlan = 2;
-        constexpr size_t kPairedMinN = 1 << 18;
+        constexpr size_t kPairedMinN = 1 << 18, kPairedNearN = 1 << 16;
         constexpr size_t kMaxSplit = 64;                        // source chunks
+        // Up to 2^14 bodies of the split layout (2^13 body records) every chunk is one tile: CTAs of
+        // 128 targets and 256 sources are enough to pack the SMs evenly, which the fitted cost of a
+        // split does not see at so few CTAs. Split bodies, softened, the plan by that cost (the
+        // small systems' kernel up to 8,192) and this: 4,700 23.0 -> 20.7 us (a step 25.0 -> 18.5),
+        // 8,192 35.2 -> 35.2 (39.2 -> 33.1), 9,555 53.6 -> 46.4, 12,289 76 -> 70, 15,000 101 -> 99.
+        constexpr size_t kOneTileMaxN = kMaxSplit * kTile, kOneTileMaxAos = kOneTileMaxN / 2;
+        // CTAs of kNarrowPlan an SM holds for body records: 44 KB of shared memory each
+        constexpr size_t kNarrowAosCtas = 5;
 
         template <int T, int B, bool PACKED = true, bool DUP = false, int U = 2>
         Variant make_variant()
@@ -467,18 +477,39 @@ namespace nbg
                                 static_cast<double>(sm_count()) };
         };
         int chosen = force_variant;
+        bool most = false;      // as many chunks as there may be
         if (chosen < 0 || chosen >= nv)
         {
             chosen = law == NBODY_LAW_CUTOFF && aos ? kWideAosPlan
                                                     : (law == NBODY_LAW_SOFTENED && n >= kPairedMinN ? kPairedPlan : kPlan);
-            // a small scratch allows few chunks: then CTAs of 128 targets pack better, at 5 %
-            // longer a pair
-            if (split_bytes < kSplitBytes && 1.05 * split_of(kNarrowPlan).least(max_js) < split_of(chosen).least(max_js))
+            if (n <= (aos ? kOneTileMaxAos : kOneTileMaxN) && max_js == units)
+            {
+                // Body records leave an SM five CTAs: where their last wave would be mostly empty,
+                // four times as many targets a CTA instead (7,600 softened: 39.5 against 33.0 us;
+                // 6,500, a wave and three quarters: 30.4 against 33.0).
+                const double waves = static_cast<double>(split_of(kNarrowPlan).tb * units)
+                                     / static_cast<double>(kNarrowAosCtas * sm_count());
+                chosen = !aos || waves >= 0.85 * std::ceil(waves) || waves <= 1.0 ? kNarrowPlan : kWideAosPlan;
+                most = true;
+            }
+            else if (split_bytes < kSplitBytes
+                     && 1.05 * split_of(kNarrowPlan).least(max_js) < split_of(chosen).least(max_js))
+            {
+                // a small scratch allows few chunks: then CTAs of 128 targets pack better, at 5 %
+                // longer a pair, and take all the chunks that fit (41,009 softened: 630 us with 12,
+                // 676 with the 7 of the fitted cost; 50,021: 922 with 10, 975 with 8)
                 chosen = kNarrowPlan;
+                most = true;
+            }
+            else if (chosen == kPlan && law == NBODY_LAW_SOFTENED && n >= kPairedNearN
+                     && split_of(kPairedPlan).least(max_js) < 1.03 * split_of(kPlan).least(max_js))
+                // pre-paired tiles take 5 % less a pair in larger CTAs: where these pack nearly as
+                // well (162,184: 9.25 -> 9.12 ms, records 9.39 -> 9.12; 175,000: 10.64 -> 10.55)
+                chosen = kPairedPlan;
         }
         const Variant& v = vs[chosen];
         const SourceSplit sp = split_of(chosen);
-        const size_t chunk = sp.chunk(max_js, 1.02);
+        const size_t chunk = most ? sp.chunk_units(max_js) * unit : sp.chunk(max_js, 1.02);
         const size_t js = std::max<size_t>(1, (n + chunk - 1) / chunk);
 
         plan.variant = chosen;

@@ -450,3 +450,29 @@ def test_body_next_to_the_origin(gpu, n, how, layout):
             assert np.isfinite(out).all(), shape
             err = scaled_err(out[tg], b, O.LAW_CUTOFF, targets=tg)
             assert err.max() <= TOL_MAX and np.median(err) <= TOL_MEDIAN, (shape, err.max())
+
+
+@pytest.mark.parametrize("layout", [0, 1], ids=["soa", "aos"])
+@pytest.mark.parametrize("law", [0, 1], ids=["cutoff", "softened"])
+@pytest.mark.parametrize("n", [3073, 4700, 5200, 6500, 8192, 8193, 9555, 16384, 16385, 70001])
+def test_unpinned_bits_are_the_shapes(gpu, n, law, layout):
+    """Beyond the small systems' kernel the planned launch, on either side of its lines (a tile a
+    chunk, by the fitted cost, pre-paired), gives the bits of the shapes that can be pinned: up
+    to a rounding tie of the last fold, one component in 10^5. Sampled targets against FP64."""
+    from nbody_gb300 import scenes
+    b = scenes.uniform_cube(n, seed=n)
+    b[:, 3] = np.float32(1e-3)
+    eps2 = 1e-6 if law == gpu.LAW_SOFTENED else 0.0
+    p = gpu.params(law=law, eps2=eps2)
+    with gpu.Context(layout) as ctx:
+        ctx.upload_bodies(b)
+        ctx.accelerate(p)
+        out = ctx.download_bodies()[:, 8:11].copy()
+        for shape in (0, 2, 9, 10, 11):
+            ctx.set_direct_variant(shape)
+            ctx.accelerate(p)
+            pinned = ctx.download_bodies()[:, 8:11]
+            assert np.count_nonzero(out.view(np.uint32) != pinned.view(np.uint32)) <= max(1, 1e-5 * out.size), shape
+    tg = np.unique(np.r_[0, n - 1, np.random.default_rng(n).integers(0, n, 60)])
+    err = scaled_err(out[tg], b, law, eps2=eps2, targets=tg)
+    assert err.max() <= TOL_MAX and np.median(err) <= TOL_MEDIAN
