@@ -711,17 +711,9 @@ int nbody_cuda_direct_autotune(nbody_cuda* ctx, const nbody_step_params* p, doub
     ctx->force_variant = -1;
     if (const int st = direct_accel(ctx, &q, false))
         return st;
-    // a small system's own kernel is not one of the shapes: unpinned, it is what runs
-    float small_ms = 1e30f;
-    for (int rep = 0; rep < 2 && ctx->last_plan.small; ++rep)
-    {
-        cudaEventRecord(ev.start, ctx->stream);
-        const int st = direct_accel(ctx, &q, false);
-        cudaEventRecord(ev.stop, ctx->stream);
-        if (st != NBODY_OK)
-            return st;
-        small_ms = std::min(small_ms, ev.elapsed_ms());
-    }
+    // a small system's own kernel is not one of the shapes: unpinned, it is what runs, and it
+    // stays so whatever the shapes' times, since its sums' bits are not theirs
+    const bool small = ctx->last_plan.small;
     int best_i = 0;
     float best_ms = 1e30f;
     for (int i = 0; i < direct_variant_count(); ++i)
@@ -748,9 +740,9 @@ int nbody_cuda_direct_autotune(nbody_cuda* ctx, const nbody_step_params* p, doub
             best_i = i;
         }
     }
-    ctx->force_variant = small_ms <= best_ms ? -1 : best_i;
+    ctx->force_variant = small ? -1 : best_i;
     if (best)
-        *best = best_i;
+        *best = ctx->force_variant;
     return check_device_error(ctx);
 }
 

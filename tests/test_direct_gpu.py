@@ -476,3 +476,35 @@ def test_unpinned_bits_are_the_shapes(gpu, n, law, layout):
     tg = np.unique(np.r_[0, n - 1, np.random.default_rng(n).integers(0, n, 60)])
     err = scaled_err(out[tg], b, law, eps2=eps2, targets=tg)
     assert err.max() <= TOL_MAX and np.median(err) <= TOL_MEDIAN
+
+
+@pytest.mark.parametrize("layout", [0, 1], ids=["soa", "aos"])
+@pytest.mark.parametrize("n", [1000, 3072, 3073, 9001])
+def test_autotune_pins_what_it_names(gpu, n, layout):
+    """The autotuner names the shape that it pinned, and none (-1) for a system small enough for the
+    kernel of its own, which is no shape: that is left unpinned, so its bits do not hang on
+    timings. A pinned shape's sum of a small system meets the file's bar like the kernel's own."""
+    from nbody_gb300 import scenes
+    b = scenes.plummer(n, seed=n)
+    p = gpu.params(law=gpu.LAW_SOFTENED, eps2=1e-4)
+    with gpu.Context(layout) as ctx:
+        ctx.upload_bodies(b)
+        ctx.accelerate(p)
+        before = ctx.download_bodies()[:, 8:11].copy()
+        best, times = ctx.direct_autotune(p)
+        assert len(times) == gpu.Context.direct_variant_count() and (times > 0).all()
+        ctx.accelerate(p)
+        cfg, after = ctx.last_direct_config(), ctx.download_bodies()[:, 8:11].copy()
+        if n <= 3072:
+            assert best == -1 and np.array_equal(before, after)
+            ctx.set_direct_variant(int(np.argmin(times)))
+            ctx.accelerate(p)
+            after = ctx.download_bodies()[:, 8:11]
+        else:
+            assert best == int(np.argmin(times))
+            assert {k: gpu.Context.direct_variant(best)[k] for k in ("targets_per_thread", "block")} == {
+                k: cfg[k] for k in ("targets_per_thread", "block")}
+            assert np.count_nonzero(before.view(np.uint32) != after.view(np.uint32)) <= 1
+    for a in (before, after):
+        err = scaled_err(a, b, O.LAW_SOFTENED, eps2=1e-4)
+        assert err.max() <= TOL_MAX and np.median(err) <= TOL_MEDIAN
