@@ -2456,10 +2456,13 @@ namespace nbg
         // Targets per warp: 128 once there are three such tiles a resident warp, 64 once there is
         // one, else 32. A wider walk opens fewer cells in all but leaves fewer tiles to balance,
         // and each takes longer. Walk in ms at 32 / 64 / 128 targets: 20,000 bodies (two Plummer
-        // spheres), theta 2: 0.47 / 0.70 / 1.05; 262,144: 1.60 / 1.59 / 1.62, theta 0.5: 0.086 /
-        // 0.088 / 0.113; 1M disk, theta 0.5: 0.213 / 0.197 / 0.244; 4M disk + halo, theta 2:
-        // 24.9 / 17.6 / 16.8. NBODY_CUDA_BH_TARGETS (32, 64, 128 or 256) overrides; all give the
-        // same sums.
+        // spheres), theta 2: 0.49 / 0.74 / 1.09; 262,144: 1.63 / 1.51 / 1.62, theta 0.5: 0.088 /
+        // 0.090 / 0.117; 1M disk, theta 0.5: 0.213 / 0.197 / 0.244; 4M disk + halo, theta 2:
+        // 24.9 / 17.6 / 16.8. Where targets have many cells (theta from 1.25) 64 already when 32
+        // would take two tiles a resident warp: 262,144 at theta 1.33 / 2, 32 against 64: disk
+        // 0.534 / 0.965 and 0.490 / 0.864, disk + halo 0.725 / 1.712 and 0.692 / 1.593, uniform
+        // cube 0.461 / 1.049 and 0.479 / 1.057; at theta 1 the disk 0.391 and 0.387, the cube 0.295
+        // and 0.322. NBODY_CUDA_BH_TARGETS (32, 64, 128 or 256) overrides; all give the same sums.
         const char* tsel = std::getenv("NBODY_CUDA_BH_TARGETS");
         const int per_warp = tsel ? std::atoi(tsel) : 0;
         const bool soft = p->law == NBODY_LAW_SOFTENED;
@@ -2484,14 +2487,13 @@ namespace nbg
         if (!per_warp)
         {
             auto resident = [&](const int i) { return static_cast<long long>(per_sm(i)) * sms * trav_warps(1 << i); };
-            fi = ni >= 3 * 128 * resident(2) ? 2 : (ni >= 64 * resident(1) ? 1 : 0);
+            const bool wide = ni >= 64 * resident(1) || (p->theta >= 1.25f && ni >= 2 * 32 * resident(0));
+            fi = ni >= 3 * 128 * resident(2) ? 2 : (wide ? 1 : 0);
         }
         // one resident wave of CTAs, each warp drawing tiles until none are left
         const int warps = trav_warps(1 << fi);
         const int tiles = (ni + (32 << fi) - 1) / (32 << fi);
-        int grid = std::min((tiles + warps - 1) / warps, sms * per_sm(fi));
-        if (grid > 3 * sms)
-            grid = grid / sms * sms;    // as many CTAs on every SM
+        const int grid = std::min((tiles + warps - 1) / warps, sms * per_sm(fi));
         launch_after(early, fns[fi], grid, warps * 32, 0, s, b.nodes, b.spm, b.srad, b.codes, b.order, ni, p->G, p->eps2, acc, body_out,
                                             ctx->dev_error, b.stats);
         ++ctx->launches;

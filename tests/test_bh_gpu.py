@@ -744,3 +744,24 @@ def test_sort_order_around_two_tiles_an_sm(gpu, past):
     """The last size of the passes that spend registers on latency, and the first one beyond."""
     import torch
     test_sort_order_at_tile_edges(gpu, 2 * torch.cuda.get_device_properties(0).multi_processor_count * 4096 + past)
+
+
+@pytest.mark.parametrize("theta,width", [(0.5, "32"), (1.0, "32"), (1.33, "64"), (2.0, "64")])
+def test_walk_width_follows_the_opening_parameter(gpu, theta, width, monkeypatch):
+    """Between two 32-target tiles and one 64-target tile a resident warp (250,000 bodies) the walk
+    is 64 targets wide from theta 1.25: the cells visited are that width's, the sums every
+    width's."""
+    from nbody_gb300 import scenes
+    b = scenes.two_plummer(125000)
+    kw = dict(theta=theta, law=gpu.LAW_SOFTENED, eps2=1e-4, size=0.0, tree_box=1)
+    out = {}
+    for w in ("32", "64", None):
+        if w:
+            monkeypatch.setenv("NBODY_CUDA_BH_TARGETS", w)
+        else:
+            monkeypatch.delenv("NBODY_CUDA_BH_TARGETS")
+        out[w] = bh_accel(gpu, b, **kw)
+    assert out["32"][1]["visits"] != out["64"][1]["visits"]
+    assert out[None][1] == out[width][1]
+    for w in ("32", "64"):
+        assert np.array_equal(out[None][0].view(np.uint32), out[w][0].view(np.uint32))
