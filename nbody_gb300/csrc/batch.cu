@@ -366,13 +366,22 @@ namespace nbg
         // few targets unused: 64 systems of 64 to 1,024 bodies take 19 us against 44 with
         // cfg<64, 4>(1024), 32 of 64 to 8,192 135 against 165, 300 of 64 to 4,096 (6e8 pairs) 240
         // against 254. From about 1e9 pairs four targets a lane and pre-paired sources win: 512
-        // systems of 64 to 8,192 (3.5e9 pairs) 1,516 us against 1,572 with small items.
+        // systems of 64 to 8,192 (3.5e9 pairs) 1,516 us against 1,572 with small items. Systems of
+        // more than 2^15 bodies (the mean over pairs) have items enough with 1,024 sources each,
+        // half the partial sums: one of 100,000 3.65 ms against 3.85 with 512 (3.79 with
+        // cfg<64, 4>(1024)), one of 65,536 and two of 100 1.59 against 1.73 (1.64), one of 50,000 and
+        // three smaller 1.13 against 1.18 (1.16); two of 32,768 0.82 against 0.85 (0.85), 20 of
+        // 12,000 1.06 both ways, 100 of 4,096 0.65 against 0.62.
         int default_config(const std::vector<int>& off)
         {
-            double pairs = 0;
+            double pairs = 0, weighted = 0;
             for (size_t s = 0; s + 1 < off.size(); ++s)
-                pairs += static_cast<double>(off[s + 1] - off[s]) * (off[s + 1] - off[s]);
-            return pairs < 1e9 ? 10 : 11;
+            {
+                const double n = off[s + 1] - off[s];
+                pairs += n * n;
+                weighted += n * n * n;
+            }
+            return pairs < 1e9 ? 10 : (weighted > 32768.0 * pairs ? 8 : 11);
         }
 
         int targets_per_item(const Config& c) { return c.block * c.t; }

@@ -211,3 +211,23 @@ def test_default_configuration(gpu, sizes, index):
         tg = np.unique(np.r_[0, len(sb) - 1, np.random.default_rng(s).integers(0, len(sb), 60)])
         ref, scale = O.direct_f64(sb[:, [0, 1, 2, 7]], 1.0, float(np.float32(EPS2)), O.LAW_SOFTENED, targets=tg, with_scale=True)
         assert (np.linalg.norm(acc[off[s]:off[s + 1]][tg] - ref, axis=1) / np.maximum(scale, 1e-30)).max() <= 5e-5
+
+
+@pytest.mark.parametrize("sizes,index", [([32769, 40000], 8), ([70001], 8), ([40000, 32768, 32768], 8),
+                                         ([33000] + [8000] * 30, 11)], ids=["two", "one", "three", "few-large"])
+def test_default_configuration_of_large_systems(gpu, sizes, index):
+    """Chunks of 1,024 sources where the systems are larger than 2^15 bodies in the mean over their
+    pairs: sampled targets against FP64 with this file's bar."""
+    b, off = make_batch(sizes)
+    p = gpu.params(mode=gpu.MODE_BATCHED, law=gpu.LAW_SOFTENED, eps2=EPS2)
+    with gpu.Context() as ctx:
+        ctx.upload_bodies(b)
+        ctx.set_systems(off)
+        assert ctx.batch_config(-1) == ctx.batch_config(index)
+        ctx.accelerate(p)
+        acc = ctx.download_bodies()[:, 8:11]
+    for s in range(min(len(sizes), 3)):
+        sb = b[off[s]:off[s + 1]]
+        tg = np.unique(np.r_[0, len(sb) - 1, np.random.default_rng(s).integers(0, len(sb), 40)])
+        ref, scale = O.direct_f64(sb[:, [0, 1, 2, 7]], 1.0, float(np.float32(EPS2)), O.LAW_SOFTENED, targets=tg, with_scale=True)
+        assert (np.linalg.norm(acc[off[s]:off[s + 1]][tg] - ref, axis=1) / np.maximum(scale, 1e-30)).max() <= 5e-5
