@@ -883,7 +883,7 @@ int nbody_cuda_update_graph(nbody_cuda* ctx, const nbody_step_params* p, const i
         NBG_CUDA(ctx, cudaGraphLaunch(ctx->graph, ctx->stream), "graph launch");
         ctx->launches += ctx->graph_launches;
     }
-    ctx->query_nodes_id = 0;    // replays rebuilt the tree without the host noticing
+    ctx->query_nodes_id = ctx->tree_host_id = 0;    // replays rebuilt the tree without the host noticing
     return NBODY_OK;
 }
 

@@ -94,6 +94,8 @@ struct nbody_cuda
     size_t query_nodes_cap = 0;
     uint64_t query_nodes_id = 0;
     size_t query_nodes_count = 0;
+    std::vector<unsigned char> tree_host;   // a small tree as exported, while tree_host_id is its build
+    uint64_t tree_host_id = 0;
     void* query_buf = nullptr;
     size_t query_buf_cap = 0;
 

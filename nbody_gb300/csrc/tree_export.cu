@@ -27,6 +27,9 @@
 //
 // The expansion ran on the host before, from a copy of the tree: a build, an export and a query
 // of 20,000 rays over 250,000 bodies took 23.6 ms, 1.6 ms with it here.
+#include <algorithm>
+#include <cstring>
+
 #include "bh.cuh"
 #include "common.cuh"
 #include "context.cuh"
@@ -308,11 +311,31 @@ extern "C" int nbody_cuda_tree_export(nbody_cuda* ctx, void* nodes, const size_t
     using namespace nbg;
     if (!ctx || !count)
         return NBODY_ERR_INVALID;
-    size_t have = 0;
-    if (const int st = tree_on_device(ctx, &have))
-        return st;
+    // A small tree is kept on the host once it was exported: exporting it again needs no device
+    // (1,000 bodies 7 us, 35 from the device). A larger one's first export would pay for it
+    // (20,000 bodies, 3.7 MB: a build and an export 691 us, 543 without; again 190 and 320).
+    constexpr size_t kHostBytes = size_t(1) << 20;
+    const uint64_t id = bh_build_id(ctx);
+    if (!id || ctx->tree_host_id != id)
+    {
+        size_t have = 0;
+        if (const int st = tree_on_device(ctx, &have))
+            return st;
+        *count = have;
+        if (!nodes || !max_nodes)
+            return NBODY_OK;
+        const size_t bytes = have * sizeof(RefNode);
+        if (bytes > kHostBytes)
+            return d2h(ctx, nodes, ctx->query_nodes, std::min(have, max_nodes) * sizeof(RefNode));
+        ctx->tree_host_id = 0;
+        ctx->tree_host.resize(bytes);
+        if (const int st = d2h(ctx, ctx->tree_host.data(), ctx->query_nodes, bytes))
+            return st;
+        ctx->tree_host_id = ctx->query_nodes_id;
+    }
+    const size_t have = ctx->tree_host.size() / sizeof(RefNode);
     *count = have;
     if (nodes && max_nodes)
-        return d2h(ctx, nodes, ctx->query_nodes, (have < max_nodes ? have : max_nodes) * sizeof(RefNode));
+        std::memcpy(nodes, ctx->tree_host.data(), std::min(have, max_nodes) * sizeof(RefNode));
     return NBODY_OK;
 }

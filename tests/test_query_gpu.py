@@ -119,3 +119,38 @@ def test_few_and_many_rays_agree(gpu, stop):
         few, nfew = ctx.tree_query(rays, stop, 64)
         many, nmany = ctx.tree_query(np.tile(rays, (100, 1)), stop, 64)
     assert np.array_equal(np.tile(few, (100, 1)), many) and np.array_equal(np.tile(nfew, 100), nmany)
+
+
+@pytest.mark.parametrize("n", [1, 1000])
+def test_small_tree_exported_again_needs_no_device(gpu, n):
+    """The second export of a small tree comes from the host: it works while the context's stream is
+    being captured, gives the same nodes, also after a query over other nodes, and is of the
+    new tree after the next build or a replayed step."""
+    import torch
+    from nbody_gb300 import scenes
+    b = scenes.plummer(n, seed=n)
+    p = gpu.params(mode=gpu.MODE_NLOGN, law=gpu.LAW_SOFTENED, eps2=1e-4, theta=0.5, size=64.0, dt=0.05)
+    s = torch.cuda.Stream()
+    x = torch.zeros(4, device="cuda")
+    torch.cuda.synchronize()
+    with gpu.Context() as ctx:
+        ctx.set_stream(s.cuda_stream)
+        ctx.upload_bodies(b)
+        ctx.accelerate(p)
+        first = ctx.tree_export()
+        lone = first[:1].copy()
+        lone["children"] = 0
+        ctx.tree_query(np.array([[0, 0, 0, 1, 2, 3]], np.float32), nodes=lone)
+        launches = ctx.launches()
+        with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=s, capture_error_mode="thread_local"):
+            x.add_(1)
+            again = ctx.tree_export()
+        assert np.array_equal(first, again) and ctx.launches() == launches
+        ctx.update(p)
+        moved = ctx.tree_export()
+        ctx.update_graph(p, 3)
+        replayed = ctx.tree_export()
+        ctx.accelerate(p)
+        if n > 1:
+            assert not np.array_equal(moved["com"], replayed["com"])
+            assert not np.array_equal(replayed["com"], ctx.tree_export()["com"])
