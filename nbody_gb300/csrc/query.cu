@@ -34,47 +34,15 @@ namespace nbg
             float o[3], d[3];
         };
 
-        // Bounds::ray_intersect_coord<i> with length = FLT_MAX: the reference only lowers
-        // length on a hit, after which ray_intersect returns.
-        __device__ __forceinline__ bool face(const Ray& r, const float c[3], const float s, const int i)
-        {
-            const int j = (i + 1) % 3, k = (i + 2) % 3;
-            float t;
-            if (r.d[i] < -FLT_EPSILON)
-                t = __fdiv_rn(__fsub_rn(__fadd_rn(c[i], s), r.o[i]), r.d[i]);
-            else if (r.d[i] > FLT_EPSILON)
-                t = __fdiv_rn(__fsub_rn(__fsub_rn(c[i], s), r.o[i]), r.d[i]);
-            else
-                return false;
-            if (!(t < FLT_MAX))
-                return false;
-            const float pj = __fadd_rn(r.o[j], __fmul_rn(r.d[j], t));
-            const float pk = __fadd_rn(r.o[k], __fmul_rn(r.d[k], t));
-            return pj > __fsub_rn(c[j], s) && pj < __fadd_rn(c[j], s) && pk > __fsub_rn(c[k], s)
-                   && pk < __fadd_rn(c[k], s);
-        }
-
+        // Bounds::ray_intersect: the origin in the box, or a face pair met (each as
+        // Bounds::ray_intersect_coord<i> with length = FLT_MAX: the reference only lowers length
+        // on a hit, after which it returns). Without branches, so that the three faces'
+        // divisions and tests overlap; a face along the ray divides by 1, since by zero is the
+        // division's slow path. Face after face with branches took, at eight lanes a
+        // ray, 410 against 360 us for 20,011 picking rays among 250,007 bodies and 7.7 against 5.9 ms
+        // for 10,000 that meet 1,540 nodes each; at one, among 2^20 bodies, 7.5 against 4.1 ms for 10^6
+        // picking rays, 30 against 11 for 100,000 that meet all, 2.03 against 2.12 for 10^6 along an axis.
         __device__ __forceinline__ bool ray_meets(const Ray& r, const float4 b)
-        {
-            const float c[3] = { b.x, b.y, b.z };
-            const float s = b.w;
-            bool inside = true;
-            for (int i = 0; i < 3; ++i)
-                if (r.o[i] < __fsub_rn(c[i], s) || r.o[i] > __fadd_rn(c[i], s))
-                {
-                    inside = false;
-                    break;
-                }
-            if (inside)
-                return true;
-            return face(r, c, s, 0) || face(r, c, s, 1) || face(r, c, s, 2);
-        }
-
-        // ray_meets without branches, for the kernel of few rays: the three faces' divisions and
-        // tests overlap instead of following one another (1,000 rays that meet 1,540 nodes each
-        // 6.4 -> 4.8 ms, 10,000 7.7 -> 5.9, 20,011 picking rays among 250,007 bodies 410 -> 360 us).
-        // A face along the ray divides by 1: by zero is the division's slow path.
-        __device__ __forceinline__ bool ray_meets_flat(const Ray& r, const float4 b)
         {
             const float c[3] = { b.x, b.y, b.z };
             const float s = b.w;
@@ -149,7 +117,7 @@ namespace nbg
         // lane each -- a block of siblings when it descends -- and the walk goes on among them
         // by their links, whatever those are, until it leaves them. A walk is a chain of
         // dependent node loads and tests, so its time is its number of such windows; with one
-        // thread a ray it is the number of nodes (20,000 rays, 250,000 bodies: 0.81 against
+        // thread a ray it is the number of nodes (20,000 rays, 250,000 bodies: 0.42 against
         // 0.34 ms). Nodes that are tested in vain cost throughput once the rays fill the GPU.
         __global__ void __launch_bounds__(kBlock) query_group_kernel(const float4* __restrict__ nodes, const uint32_t count,
                                                                const float* __restrict__ rays, const uint32_t nrays,
@@ -192,7 +160,7 @@ namespace nbg
                     const uint2 links = __ldg(reinterpret_cast<const uint2*>(&nodes[at + 2]));
                     next = links.x;
                     children = links.y;
-                    met = __ballot_sync(group, ray_meets_flat(r, bounds)) >> (threadIdx.x & 24);
+                    met = __ballot_sync(group, ray_meets(r, bounds)) >> (threadIdx.x & 24);
                     bodies = __ballot_sync(group, links.y == 0 && mass != 0.f) >> (threadIdx.x & 24);
                 }
                 const uint32_t w = idx - base;
@@ -275,9 +243,9 @@ namespace nbg
         if (const int st = h2d(ctx, buf, rays, ray_bytes))
             return st;
         // Eight lanes a ray while every ray's lanes are resident at once (38,912 rays), else one.
-        // Picking in 2^20 bodies with copies, one / eight lanes: 1,000 rays 0.25 / 0.20 ms, 20,000
-        // 0.30 / 0.28, 100,000 0.54 / 0.71, 10^6 2.46 / 4.24; all nodes met (1,540 a ray): 1,000
-        // 22.1 / 4.8, 10,000 24.7 / 5.9, 100,000 30.1 / 28.2, 10^6 177 / 232.
+        // Calls among 2^20 bodies in ms, eight lanes / one, picking: 1,000 rays 0.28 / 0.41, 20,000 0.46 /
+        // 0.58, 38,912 0.68 / 0.64, 100,000 1.25 / 0.83, 10^6 9.2 / 4.1; all nodes met: 1,000 6.4 / 10.6,
+        // 10,000 7.0 / 9.4, 20,000 9.8 / 9.3, 100,000 36 / 11.
         int sms = 0, threads = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
         cudaDeviceGetAttribute(&threads, cudaDevAttrMaxThreadsPerMultiProcessor, ctx->device);
