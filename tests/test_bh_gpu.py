@@ -765,3 +765,26 @@ def test_walk_width_follows_the_opening_parameter(gpu, theta, width, monkeypatch
     assert out[None][1] == out[width][1]
     for w in ("32", "64"):
         assert np.array_equal(out[None][0].view(np.uint32), out[w][0].view(np.uint32))
+
+
+@pytest.mark.parametrize("width", ["32", "64", "128", "256"])
+@pytest.mark.parametrize("theta", [0.5, 2.0])
+@pytest.mark.parametrize("n", [31, 33, 65, 131, 259, 1025])
+def test_walk_of_special_bodies_against_the_oracle(gpu, n, theta, width, monkeypatch):
+    """Coincident bodies (a bucket, of more than eight in the larger systems), massless ones, and
+    last a massless body that is not a number, whose tile decides target by target: each
+    width's accelerations are those of the reference's octree over the numbers alone, which a
+    massless body does not change, to the file's bar but for two bodies."""
+    from nbody_gb300 import scenes
+    b = scenes.plummer(n, seed=100 + n)
+    b[:, 3] = np.float32(1e-3)
+    b[7:10 if n < 100 else 20, :3] = b[3, :3]
+    b[21:24, 7] = 0.0
+    ref, _ = O.barnes_hut(b, 64.0, theta, 1.0)
+    monkeypatch.setenv("NBODY_CUDA_BH_TARGETS", width)
+    acc, _ = bh_accel(gpu, b, theta=theta, law=0, size=64.0)
+    compare_to_reference(acc, ref[:, 8:11], b, allowed_outliers=2)
+    odd = np.concatenate([b, b[:1]])
+    odd[n, 0], odd[n, 7] = np.nan, 0.0
+    with_odd, _ = bh_accel(gpu, odd, theta=theta, law=0, size=64.0)
+    compare_to_reference(with_odd[:n], ref[:, 8:11], b, allowed_outliers=2)
