@@ -2295,9 +2295,10 @@ namespace nbg
         // tree_box = 0 is the reference's fixed root box; it needs a positive size
         const bool auto_box = p->tree_box != 0 || !(p->size > 0.f);
         // the bounds pass runs for the fixed box too: the cell sums' scale comes from it
-        launch_after(early, bbox_kernel, std::min<unsigned>(kBboxBlocks, std::max(1u, ceil_div(n, 1024))), 256, 0, s, 
-            src, stride, ni, auto_box ? 1 : 0, p->size, b.bbox_part, b.box_ticket, reinterpret_cast<uint4*>(b.stats),
-            count_bytes(n) / 16, static_cast<uint4*>(b.temp), sort_zero_bytes(n) / 16, b.box);
+        launch_after(early, bbox_kernel, std::min<unsigned>(kBboxBlocks, std::max(1u, ceil_div(n, 1024))), 256, 0, s,
+                     src, stride, ni, auto_box ? 1 : 0, p->size, b.bbox_part, b.box_ticket,
+                     reinterpret_cast<uint4*>(b.stats), count_bytes(n) / 16, static_cast<uint4*>(b.temp),
+                     sort_zero_bytes(n) / 16, b.box);
         ++L;
         launch_after(early, morton_kernel, ceil_div(n, 256 * kMortonItems), 256, 0, s, src, stride, ni, b.box, b.keys[0], b.vals[0]);
         ++L;
@@ -2328,17 +2329,16 @@ namespace nbg
         // the last tile gives the sum of all bodies)
         Int64x4* tile_sum = static_cast<Int64x4*>(b.temp);
         Int64x4* tile_prefix = tile_sum + tiles + 1;
-        // adjacent prefix lengths, key samples and the far nodes' list live in the sort's
-        // other key and value buffers, free until the next build
+        // adjacent prefix lengths and key samples live in the sort's other key buffer, free until
+        // the next build
         const int other = in_alt ? 0 : 1;
         uint8_t* dl = reinterpret_cast<uint8_t*>(b.keys[other]);
         // (n rounded up to 8 bytes, then n / 64 + 1 keys: within the buffer's 8 n bytes for n >= 2)
         uint64_t* smp = reinterpret_cast<uint64_t*>(dl + ((n + 7) & ~size_t(7)));
         const bool radius = p->law == NBODY_LAW_CUTOFF;
         launch_after(early, gather_sum_kernel, tiles, kMomThreads, 0, s, src, stride,
-                                                        radius && ctx->layout != NBODY_LAYOUT_AOS ? ctx->vr : nullptr,
-                                                        order, ni, b.box, b.spm, radius ? b.srad : nullptr, b.psum,
-                                                        tile_sum, keys, dl, smp);
+                     radius && ctx->layout != NBODY_LAYOUT_AOS ? ctx->vr : nullptr, order, ni, b.box, b.spm,
+                     radius ? b.srad : nullptr, b.psum, tile_sum, keys, dl, smp);
         ++L;
         if (n < 2)
         {
@@ -2356,9 +2356,8 @@ namespace nbg
         ++L;
         launch_after(early, number_kernel, ceil_div(m, kNumTile), 1024, 0, s, b.octflag, m, b.octidx, b.numbering, ctx->dev_error);
         ++L;
-        launch_after(early, octnode_kernel, ceil_div(m, 256 * kOctSpan), 256, 0, s, b.child, b.range, b.prefix, b.octidx, b.psum,
-                                                                    tile_prefix, m, b.box, p->theta, b.nodes,
-                                                                    ctx->dev_error, b.stats);
+        launch_after(early, octnode_kernel, ceil_div(m, 256 * kOctSpan), 256, 0, s, b.child, b.range, b.prefix, b.octidx,
+                     b.psum, tile_prefix, m, b.box, p->theta, b.nodes, ctx->dev_error, b.stats);
         ++L;
         e = cudaGetLastError();
         if (e != cudaSuccess)

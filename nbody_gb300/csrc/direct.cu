@@ -106,9 +106,9 @@ namespace nbg
     // first gathered to {x, y, z, m}: one load a source in the loop instead of two.
     // U sources a loop iteration: their chains overlap. Bound by the FP32 pipe (12 packed
     // instructions a source and pair of targets; 91 % of it at 200,000 bodies). Before, with
-    // two sources an iteration and chunks planned by whole waves, and now: 20,011 bodies softened
-    // 176 -> 166 us, records under the cutoff law 221 -> 192; 32,768: 438 -> 419, 532 -> 450;
-    // 100,003: 3.61 -> 3.52 ms, 4.38 -> 3.95.
+    // two sources an iteration and chunks planned by whole waves, and now: one sum of 20,011
+    // bodies, softened, among other calls 147 -> 143 us; back to back, records under the cutoff
+    // law, 214 -> 185; 32,768: 438 -> 419 and 532 -> 450; 100,003: 3.63 -> 3.54 ms and 4.40 -> 3.96.
     template <int T, int BLOCK, int TILE, int STAGES, int LAW, bool AOS, bool PACKED, bool DUP, int U>
     __global__ void __launch_bounds__(BLOCK, (T >= 8 ? 2 : 3))
     direct_fp32_kernel(const float4* __restrict__ src,        // pos_mass (SoA) or Body (AoS)

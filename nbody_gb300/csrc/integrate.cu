@@ -148,11 +148,11 @@ namespace nbg
         if (n <= 0)
             return cudaSuccess;
         if (part && combine_width(n, js) == 8)
-            launch_after(true, integrate_soa_kernel<8>, ceil_div(static_cast<size_t>(n) * 8, kBlock), kBlock, 0, stream, 
-                pm, vr, acc, part, js, n, G, dt, size, wrap);
+            launch_after(true, integrate_soa_kernel<8>, ceil_div(static_cast<size_t>(n) * 8, kBlock), kBlock, 0, stream,
+                         pm, vr, acc, part, js, n, G, dt, size, wrap);
         else
-            launch_after(true, integrate_soa_kernel<1>, ceil_div(n, kBlock), kBlock, 0, stream, pm, vr, acc, part, js, n, G, dt, size,
-                                                                             wrap);
+            launch_after(true, integrate_soa_kernel<1>, ceil_div(n, kBlock), kBlock, 0, stream, pm, vr, acc, part, js,
+                         n, G, dt, size, wrap);
         ++*launches;
         return cudaGetLastError();
     }
@@ -164,11 +164,11 @@ namespace nbg
         if (n <= 0)
             return cudaSuccess;
         if (part && combine_width(n, js) == 8)
-            launch_after(true, integrate_aos_kernel<8>, ceil_div(static_cast<size_t>(n) * 8, kBlock), kBlock, 0, stream, 
-                bodies, part, js, n, G, dt, size, wrap);
+            launch_after(true, integrate_aos_kernel<8>, ceil_div(static_cast<size_t>(n) * 8, kBlock), kBlock, 0, stream,
+                         bodies, part, js, n, G, dt, size, wrap);
         else
-            launch_after(true, integrate_aos_kernel<1>, ceil_div(n, kBlock), kBlock, 0, stream, bodies, part, js, n, G, dt, size,
-                                                                             wrap);
+            launch_after(true, integrate_aos_kernel<1>, ceil_div(n, kBlock), kBlock, 0, stream, bodies, part, js, n, G,
+                         dt, size, wrap);
         ++*launches;
         return cudaGetLastError();
     }

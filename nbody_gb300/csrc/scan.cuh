@@ -42,11 +42,6 @@ namespace nbg
             return Int64x4{ __shfl_up_sync(0xffffffffu, v.x, d), __shfl_up_sync(0xffffffffu, v.y, d),
                             __shfl_up_sync(0xffffffffu, v.z, d), __shfl_up_sync(0xffffffffu, v.w, d) };
         }
-        static __device__ __forceinline__ Int64x4 shfl_down(Int64x4 v, int d)
-        {
-            return Int64x4{ __shfl_down_sync(0xffffffffu, v.x, d), __shfl_down_sync(0xffffffffu, v.y, d),
-                            __shfl_down_sync(0xffffffffu, v.z, d), __shfl_down_sync(0xffffffffu, v.w, d) };
-        }
     };
 
     // Number of T elements of temporary storage exclusive_scan needs for n items.

@@ -524,7 +524,8 @@ namespace nbg
         const auto pass_kernel = tiles <= kAheadTiles * setup.sms ? digit_pass_ahead_kernel : digit_pass_kernel;
         const TempLayout t = layout(temp, static_cast<size_t>(tiles));
         const int hist_grid = std::max(1, std::min((static_cast<int>(n) + kHistThreads - 1) / kHistThreads, 2 * setup.sms));
-        launch_after(early, digit_hist_kernel, hist_grid, kHistThreads, 0, stream, keys, static_cast<int>(n), begin_bit, passes, t.ghist);
+        launch_after(early, digit_hist_kernel, hist_grid, kHistThreads, 0, stream, keys, static_cast<int>(n), begin_bit,
+                     passes, t.ghist);
         ++*launches;
         cudaError_t e = cudaGetLastError();
         uint64_t* kin = keys;
@@ -533,9 +534,9 @@ namespace nbg
         uint32_t* vout = vals_alt;
         for (int p = 0; p < passes && e == cudaSuccess; ++p)
         {
-            launch_after(early, pass_kernel, tiles, kThreads, kPassSmem, stream, kin, vin, kout, vout, static_cast<int>(n),
-                                                                      begin_bit + p * kBits, p, t.ghist + p * kDigits,
-                                                                      t.status, t.tickets + p, err);
+            launch_after(early, pass_kernel, tiles, kThreads, kPassSmem, stream, kin, vin, kout, vout,
+                         static_cast<int>(n), begin_bit + p * kBits, p, t.ghist + p * kDigits, t.status, t.tickets + p,
+                         err);
             ++*launches;
             e = cudaGetLastError();
             std::swap(kin, kout);
