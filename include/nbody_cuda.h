@@ -367,7 +367,7 @@ int nbody_cuda_set_direct_variant(nbody_cuda* ctx, int index);
 
 /* Time every direct-sum kernel shape on the current bodies (FP32, p->law), pin the fastest
  * and return its index in *best; times_ms (optional, ntimes entries) receives each shape's
- * accelerate time. A system of up to 3072 bodies has a kernel of its own, which is none of the
+ * accelerate time. A system of up to 8192 bodies has a kernel of its own, which is none of the
  * shapes: it is left unpinned, and *best is -1 (which nbody_cuda_set_direct_variant takes for
  * "none"). Synchronous. */
 int nbody_cuda_direct_autotune(nbody_cuda* ctx, const nbody_step_params* p, double* times_ms,

@@ -27,10 +27,9 @@
 //     combine_partials). The runs are the same sources
 //     for every kernel shape and split, so the result does not depend on the
 //     launch shape (up to a rounding tie of the last fold), and it is more accurate than
-//     one FP32 running sum over all N sources. Systems of up to 3072 bodies are the exception
+//     one FP32 running sum over all N sources. Systems of up to 8192 bodies are the exception
 //     while no shape is pinned: their own kernel (direct_small.cu) sums shorter runs.
 #include <algorithm>
-#include <cmath>
 #include <cstdio>
 
 #include "common.cuh"
@@ -390,14 +389,12 @@ namespace nbg
         constexpr int kPlan = 10, kWideAosPlan = 11, kPairedPlan = 0, kNarrowPlan = 2;
         constexpr size_t kPairedMinN = 1 << 18, kPairedNearN = 1 << 16;
         constexpr size_t kMaxSplit = 64;                        // source chunks
-        // Up to 2^14 bodies of the split layout (2^13 body records) every chunk is one tile: CTAs of
-        // 128 targets and 256 sources are enough to pack the SMs evenly, which the fitted cost of a
-        // split does not see at so few CTAs. Split bodies, softened, the plan by that cost (the
-        // small systems' kernel up to 8,192) and this: 4,700 23.0 -> 20.7 us (a step 25.0 -> 18.5),
-        // 8,192 35.2 -> 35.2 (39.2 -> 33.1), 9,555 53.6 -> 46.4, 12,289 76 -> 70, 15,000 101 -> 99.
-        constexpr size_t kOneTileMaxN = kMaxSplit * kTile, kOneTileMaxAos = kOneTileMaxN / 2;
-        // CTAs of kNarrowPlan an SM holds for body records: 44 KB of shared memory each
-        constexpr size_t kNarrowAosCtas = 5;
+        // Up to 2^14 bodies of the split layout every chunk is one tile: CTAs of 128 targets and 256
+        // sources are enough to pack the SMs evenly, which the fitted cost of a split does not see
+        // at so few CTAs. Softened, the plan by that cost and this: 8,700 43.4 -> 39.2 us, 9,555
+        // 53.6 -> 46.4, 12,289 76 -> 70, 15,000 101 -> 99; body records, whose tiles leave an SM five
+        // such CTAs: 9,001 43.3 and 45.3, 10,200 55.7 and 55.6, by the cost.
+        constexpr size_t kOneTileMaxN = kMaxSplit * kTile;
 
         template <int T, int B, bool PACKED = true, bool DUP = false, int U = 2>
         Variant make_variant()
@@ -482,14 +479,9 @@ namespace nbg
         {
             chosen = law == NBODY_LAW_CUTOFF && aos ? kWideAosPlan
                                                     : (law == NBODY_LAW_SOFTENED && n >= kPairedMinN ? kPairedPlan : kPlan);
-            if (n <= (aos ? kOneTileMaxAos : kOneTileMaxN) && max_js == units)
+            if (!aos && n <= kOneTileMaxN && max_js == units)
             {
-                // Body records leave an SM five CTAs: where their last wave would be mostly empty,
-                // four times as many targets a CTA instead (7,600 softened: 39.5 against 33.0 us;
-                // 6,500, a wave and three quarters: 30.4 against 33.0).
-                const double waves = static_cast<double>(split_of(kNarrowPlan).tb * units)
-                                     / static_cast<double>(kNarrowAosCtas * sm_count());
-                chosen = !aos || waves >= 0.85 * std::ceil(waves) || waves <= 1.0 ? kNarrowPlan : kWideAosPlan;
+                chosen = kNarrowPlan;
                 most = true;
             }
             else if (split_bytes < kSplitBytes

@@ -40,8 +40,7 @@ namespace nbg
     }
 
     // Systems small enough for direct_small.cu, and for two targets a lane there (see the kernel).
-    // Beyond, chunks of one tile on CTAs of two warps are faster (plan_direct).
-    constexpr size_t kSmallDirect = 3072, kSmallPair = 2048;
+    constexpr size_t kSmallDirect = 8192, kSmallPair = 2048;
     constexpr int kSmallBlock = 256;
     constexpr int kSmallSplit = 8;      // CTAs a cluster: they share targets and split the sources
 

@@ -1,25 +1,28 @@
 // Direct-sum accelerations of small systems (the reference's N^2 mode) in one launch, for sm_103a.
 //
-// Up to 3072 bodies the direct sum is bound by latency: the launch, and the chain of dependent
+// Up to 8192 bodies the direct sum is bound by latency: the launch, and the chain of dependent
 // steps a thread runs through. So the work is spread as widely as the GPU is:
 //   - a cluster of 8 CTAs shares 32 T targets and splits the sources 64 ways, a contiguous
 //     slice per warp; every lane of a warp holds T targets as packed pairs and applies the
 //     warp's sources to them, staged 32 at a time in the warp's own shared memory as operand
 //     pairs ({x,x,y,y}, {z,z,m,m}) while the next 32 are on their way. No warp waits for
 //     another until its slice is summed;
-//   - a slice is at most 48 sources, where the larger shapes sum runs of 256 in FP32 (direct.cu):
-//     more accurate, but not their bits, so a system of up to 3072 bodies gets other bits when a
+//   - a slice is at most 128 sources, where the larger shapes sum runs of 256 in FP32 (direct.cu):
+//     more accurate, but not their bits, so a system of up to 8192 bodies gets other bits when a
 //     shape is pinned. The eight warps' sums are folded exactly into (S, C) pairs, and the eight
 //     CTAs' pairs are added through distributed shared memory as combine_partials adds a
 //     split's chunks. No partial goes through global memory and no second launch sums them.
 //
 // T = 2 up to 2048 bodies, where the CTAs are too few to fill the SMs otherwise (2000 bodies: 8.4
-// against 9.3 us a call); T = 4 beyond.
+// against 9.3 us a call, 4096: 15.0 against 14.6); T = 4 beyond.
 //
-// Steps one after another, before (a chunk of 256 sources per 64-thread CTA, then a sum of the
-// partials) and now: 500 bodies 24.7 -> 4.4 us, 1000 24.7 -> 5.6, 2000 24.7 -> 10.0, 3000 25.8 -> 13.2.
-// One accelerate of 1000 body records among others: 12.7 -> 7.0-7.4. The larger shapes with a chunk
-// a tile (plan_direct) do better from about 3500: 4096 bodies 18.6 -> 14.4 a step, 8192 36.9 -> 33.0.
+// Before (a chunk of 256 sources per 64-thread CTA, then a sum of the partials) and now. One
+// accelerate of 1000 body records among others: 12.7 -> 7.0-7.4 us; a sum that is waited for, 4096
+// bodies 34 -> 27, 8192 56 -> 52. Steps one after another: 500 bodies 24.7 -> 4.4, 1000 24.7 -> 5.6,
+// 2000 24.7 -> 10.0, 3000 25.8 -> 13.2, 4096 18.3 -> 18.7 (replayed 16.7 -> 14.5), 6000 27.8 -> 28.8
+// (27.0 -> 24.8), 8192 37.1 -> 36.9 (37.0 -> 39.1). Chunks of one tile (plan_direct) would step 4096 in 14.4
+// and 8192 in 33.0 us, but with runs of 256 for twice the error; folded every 64 sources they keep it
+// and take 14 % longer for a sum of 4096 that is waited for, 37 % for one of 4400.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
